@@ -16,17 +16,28 @@ template <> struct cx_t<float> { using type = float2; };
 template <> struct cx_t<double> { using type = double2; };
 template <typename T> using cx = typename cx_t<T>::type;
 
+// Multiply, add and fused multiply-add with one rounding each, never contracted or split by
+// the compiler.  Everything a field value passes through is written with these, so that every
+// kernel that inlines it rounds alike: the fused, wide and multi-pass marches of one instance
+// give the same bits.
+__device__ __forceinline__ float fma_r(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_r(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float mul_r(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_r(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float add_r(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double add_r(double a, double b) { return __dadd_rn(a, b); }
+
 template <typename T> __device__ __forceinline__ cx<T> mk(T re, T im) { cx<T> c; c.x = re; c.y = im; return c; }
-template <typename T> __device__ __forceinline__ cx<T> add(cx<T> a, cx<T> b) { return mk<T>(a.x + b.x, a.y + b.y); }
-template <typename T> __device__ __forceinline__ cx<T> sub(cx<T> a, cx<T> b) { return mk<T>(a.x - b.x, a.y - b.y); }
+template <typename T> __device__ __forceinline__ cx<T> add(cx<T> a, cx<T> b) { return mk<T>(add_r(a.x, b.x), add_r(a.y, b.y)); }
+template <typename T> __device__ __forceinline__ cx<T> sub(cx<T> a, cx<T> b) { return mk<T>(add_r(a.x, -b.x), add_r(a.y, -b.y)); }
 template <typename T> __device__ __forceinline__ cx<T> mul(cx<T> a, cx<T> b) {
-    return mk<T>(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+    return mk<T>(fma_r(a.x, b.x, mul_r(-a.y, b.y)), fma_r(a.x, b.y, mul_r(a.y, b.x)));
 }
 // a * conj(b)
 template <typename T> __device__ __forceinline__ cx<T> mulc(cx<T> a, cx<T> b) {
-    return mk<T>(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y);
+    return mk<T>(fma_r(a.x, b.x, mul_r(a.y, b.y)), fma_r(a.y, b.x, mul_r(-a.x, b.y)));
 }
-template <typename T> __device__ __forceinline__ cx<T> scale(cx<T> a, T s) { return mk<T>(a.x * s, a.y * s); }
+template <typename T> __device__ __forceinline__ cx<T> scale(cx<T> a, T s) { return mk<T>(mul_r(a.x, s), mul_r(a.y, s)); }
 
 // FP32 complex add / sub as one packed two-lane instruction each (sm_100 f32x2).  Both
 // lanes round to nearest like the scalar pair; a - b is fma(b, -1, a), exact in the product.
@@ -67,14 +78,26 @@ __host__ __device__ constexpr double sin32(int m) { return cos32((m + 24) & 31);
 // into hi + lo parts and applied with fused multiply-adds, so its rounding does not
 // bias the modulus of every transform by the same relative amount step after step (a
 // coherent error that would grow linearly with the number of SSFM steps).
+//
+// The sum of two products fuses one of them into the add; which one is a free choice, made
+// here (re2, im2: the second) as the compiler made it in the fused march before the choice was
+// written out, so the FP32 fields of a plain run kept their bits.
 template <typename T>
 __device__ __forceinline__ cx<T> rot_const(cx<T> v, double c, double s) {
+    const bool diag = c == s, anti = c == -s;  // odd multiples of 45 degrees
+    const bool re2 = sizeof(T) == 8 && diag, im2 = sizeof(T) == 8 ? !anti : !diag;
+    auto re = [&](T cc, T ss) {  // x c - y s
+        return re2 ? fma_r(-v.y, ss, mul_r(v.x, cc)) : fma_r(v.x, cc, mul_r(-v.y, ss));
+    };
+    auto im = [&](T cc, T ss) {  // x s + y c
+        return im2 ? fma_r(v.y, cc, mul_r(v.x, ss)) : fma_r(v.x, ss, mul_r(v.y, cc));
+    };
     if constexpr (sizeof(T) == 8) {
-        return mk<T>(v.x * c - v.y * s, v.x * s + v.y * c);
+        return mk<T>(re(c, s), im(c, s));
     } else {
         const float ch = (float)c, sh = (float)s;
         const float cl = (float)(c - (double)ch), sl = (float)(s - (double)sh);
-        return mk<T>(fmaf(v.x, ch, fmaf(-v.y, sh, v.x * cl - v.y * sl)), fmaf(v.x, sh, fmaf(v.y, ch, v.x * sl + v.y * cl)));
+        return mk<T>(fma_r(v.x, ch, fma_r(-v.y, sh, re(cl, sl))), fma_r(v.x, sh, fma_r(v.y, ch, im(cl, sl))));
     }
 }
 
@@ -117,19 +140,27 @@ template <> __host__ __device__ __forceinline__ float4 make_mult<float>(double r
 
 // v * w
 __device__ __forceinline__ double2 mulw(double2 v, double2 w) {
-    return make_double2(v.x * w.x - v.y * w.y, v.x * w.y + v.y * w.x);
+    return make_double2(fma_r(v.x, w.x, mul_r(-v.y, w.y)), fma_r(v.y, w.x, mul_r(v.x, w.y)));
 }
 __device__ __forceinline__ float2 mulw(float2 v, float4 w) {
-    return make_float2(fmaf(v.x, w.x, fmaf(-v.y, w.y, v.x * w.z - v.y * w.w)),
-                       fmaf(v.x, w.y, fmaf(v.y, w.x, v.x * w.w + v.y * w.z)));
+    return make_float2(fma_r(v.x, w.x, fma_r(-v.y, w.y, fma_r(v.x, w.z, mul_r(-v.y, w.w)))),
+                       fma_r(v.x, w.y, fma_r(v.y, w.x, fma_r(v.y, w.z, mul_r(v.x, w.w)))));
+}
+// conj(v) * w
+__device__ __forceinline__ double2 mulw_cj(double2 v, double2 w) {
+    return make_double2(fma_r(v.x, w.x, mul_r(v.y, w.y)), fma_r(v.x, w.y, mul_r(-v.y, w.x)));
+}
+__device__ __forceinline__ float2 mulw_cj(float2 v, float4 w) {
+    return make_float2(fma_r(v.x, w.x, fma_r(v.y, w.y, fma_r(v.x, w.z, mul_r(v.y, w.w)))),
+                       fma_r(v.x, w.y, fma_r(-v.y, w.x, fma_r(v.x, w.w, mul_r(-v.y, w.z)))));
 }
 // v * conj(w)
 __device__ __forceinline__ double2 mulwc(double2 v, double2 w) {
-    return make_double2(v.x * w.x + v.y * w.y, v.y * w.x - v.x * w.y);
+    return make_double2(fma_r(v.x, w.x, mul_r(v.y, w.y)), fma_r(v.y, w.x, mul_r(-v.x, w.y)));
 }
 __device__ __forceinline__ float2 mulwc(float2 v, float4 w) {
-    return make_float2(fmaf(v.x, w.x, fmaf(v.y, w.y, v.x * w.z + v.y * w.w)),
-                       fmaf(v.y, w.x, fmaf(-v.x, w.y, v.y * w.z - v.x * w.w)));
+    return make_float2(fma_r(v.x, w.x, fma_r(v.y, w.y, fma_r(v.x, w.z, mul_r(v.y, w.w)))),
+                       fma_r(v.y, w.x, fma_r(-v.x, w.y, fma_r(v.y, w.z, mul_r(-v.x, w.w)))));
 }
 
 template <int M, int SIGN, typename T> struct Dft;
@@ -150,7 +181,7 @@ template <int SIGN, typename T> struct Dft<3, SIGN, T> {
     static __device__ __forceinline__ void run(cx<T> (&v)[3]) {
         cx<T> t = add<T>(v[1], v[2]);
         cx<T> u = sub<T>(v[1], v[2]);
-        cx<T> m = mk<T>(v[0].x - (T)0.5 * t.x, v[0].y - (T)0.5 * t.y);
+        cx<T> m = mk<T>(fma_r((T)-0.5, t.x, v[0].x), fma_r((T)-0.5, t.y, v[0].y));
         v[0] = add<T>(v[0], t);
         // X1 = m + SIGN*i*h*u, X2 = m - SIGN*i*h*u, h = sqrt(3)/2
         const cx<T> hu = rot_const<T>(u, 0.866025403784438646764, 0.0);

@@ -53,6 +53,18 @@ cudaError_t fork_streams(int dev, ForkStreams** out) {
     return cudaSuccess;
 }
 
+// The wide march for `count` plain runs p of variant v's class on their own; null where the
+// caller or a tuner chose the march, or the wide one is not faster.
+const PlainVariant* wide_choice(const shg_params& p, const PlainVariant* v, int count) {
+    if (p.march != SHG_MARCH_AUTO || has_plain_choice(v->precision, v->n, 0)) return nullptr;
+    return wide_variant_for(v->precision, v->n, 0, count);
+}
+
+// The descriptor of one run, as a kernel argument: no copy from the caller's stack.
+__global__ void put_desc_kernel(InstDesc d, InstDesc* out) {
+    if (threadIdx.x == 0) *out = d;
+}
+
 }  // namespace
 
 shg_status plain_solve_device(const shg_params& p, const void* signal_in, void* pump_out, void* signal_out,
@@ -61,6 +73,7 @@ shg_status plain_solve_device(const shg_params& p, const void* signal_in, void* 
     int out32 = 0;
     const PlainVariant* v = plain_variant_of(p, &out32);
     if (!v) return fail(SHG_ERR_UNSUPPORTED, "no kernel for grid side %d", p.nx);
+    if (const PlainVariant* w = wide_choice(p, v, 1)) v = w;
     InstDesc d = make_plain_desc(p, p.temp, p.temp);
     d.out32 = out32;
     d.signal_in = signal_in;
@@ -81,8 +94,9 @@ shg_status plain_solve_device(const shg_params& p, const void* signal_in, void* 
     shg_status rc = SHG_OK;
     cudaEvent_t t0 = nullptr, t1 = nullptr;
     do {
-        if ((e = cudaMemcpyAsync(dd, &d, sizeof(d), cudaMemcpyHostToDevice, stream)) != cudaSuccess) {
-            rc = cuda_fail(e, "cudaMemcpyAsync desc");
+        put_desc_kernel<<<1, 32, 0, stream>>>(d, dd);
+        if ((e = cudaGetLastError()) != cudaSuccess) {
+            rc = cuda_fail(e, "launch put_desc_kernel");
             break;
         }
         if (stats) {
@@ -109,6 +123,8 @@ shg_status plain_solve_device(const shg_params& p, const void* signal_in, void* 
             stats->device_ms = ms;
             if (!std::isfinite(h[0]) || !std::isfinite(h[1]))
                 rc = fail(SHG_ERR_NONFINITE, "SH / pump power %g / %g", h[0], h[1]);
+            else if (h[0] < 0.0)
+                rc = fail(SHG_ERR_CUDA, "a grid barrier of the march ran out");
         }
     } while (0);
     if (t0) cudaEventDestroy(t0);
@@ -140,6 +156,19 @@ static BatchLayout batch_layout(const shg_params* params, int count, void* const
         const PlainVariant* v = plain_variant_of(params[i], &out32);
         items[i] = {v, i, (double)params[i].nx * params[i].nx * shg_steps(&params[i]), out32};
     }
+    // A batch small enough to march side by side on the wide march takes it: the classes share
+    // the device, so the parts of it that they fill must add up to at most one.
+    std::vector<const PlainVariant*> wide;
+    double share = 0.0;
+    for (int i = 0; i < count && share < 1.0 + 1e-9; ++i) {
+        int fit = 0;
+        const PlainVariant* w = wide_choice(params[i], items[i].v, 1);
+        if (!w || w->fit(&fit) != cudaSuccess) break;
+        wide.push_back(w);
+        share += 1.0 / fit;
+    }
+    if ((int)wide.size() == count && share < 1.0 + 1e-9)
+        for (int i = 0; i < count; ++i) items[i].v = wide[i];
     std::stable_sort(items.begin(), items.end(), [](const Item& a, const Item& b) {
         if (a.v != b.v) return a.v < b.v;
         return a.cost > b.cost;
@@ -322,6 +351,8 @@ shg_status plain_solve_batch(const shg_params* params, int count, void* const* p
                 break;
             }
             for (int i = 0; i < count; ++i) sh_power_out[i] = h[2 * (size_t)i];
+            for (int i = 0; i < count && rc == SHG_OK; ++i)
+                if (h[2 * (size_t)i] < 0.0) rc = fail(SHG_ERR_CUDA, "instance %d: a grid barrier of the march ran out", i);
             for (int i = 0; i < count && rc == SHG_OK; ++i)
                 if (!std::isfinite(h[2 * (size_t)i]) || !std::isfinite(h[2 * (size_t)i + 1]))
                     rc = fail(SHG_ERR_NONFINITE, "instance %d: SH / pump power %g / %g", i, h[2 * (size_t)i],

@@ -50,6 +50,8 @@ struct InstDesc {
     double bf_s;           // βs 0.5 ε0 c (the two-photon term is bf_s n_s |S|^2)
     double q_p, q_s, q_h;  // αp 0.5 c ε0, αs 0.5 c ε0, 0.5 c ε0: Q = q_p n_p |P|^2 + q_s n_s |S|^2 + βs (q_h n_s |S|^2)^2
     double beta_s;         // βs
+    double* w_out;         // thermal: device, [2][n*n]: n_s |S|^2 and n_p |P|^2 of the output fields, which
+                           // launch_thermal_power sums in one order whichever march wrote them
 };
 
 }  // namespace shg

@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(NT, MARCH_ONLY ? 2 : 1) ssfm_adjoint_kernel(co
         if (inv) {
             v[0] = cj(v[0]);
 #pragma unroll
-            for (int k = 1; k < R2; ++k) v[k] = mulw(cj(v[k]), tw[k * 16 + n1]);
+            for (int k = 1; k < R2; ++k) v[k] = mulw_cj(v[k], tw[k * 16 + n1]);
         }
         Dft<R2, -1, T>::run(v);
         if (inv) {
@@ -406,7 +406,7 @@ __global__ void __launch_bounds__(NT, MARCH_ONLY ? 2 : 1) ssfm_adjoint_kernel(co
                 if (inv) {
                     v[0] = cj(v[0]);
 #pragma unroll
-                    for (int k = 1; k < R2; ++k) v[k] = mulw(cj(v[k]), tw[k * 16 + n1]);
+                    for (int k = 1; k < R2; ++k) v[k] = mulw_cj(v[k], tw[k * 16 + n1]);
                 }
                 Dft<R2, -1, T>::run(v);
                 if (inv) {
@@ -476,7 +476,7 @@ __global__ void __launch_bounds__(NT, MARCH_ONLY ? 2 : 1) ssfm_adjoint_kernel(co
                                 const T sy = (T)(fy < N / 2 ? fy : fy - N);
                                 wsum += c * (fxq + dfy2 * (sy * sy));
                                 // conjugate propagator: conj(py) conj(px), via conj(conj(u) py px)
-                                u[k1] = cj(mulw(mulw(cj(u[k1]), py[fy]), px));
+                                u[k1] = cj(mulw(mulw_cj(u[k1], py[fy]), px));
                             }
                         }
                     } else {

@@ -11,9 +11,8 @@
 //
 // The transforms are the four-step FFT of the fused march (ssfm_plain.cuh) with N = 16 R2
 // (R2 = 32 at N = 512): the same digit-reversed frequency order between the passes, the same
-// twiddle and propagator tables, the same per-point arithmetic in the same order.  On a grid
-// side both kernels are built for, the two agree up to where the compiler contracts a
-// multiply and an add into one fused multiply-add differently (a last-bit effect).
+// twiddle and propagator tables, the same per-point arithmetic in the same order with explicit
+// rounding, so on a grid side several marches are built for they give the same bits.
 //
 // Reference counterparts as for the fused march: Solver::SSFM / CWES (src/headers/Solver.h:
 // 267-308) with solverRK4 (:189-264) and diffraction (:153-186, cuFFT, kernelComplexProduct,
@@ -32,10 +31,10 @@ struct MpCfg {
     static constexpr int RNT = RB * 16;                  // row-pass threads: one (row, n1) job each
     static constexpr int CW = SW;                        // columns per column-pass CTA: one 128 B row segment
     static constexpr int CNT = 16 * CW;                  // column-pass threads: one (column, n1) job each
-    static constexpr int RPART = N / RB;                 // row-pass CTAs per instance (power partials)
+    static constexpr int RPART = N / RB;                 // row-pass CTAs per instance
     // (FP32: plus the packed RK4 stage constants of the two steps, 6 Rk4Pack)
     static constexpr size_t row_smem = sizeof(cx<T>) * (2 * (size_t)RB * N + 12) + sizeof(mult<T>) * N +
-                                       sizeof(double) * 2 * (RNT / 32) + (sizeof(T) == 4 ? 6 * sizeof(Rk4Pack) : 0);
+                                       (sizeof(T) == 4 ? 6 * sizeof(Rk4Pack) : 0);
     static constexpr size_t col_smem = sizeof(cx<T>) * (size_t)N * CW + sizeof(mult<T>) * (2 * (size_t)N + CW);
     // The thermal row pass gives each (row, n1) job several threads in its pointwise work (the
     // RK4 half steps with per-voxel coefficients, by far its longest part): a single instance
@@ -43,9 +42,6 @@ struct MpCfg {
     // in FP32 (the kernel fits the 128 registers of a 512-thread block), two in FP64.
     __host__ __device__ static constexpr int row_px(bool therm) { return therm ? (sizeof(T) == 4 ? 4 : 2) : 1; }
     __host__ __device__ static constexpr int row_threads(bool therm) { return RNT * row_px(therm); }
-    __host__ __device__ static constexpr size_t row_smem_for(bool therm) {
-        return row_smem + sizeof(double) * 2 * (RNT / 32) * (row_px(therm) - 1);
-    }
     static_assert(N % 16 == 0 && RB * RPART == N && N % CW == 0, "bad multi-pass split");
 };
 
@@ -68,7 +64,7 @@ __host__ __device__ inline MpLayout mp_layout(char* base, int max_steps, bool th
     L.off_s = up(plane);
     L.off_tab = L.off_s + up(plane);
     L.off_part = L.off_tab + up(sizeof(mult<T>) * 5 * (size_t)N);
-    L.off_dk = L.off_part + up(sizeof(double) * 2 * Cfg::RPART);
+    L.off_dk = L.off_part + up(sizeof(double) * 2 * N);
     L.off_zs = L.off_dk + (thermal ? up(sizeof(double) * (size_t)N * N) : 0);
     L.stride = L.off_zs + up(sizeof(double) * ((size_t)max_steps + 1));
     return L;
@@ -101,7 +97,7 @@ __device__ __forceinline__ void r2_stage(cx<T> (&v)[R2], const mult<T>* tw, int 
     if (inv) {
         v[0] = cj(v[0]);
 #pragma unroll
-        for (int k = 1; k < R2; ++k) v[k] = mulw(cj(v[k]), tw[k * 16 + n1]);
+        for (int k = 1; k < R2; ++k) v[k] = mulw_cj(v[k], tw[k * 16 + n1]);
     }
     Dft<R2, -1, T>::run(v);
     if (inv) {
@@ -150,12 +146,11 @@ __global__ void __launch_bounds__(MpCfg<T, N>::row_threads(THERM))
     V* Ss = Ps + RB * N;
     V* coef = Ss + RB * N;  // [0..5] step s, [6..11] step s+1
     W* tw = reinterpret_cast<W*>(coef + 12);
-    double* red = reinterpret_cast<double*>(tw + N);
     const int tid = threadIdx.x, y0 = blockIdx.x * RB;
     auto cj = [](V a) { return mk<T>(a.x, -a.y); };
-    // FP32 plain: packed RK4 stage constants [2][3] (steps s, s + 1), after the reduction area
+    // FP32 plain: packed RK4 stage constants [2][3] (steps s, s + 1)
     constexpr bool PACK = !THERM && sizeof(T) == 4;
-    Rk4Pack* kpk = reinterpret_cast<Rk4Pack*>(red + 2 * (NT / 32));
+    Rk4Pack* kpk = reinterpret_cast<Rk4Pack*>(tw + N);
 
     if constexpr (THERM) {
         // step s reads slices s and s + 1 of the per-voxel optics; slice s + 1 is cold in
@@ -231,7 +226,6 @@ __global__ void __launch_bounds__(MpCfg<T, N>::row_threads(THERM))
     }
 
     const T hap = (T)d.hap, has = (T)d.has, qs = (T)d.qs, dz6 = (T)(d.dz / 6.0);
-    double acc_s = 0.0, acc_p = 0.0;
     {
         // one (row, n1) job per JOBS threads; its R2 stages on the job's first thread, its
         // points shared by the job's PX threads (point k on thread part = k mod PX)
@@ -289,11 +283,9 @@ __global__ void __launch_bounds__(MpCfg<T, N>::row_threads(THERM))
             if (k + PX < R2) nxt = pre_of(k + PX);
             V p = Ps[o], q = Ss[o];
             boundary_point<T, THERM>(d, mode, s, g, (size_t)N * N, p, q, coef, coef + 6, hap, has, qs, dz6,
-                                     THERM ? dkint + g : nullptr, acc_s, acc_p, cur);
-            if (mode != 2) {
-                Ps[o] = p;
-                Ss[o] = q;
-            }
+                                     THERM ? dkint + g : nullptr, cur);
+            Ps[o] = p;
+            Ss[o] = q;
         }
         if constexpr (PX > 1) __syncthreads();
 #pragma unroll 1
@@ -308,29 +300,12 @@ __global__ void __launch_bounds__(MpCfg<T, N>::row_threads(THERM))
         }
     }
     __syncthreads();
-    if (s + 1 == d.out_after) {
-        // the pass that wrote the outputs (the last step of a plain run, the one before the
-        // last of a thermal run): this CTA's share of the SH and pump power sums,
-        // block-reduced in a fixed order
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            acc_s += __shfl_down_sync(0xffffffffu, acc_s, o);
-            acc_p += __shfl_down_sync(0xffffffffu, acc_p, o);
-        }
-        if ((tid & 31) == 0) {
-            red[2 * (tid >> 5)] = acc_s;
-            red[2 * (tid >> 5) + 1] = acc_p;
-        }
-        __syncthreads();
-        if (tid == 0) {
-            double a = 0.0, b = 0.0;
-            for (int w = 0; w < NT / 32; ++w) {
-                a += red[2 * w];
-                b += red[2 * w + 1];
-            }
-            double* part = reinterpret_cast<double*>(wbase + L.off_part);
-            part[2 * blockIdx.x] = a;
-            part[2 * blockIdx.x + 1] = b;
+    if (!THERM && mode == 2) {
+        // the last step of a plain run wrote the outputs: the rows' sums of |S|^2 and |P|^2
+        double* part = reinterpret_cast<double*>(wbase + L.off_part);
+        for (int r = tid >> 5; r < 2 * RB; r += NT / 32) {
+            const double a = row_abs2<T, N>(r < RB ? Ss : Ps, r % RB, tid & 31);
+            if ((tid & 31) == 0) part[(r < RB ? 0 : N) + y0 + r % RB] = a;
         }
     }
     if (mode != 2) {
@@ -422,19 +397,16 @@ __global__ void __launch_bounds__(MpCfg<T, N>::CNT)
     }
 }
 
-// SH and pump power of each instance from its row-pass partials, summed in a fixed order.
+// SH and pump power of each plain instance from its row sums (one warp).
 template <typename T, int N>
 __global__ void mp_power_kernel(const InstDesc* __restrict__ descs, MpLayout L) {
     const InstDesc& d = descs[blockIdx.x];
-    if (threadIdx.x != 0 || !d.power_out) return;
+    if (!d.power_out) return;
     const double* part = reinterpret_cast<const double*>(L.base + (size_t)blockIdx.x * L.stride + L.off_part);
-    double a = 0.0, b = 0.0;
-    for (int r = 0; r < MpCfg<T, N>::RPART; ++r) {
-        a += part[2 * r];
-        b += part[2 * r + 1];
+    for (int f = 0; f < 2; ++f) {
+        const double a = sum_rows<N>([&](int y) { return part[f * N + y]; }, threadIdx.x);
+        if (threadIdx.x == 0) d.power_out[f] = a * (f ? d.pw_p : d.pw_s);
     }
-    d.power_out[0] = a * d.pw_s;
-    d.power_out[1] = b * d.pw_p;
 }
 
 }  // namespace shg

@@ -51,7 +51,7 @@ struct PlainCfg {
     static constexpr int PLANE = RL * N;       // complex elements per field per CTA
     static_assert(N % 16 == 0 && 16 % C == 0 && RL * C == N, "bad grid / cluster split");
     // dynamic shared memory: P, S planes, twiddles + 4 propagator vectors (multiplier
-    // tables), 2x6 coefficients, reduction scratch
+    // tables), 2x6 coefficients, reduction scratch (adjoint)
     // (thermal: plus the running Δk prefix of this CTA's points, FP64)
     // (plain FP32: plus the packed RK4 stage constants, 2 steps x 3 phases of Rk4Pack)
     static constexpr size_t smem_bytes = sizeof(cx<T>) * (2 * (size_t)PLANE + 12) + sizeof(mult<T>) * 5 * (size_t)N +
@@ -72,13 +72,12 @@ __device__ __forceinline__ int sidx(int lr, int p) {
 template <typename T>
 __device__ __forceinline__ void dadz(cx<T> p, cx<T> s, cx<T> cP, cx<T> cS, T hap, T has, T qs, cx<T>& dp,
                                      cx<T>& ds) {
-    cx<T> sp = mulc<T>(s, p);
-    cx<T> tp = mul<T>(cP, sp);
-    dp = mk<T>(tp.x - hap * p.x, tp.y - hap * p.y);
-    cx<T> pp = mk<T>(p.x * p.x - p.y * p.y, (T)2 * p.x * p.y);
-    cx<T> ts = mul<T>(cS, pp);
-    T g = has + qs * (s.x * s.x + s.y * s.y);
-    ds = mk<T>(ts.x - g * s.x, ts.y - g * s.y);
+    const cx<T> tp = mul<T>(cP, mulc<T>(s, p));
+    dp = mk<T>(fma_r(-hap, p.x, tp.x), fma_r(-hap, p.y, tp.y));
+    const cx<T> pp = mk<T>(fma_r(p.x, p.x, mul_r(-p.y, p.y)), mul_r(add_r(p.x, p.x), p.y));
+    const cx<T> ts = mul<T>(cS, pp);
+    const T g = fma_r(qs, fma_r(s.x, s.x, mul_r(s.y, s.y)), has);
+    ds = mk<T>(fma_r(-g, s.x, ts.x), fma_r(-g, s.y, ts.y));
 }
 
 // One application of the reference's RK4 scheme (Solver.h:231-259): stage inputs
@@ -87,30 +86,28 @@ __device__ __forceinline__ void dadz(cx<T> p, cx<T> s, cx<T> cP, cx<T> cS, T hap
 // phases, cf[3..5] = cS.
 template <typename T>
 __device__ __forceinline__ void rk4_point(cx<T>& P, cx<T>& S, const cx<T>* cf, T hap, T has, T qs, T dz6) {
-    cx<T> p = P, s = S, kp, ks, ap, as;
+    // v + h k, component by component
+    auto axpy = [](cx<T> v, T h, cx<T> k) { return mk<T>(fma_r(h, k.x, v.x), fma_r(h, k.y, v.y)); };
+    const cx<T> p = P, s = S;
+    cx<T> kp, ks;
     dadz<T>(p, s, cf[0], cf[3], hap, has, qs, kp, ks);
-    ap = kp; as = ks;
-    dadz<T>(mk<T>(p.x + (T)0.5 * kp.x, p.y + (T)0.5 * kp.y), mk<T>(s.x + (T)0.5 * ks.x, s.y + (T)0.5 * ks.y), cf[1],
-            cf[4], hap, has, qs, kp, ks);
-    ap = mk<T>(ap.x + (T)2 * kp.x, ap.y + (T)2 * kp.y);
-    as = mk<T>(as.x + (T)2 * ks.x, as.y + (T)2 * ks.y);
-    dadz<T>(mk<T>(p.x + (T)0.5 * kp.x, p.y + (T)0.5 * kp.y), mk<T>(s.x + (T)0.5 * ks.x, s.y + (T)0.5 * ks.y), cf[1],
-            cf[4], hap, has, qs, kp, ks);
-    ap = mk<T>(ap.x + (T)2 * kp.x, ap.y + (T)2 * kp.y);
-    as = mk<T>(as.x + (T)2 * ks.x, as.y + (T)2 * ks.y);
+    cx<T> ap = kp, as = ks;
+#pragma unroll
+    for (int st = 0; st < 2; ++st) {
+        dadz<T>(axpy(p, (T)0.5, kp), axpy(s, (T)0.5, ks), cf[1], cf[4], hap, has, qs, kp, ks);
+        ap = axpy(ap, (T)2, kp);
+        as = axpy(as, (T)2, ks);
+    }
     dadz<T>(add<T>(p, kp), add<T>(s, ks), cf[2], cf[5], hap, has, qs, kp, ks);
-    ap = add<T>(ap, kp);
-    as = add<T>(as, ks);
-    P = mk<T>(p.x + ap.x * dz6, p.y + ap.y * dz6);
-    S = mk<T>(s.x + as.x * dz6, s.y + as.y * dz6);
+    P = axpy(p, dz6, add<T>(ap, kp));
+    S = axpy(s, dz6, add<T>(as, ks));
 }
 
 // Two points of the FP32 RK4 at once in packed two-lane arithmetic (sm_100 f32x2): the real
 // parts of the two points share one register pair, the imaginary parts another, and each
 // packed instruction does the work of two scalar ones.  The per-phase stage constants are
 // held with each value in both lanes (Rk4Pack, written by stage_pack).  The operations and
-// their order are those of dadz / rk4_point; only where the compiler would choose to fuse
-// a multiply into an add is fixed here.
+// their order are those of dadz / rk4_point, but for which product of a sum is fused.
 struct Cx2 {
     float2 r, i;
 };
@@ -190,7 +187,7 @@ __device__ __forceinline__ void stage_pack(const float2* cf, int j, Rk4Pack* kp)
 template <typename T>
 __device__ __forceinline__ void stage_coef(const InstDesc& d, int s, double z, int j, cx<T>* cf) {
     const double inc = j == 0 ? 0.0 : (j == 1 ? 0.25 : 0.5);
-    const double phi = (z + d.dz * inc) * d.dk + (d.poling ? d.poling[s] : 0.0);
+    const double phi = fma_r(fma_r(d.dz, inc, z), d.dk, d.poling ? d.poling[s] : 0.0);
     double sn, cs;
     sincos(phi, &sn, &cs);
     // i κ e^{-iφ} = κ (sin φ, cos φ);  i κ e^{+iφ} = κ (-sin φ, cos φ)
@@ -198,35 +195,44 @@ __device__ __forceinline__ void stage_coef(const InstDesc& d, int s, double z, i
     cf[3 + j] = mk<T>((T)(-d.kap_s * sn), (T)(d.kap_s * cs));
 }
 
-// Multiplier tables of one instance: twiddles tw[k*16 + n1] = W_N^{n1 k}; the x factors of
-// the pump / SH propagators by physical column position (frequency perm(j) = (j>>4) +
-// R2*(j&15)); the y factors by frequency with the 1/(NX*NY) of the inverse FFT folded in.
-// Propagator phase θ = -dz (a (dfx^2 sx^2 + dfy^2 sy^2) + b sx) (Efields.h:122-141) with the
-// fftshift of Efields.h:32-81 expressed through signed frequency indices.
+// Multiplier tables of one instance, entry by entry: twiddles tw[k*16 + n1] = W_N^{n1 k}; the
+// x factors of the pump / SH propagators by physical column position (frequency perm(j) =
+// (j>>4) + R2*(j&15)); the y factors by frequency with the 1/(NX*NY) of the inverse FFT folded
+// in.  Propagator phase θ = -dz (a (dfx^2 sx^2 + dfy^2 sy^2) + b sx) (Efields.h:122-141) with
+// the fftshift of Efields.h:32-81 expressed through signed frequency indices.
+template <typename T, int N>
+__device__ __forceinline__ mult<T> twiddle(int j) {
+    double sn, cs;
+    sincospi(-2.0 * (double)((j & 15) * (j >> 4)) / (double)N, &sn, &cs);
+    return make_mult<T>(cs, sn);
+}
+template <typename T, int N>
+__device__ __forceinline__ mult<T> prop_x(const InstDesc& d, double a, double b, int j) {
+    const int fx = (j >> 4) + (N / 16) * (j & 15);
+    const double sx = (double)(fx < N / 2 ? fx : fx - N);
+    const double th = mul_r(-d.dz, fma_r(a, mul_r(mul_r(d.dfx, d.dfx), sx * sx), mul_r(b, sx)));
+    double sn, cs;
+    sincos(th, &sn, &cs);
+    return make_mult<T>(cs, sn);
+}
+template <typename T, int N>
+__device__ __forceinline__ mult<T> prop_y(const InstDesc& d, double a, int j) {
+    const double sy = (double)(j < N / 2 ? j : j - N);
+    const double inv = 1.0 / ((double)N * (double)N);
+    const double th = mul_r(-d.dz, mul_r(a, mul_r(mul_r(d.dfy, d.dfy), sy * sy)));
+    double sn, cs;
+    sincos(th, &sn, &cs);
+    return make_mult<T>(mul_r(cs, inv), mul_r(sn, inv));
+}
 template <typename T, int N>
 __device__ __forceinline__ void init_tables(const InstDesc& d, mult<T>* tw, mult<T>* pxp, mult<T>* pxs, mult<T>* pyp,
                                             mult<T>* pys, int tid, int nt) {
-    constexpr int R2 = N / 16;
     for (int j = tid; j < N; j += nt) {
-        double sn, cs;
-        sincospi(-2.0 * (double)((j & 15) * (j >> 4)) / (double)N, &sn, &cs);
-        tw[j] = make_mult<T>(cs, sn);
-        const int fx = (j >> 4) + R2 * (j & 15);
-        const double sx = (double)(fx < N / 2 ? fx : fx - N);
-        const double thxp = -d.dz * (d.a_p * (d.dfx * d.dfx * (sx * sx)) + d.b_p * sx);
-        const double thxs = -d.dz * (d.a_s * (d.dfx * d.dfx * (sx * sx)) + d.b_s * sx);
-        sincos(thxp, &sn, &cs);
-        pxp[j] = make_mult<T>(cs, sn);
-        sincos(thxs, &sn, &cs);
-        pxs[j] = make_mult<T>(cs, sn);
-        const double sy = (double)(j < N / 2 ? j : j - N);
-        const double inv = 1.0 / ((double)N * (double)N);
-        const double thyp = -d.dz * (d.a_p * (d.dfy * d.dfy * (sy * sy)));
-        const double thys = -d.dz * (d.a_s * (d.dfy * d.dfy * (sy * sy)));
-        sincos(thyp, &sn, &cs);
-        pyp[j] = make_mult<T>(cs * inv, sn * inv);
-        sincos(thys, &sn, &cs);
-        pys[j] = make_mult<T>(cs * inv, sn * inv);
+        tw[j] = twiddle<T, N>(j);
+        pxp[j] = prop_x<T, N>(d, d.a_p, d.b_p, j);
+        pxs[j] = prop_x<T, N>(d, d.a_s, d.b_s, j);
+        pyp[j] = prop_y<T, N>(d, d.a_p, j);
+        pys[j] = prop_y<T, N>(d, d.a_s, j);
     }
 }
 
@@ -235,26 +241,24 @@ __device__ __forceinline__ void init_tables(const InstDesc& d, mult<T>* tw, mult
 // the separable variant amp * exp(-ax^2 / (wX2 MX) - ay^2 / (wY2 MY)) (Efields.h:113-115).
 __device__ __forceinline__ double2 pump_value(const InstDesc& d, int x, int y, double amp_re, double amp_im,
                                               double den_re, double den_im) {
-    const double ax = ((double)x - d.ux) * d.dx, ay = ((double)y - d.uy) * d.dy;
+    const double ax = mul_r((double)x - d.ux, d.dx), ay = mul_r((double)y - d.uy, d.dy);
+    const double ax2 = mul_r(ax, ax), ay2 = mul_r(ay, ay);
+    const double dd = fma_r(den_re, den_re, mul_r(den_im, den_im));
+    double are, aim;
     if (d.elliptic) {
-        const double dx2 = den_re * den_re + den_im * den_im;
-        const double dy2 = d.deny_re * d.deny_re + d.deny_im * d.deny_im;
-        const double are = -(ax * ax) * den_re / dx2 - (ay * ay) * d.deny_re / dy2;
-        const double aim = (ax * ax) * den_im / dx2 + (ay * ay) * d.deny_im / dy2;
-        const double ex = exp(are);
-        double sn, cs;
-        sincos(aim, &sn, &cs);
-        const double er = ex * cs, ei = ex * sn;
-        return make_double2(amp_re * er - amp_im * ei, amp_re * ei + amp_im * er);
+        const double dy2 = fma_r(d.deny_re, d.deny_re, mul_r(d.deny_im, d.deny_im));
+        are = -(mul_r(ax2, den_re) / dd) - mul_r(ay2, d.deny_re) / dy2;
+        aim = mul_r(ax2, den_im) / dd + mul_r(ay2, d.deny_im) / dy2;
+    } else {
+        const double num = fma_r(-ay, ay, -ax2);
+        are = mul_r(num, den_re) / dd;
+        aim = mul_r(-num, den_im) / dd;
     }
-    const double num = -(ax * ax) - (ay * ay);
-    const double dd = den_re * den_re + den_im * den_im;
-    const double are = (num * den_re) / dd, aim = (-num * den_im) / dd;
     const double ex = exp(are);
     double sn, cs;
     sincos(aim, &sn, &cs);
-    const double er = ex * cs, ei = ex * sn;
-    return make_double2(amp_re * er - amp_im * ei, amp_re * ei + amp_im * er);
+    const double er = mul_r(ex, cs), ei = mul_r(ex, sn);
+    return make_double2(fma_r(amp_re, er, mul_r(-amp_im, ei)), fma_r(amp_re, ei, mul_r(amp_im, er)));
 }
 
 // Caller buffers of an instance (signal_in, outputs, slices) hold complex values of the
@@ -283,38 +287,60 @@ __device__ __forceinline__ cx<T> get_field(const InstDesc& d, const void* base, 
 
 // Thermal stage coefficients at one voxel (Solver.h:33-55): κ = kf / n(λ, T(x,y,s)) and the
 // phase DKint (dz inc + s dz) / (s + 1), DKint the running sum of Δk over slices 0..s
-// (PhaseMatching.h:27-44), in FP64.
+// (PhaseMatching.h:27-44), in FP64.  thermal_phase gives the cosine (x) and sine (y) of the three
+// phases, which depend on the voxel and slice alone; thermal_cf the coefficients.
 template <typename T>
-__device__ __forceinline__ void thermal_coef(const InstDesc& d, double dki, int sl, double np, double ns, cx<T>* cf) {
+__device__ __forceinline__ void thermal_phase(const InstDesc& d, double dki, int sl, cx<T>* cs3) {
     const double sr = (double)sl, b = sr + 1.0;
-    if constexpr (sizeof(T) == 4) {
-        // FP32 run: the phases (up to hundreds of radians) and their reduction to [-π, π] in
-        // FP64, then sine, cosine and κ/n in FP32, accurate to the float rounding the
-        // coefficients get anyway; one FP64 division instead of five and no FP64 sincos
-        const double q = dki / b, two_pi = 6.283185307179586476925, inv_two_pi = 0.159154943091895335769;
-        const float kp = (float)d.kf_p / (float)np, ks = (float)d.kf_s / (float)ns;
+    // FP32 run: the phases (up to hundreds of radians) and their reduction to [-π, π] in FP64,
+    // then sine and cosine in FP32, accurate to the float rounding the coefficients get anyway;
+    // one FP64 division instead of three and no FP64 sincos
+    const double q = sizeof(T) == 4 ? dki / b : 0.0;
 #pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            const double inc = j == 0 ? 0.0 : (j == 1 ? 0.25 : 0.5);
-            const double phi = q * (d.dz * inc + sr * d.dz);
-            const float r = (float)fma(-two_pi, rint(phi * inv_two_pi), phi);
-            float sn, cs;
-            sincosf(r, &sn, &cs);
-            cf[j] = mk<T>(kp * sn, kp * cs);
-            cf[3 + j] = mk<T>(-ks * sn, ks * cs);
+    for (int j = 0; j < 3; ++j) {
+        const double inc = j == 0 ? 0.0 : (j == 1 ? 0.25 : 0.5);
+        const double zj = fma_r(sr, d.dz, mul_r(d.dz, inc));
+        T sn, cs;
+        if constexpr (sizeof(T) == 4) {
+            const double two_pi = 6.283185307179586476925, inv_two_pi = 0.159154943091895335769;
+            const double phi = mul_r(q, zj);
+            sincosf((float)fma_r(-two_pi, rint(mul_r(phi, inv_two_pi)), phi), &sn, &cs);
+        } else {
+            sincos(mul_r(dki, zj) / b, &sn, &cs);
         }
-    } else {
-        const double kp = d.kf_p / np, ks = d.kf_s / ns;
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            const double inc = j == 0 ? 0.0 : (j == 1 ? 0.25 : 0.5);
-            const double phi = dki * (d.dz * inc + sr * d.dz) / b;
-            double sn, cs;
-            sincos(phi, &sn, &cs);
-            cf[j] = mk<T>((T)(kp * sn), (T)(kp * cs));
-            cf[3 + j] = mk<T>((T)(-ks * sn), (T)(ks * cs));
-        }
+        cs3[j] = mk<T>(cs, sn);
     }
+}
+template <typename T>
+__device__ __forceinline__ void thermal_cf(const InstDesc& d, T np, T ns, const cx<T>* cs3, cx<T>* cf) {
+    const T kp = (T)d.kf_p / np, ks = (T)d.kf_s / ns;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        cf[j] = mk<T>(mul_r(kp, cs3[j].y), mul_r(kp, cs3[j].x));
+        cf[3 + j] = mk<T>(mul_r(-ks, cs3[j].y), mul_r(ks, cs3[j].x));
+    }
+}
+template <typename T>
+__device__ __forceinline__ void thermal_coef(const InstDesc& d, double dki, int sl, T np, T ns, cx<T>* cf) {
+    cx<T> cs3[3];
+    thermal_phase<T>(d, dki, sl, cs3);
+    thermal_cf<T>(d, np, ns, cs3, cf);
+}
+// qs of the RK4 stages at one voxel, and kernelSetQ (Tfield.h:260-276) there
+template <typename T>
+__device__ __forceinline__ T thermal_qs(const InstDesc& d, T ns) {
+    return (T)(0.5 * mul_r(d.bf_s, (double)ns));
+}
+template <typename T>
+__device__ __forceinline__ T thermal_q(const InstDesc& d, T np, T ns, cx<T> p, cx<T> q) {
+    const T ap2 = fma_r(p.y, p.y, mul_r(p.x, p.x)), as2 = fma_r(q.y, q.y, mul_r(q.x, q.x));
+    const T is = mul_r(mul_r((T)d.q_h, ns), as2);
+    return fma_r((T)d.beta_s, mul_r(is, is), fma_r(mul_r((T)d.q_s, ns), as2, mul_r(mul_r((T)d.q_p, np), ap2)));
+}
+// |v|^2 with weight w, for the power sums
+template <typename T>
+__device__ __forceinline__ double weighted_abs2(double w, cx<T> v) {
+    return mul_r(w, fma_r((double)v.y, (double)v.y, mul_r((double)v.x, (double)v.x)));
 }
 
 // The per-voxel values a thermal boundary_point reads from global memory, fetched apart from
@@ -355,14 +381,13 @@ __device__ __forceinline__ ThermPre<T> thermal_pre(const InstDesc& d, int mode, 
 // applications around a step boundary, h = 0 the second half of step s and h = 1 the first
 // half of step s+1 (Solver.h:267-273); mode 0 (s = -1, the first pass) runs h = 1 only, mode
 // 2 (the last step) h = 0 only.  With them: the heat source of slice s (thermal), the
-// per-slice record of the fields before step s+1 and the outputs after step out_after with
-// their power sums.  Thermal: pre holds the point's optics and running Δk prefix
+// per-slice record of the fields before step s+1 and the outputs after step out_after
+// (thermal: with their weighted squares).  Thermal: pre holds the point's optics and running Δk prefix
 // (thermal_pre), and dki receives the prefix through slice s + 1.
 template <typename T, bool THERM>
 __device__ __forceinline__ void boundary_point(const InstDesc& d, int mode, int s, size_t g, size_t nn, cx<T>& p,
                                                cx<T>& q, const cx<T>* cf_prev, const cx<T>* cf_next, T hap, T has,
-                                               T qs, T dz6, double* dki, double& acc_s, double& acc_p,
-                                               const ThermPre<T>& pre) {
+                                               T qs, T dz6, double* dki, const ThermPre<T>& pre) {
     using V = cx<T>;
     using R = T;  // real type of the thermal 3D arrays
     const R* tnp = reinterpret_cast<const R*>(d.t_np);
@@ -380,16 +405,11 @@ __device__ __forceinline__ void boundary_point(const InstDesc& d, int mode, int 
                 *dki = dk_run;
             }
             // this half step's optics (selects, so that the rolled loop indexes no array)
-            const double np = (double)(h ? pre.np[1] : pre.np[0]), ns = (double)(h ? pre.ns[1] : pre.ns[0]);
+            const T np = h ? pre.np[1] : pre.np[0], ns = h ? pre.ns[1] : pre.ns[0];
             V cf[6];
             thermal_coef<T>(d, dk_run, sl, np, ns, cf);
-            rk4_point<T>(p, q, cf, hap, has, (T)(0.5 * (d.bf_s * ns)), dz6);
-            if (h == 0 && tq) {
-                // kernelSetQ (Tfield.h:260-276) for slice s, after its step
-                const R ap2 = p.x * p.x + p.y * p.y, as2 = q.x * q.x + q.y * q.y;
-                const R is = (R)d.q_h * (R)ns * as2;
-                tq[gz] = (R)d.q_p * (R)np * ap2 + (R)d.q_s * (R)ns * as2 + (R)d.beta_s * (is * is);
-            }
+            rk4_point<T>(p, q, cf, hap, has, thermal_qs<T>(d, ns), dz6);
+            if (h == 0 && tq) tq[gz] = thermal_q<T>(d, np, ns, p, q);  // slice s, after its step
         } else {
             (void)dki;
             (void)pre;
@@ -404,15 +424,34 @@ __device__ __forceinline__ void boundary_point(const InstDesc& d, int mode, int 
         if (h == 0 && s + 1 == d.out_after) {
             if (d.pump_out) put_field<T>(d, d.pump_out, g, p);
             if (d.signal_out) put_field<T>(d, d.signal_out, g, q);
-            double ws = 1.0, wp = 1.0;
             if constexpr (THERM) {
-                ws = (double)tns[(size_t)(s + 1) * nn + g];
-                wp = (double)tnp[(size_t)(s + 1) * nn + g];
+                d.w_out[g] = weighted_abs2<T>((double)tns[(size_t)(s + 1) * nn + g], q);
+                d.w_out[nn + g] = weighted_abs2<T>((double)tnp[(size_t)(s + 1) * nn + g], p);
             }
-            acc_s += ws * ((double)q.x * (double)q.x + (double)q.y * (double)q.y);
-            acc_p += wp * ((double)p.x * (double)p.x + (double)p.y * (double)p.y);
         }
     }
+}
+
+// Sum of |v|^2 over one row of a plane in shared memory, by a warp: each lane's columns in
+// order, then the lanes by a shuffle tree.  The plain marches add a row's points like this and
+// then the rows like this (sum_rows), so an instance's powers do not depend on the march or on
+// the split that ran it.
+template <typename T, int N>
+__device__ __forceinline__ double row_abs2(const cx<T>* F, int lr, int lane) {
+    constexpr int R2 = N / 16, SW = sizeof(T) == 4 ? 16 : 8;
+    double a = 0.0;
+    for (int x = lane; x < N; x += 32) a = add_r(a, weighted_abs2<T>(1.0, F[sidx<N, R2, SW>(lr, x)]));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a = add_r(a, __shfl_xor_sync(0xffffffffu, a, o));
+    return a;
+}
+template <int N, typename Get>
+__device__ __forceinline__ double sum_rows(Get&& row, int lane) {
+    double a = 0.0;
+    for (int y = lane; y < N; y += 32) a = add_r(a, row(y));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a = add_r(a, __shfl_xor_sync(0xffffffffu, a, o));
+    return a;
 }
 
 // Persistent march: each cluster takes instances from the device work queue *queue (an
@@ -438,8 +477,7 @@ __global__ void __launch_bounds__(NT, MINB)
     W* pxs = pxp + N;            // SH   propagator, x factor
     W* pyp = pxs + N;            // pump propagator, y factor by frequency, × 1/N^2
     W* pys = pyp + N;            // SH   propagator, y factor
-    double* red = reinterpret_cast<double*>(pys + N);  // [2*(NT/32)] + [4]
-    double* dkint = red + 2 * (NT / 32) + 4;           // thermal: [RL*N] running Δk prefix
+    double* dkint = reinterpret_cast<double*>(pys + N) + 2 * (NT / 32) + 4;  // thermal: [RL*N] running Δk prefix
     // plain FP32: packed RK4 stage constants [2][3], in the place of the thermal prefix
     Rk4Pack* kpk = reinterpret_cast<Rk4Pack*>(dkint);
     constexpr bool PACK = !THERM && sizeof(T) == 4;
@@ -506,7 +544,7 @@ __global__ void __launch_bounds__(NT, MINB)
         // RK4(z_{s+1}), forward), 2: last (inverse, RK4(z_s), outputs)
 
         // s: index of the step that ends in this pass (-1 in the first pass)
-        auto pass_ra = [&](int mode, int s, const V* cf_prev, const V* cf_next, double& acc_s, double& acc_p) {
+        auto pass_ra = [&](int mode, int s, const V* cf_prev, const V* cf_next) {
             for (int j = tid; j < JA; j += NT) {
                 const int n1 = j & 15, lr = j >> 4;
 #pragma unroll 1
@@ -557,11 +595,9 @@ __global__ void __launch_bounds__(NT, MINB)
                             double* dkp = THERM ? &dkint[lr * N + x] : nullptr;
                             const ThermPre<T> pre = thermal_pre<T, THERM>(d, mode, s, g, (size_t)N * N, dkp);
                             boundary_point<T, THERM>(d, mode, s, g, (size_t)N * N, p, q, cf_prev, cf_next, hap, has,
-                                                     qs, dz6, dkp, acc_s, acc_p, pre);
-                            if (mode != 2) {
-                                Ps[o] = p;
-                                Ss[o] = q;
-                            }
+                                                     qs, dz6, dkp, pre);
+                            Ps[o] = p;
+                            Ss[o] = q;
                         }
                         continue;
                     }
@@ -574,7 +610,7 @@ __global__ void __launch_bounds__(NT, MINB)
                     if (inv) {
                         v[0] = cj(v[0]);
 #pragma unroll
-                        for (int k = 1; k < R2; ++k) v[k] = mulw(cj(v[k]), tw[k * 16 + n1]);
+                        for (int k = 1; k < R2; ++k) v[k] = mulw_cj(v[k], tw[k * 16 + n1]);
                     }
                     Dft<R2, -1, T>::run(v);
                     if (inv) {
@@ -624,7 +660,7 @@ __global__ void __launch_bounds__(NT, MINB)
                     if (inv) {
                         v[0] = cj(v[0]);
 #pragma unroll
-                        for (int k = 1; k < R2; ++k) v[k] = mulw(cj(v[k]), tw[k * 16 + n1]);
+                        for (int k = 1; k < R2; ++k) v[k] = mulw_cj(v[k], tw[k * 16 + n1]);
                     }
                     Dft<R2, -1, T>::run(v);
                     if (inv) {
@@ -695,8 +731,7 @@ __global__ void __launch_bounds__(NT, MINB)
             else __syncthreads();
         };
 
-        double acc_s = 0.0, acc_p = 0.0;
-        pass_ra(0, -1, coef, coef, acc_s, acc_p);
+        pass_ra(0, -1, coef, coef);
         row_sync();
 
         double z = 0.0;
@@ -717,41 +752,31 @@ __global__ void __launch_bounds__(NT, MINB)
             __syncthreads();
             pass_rb(true);
             row_sync();
-            pass_ra(s + 1 < nsteps ? 1 : 2, s, cf_cur, cf_nxt, acc_s, acc_p);
+            pass_ra(s + 1 < nsteps ? 1 : 2, s, cf_cur, cf_nxt);
             row_sync();
             z += d.dz;
         }
 
-        // ---- SH and pump power: deterministic block + cluster reduction --------------------
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            acc_s += __shfl_down_sync(0xffffffffu, acc_s, o);
-            acc_p += __shfl_down_sync(0xffffffffu, acc_p, o);
-        }
-        const int warp = tid >> 5, lane = tid & 31;
-        if (lane == 0) {
-            red[2 * warp] = acc_s;
-            red[2 * warp + 1] = acc_p;
-        }
-        __syncthreads();
-        double* part = red + 2 * (NT / 32);
-        if (tid == 0) {
-            double a = 0.0, b = 0.0;
-            for (int w = 0; w < NT / 32; ++w) { a += red[2 * w]; b += red[2 * w + 1]; }
-            part[0] = a;
-            part[1] = b;
-        }
-        cluster_sync();
-        if (crank == 0 && tid == 0 && d.power_out) {
-            double a = 0.0, b = 0.0;
-            for (int r = 0; r < C; ++r) {
-                const double* pr = part;
-                if constexpr (C > 1) pr = cg::this_cluster().map_shared_rank(part, r);
-                a += pr[0];
-                b += pr[1];
+        // ---- SH and pump power: row sums (in the twiddles' place), then the rows ------------
+        if constexpr (!THERM) {
+            double* rows = reinterpret_cast<double*>(tw);  // [2][RL]: SH, pump
+            const int warp = tid >> 5, lane = tid & 31;
+            __syncthreads();
+            for (int r = warp; r < 2 * Cfg::RL; r += NT / 32) {
+                const double a = row_abs2<T, N>(r < Cfg::RL ? Ss : Ps, r % Cfg::RL, lane);
+                if (lane == 0) rows[r] = a;
             }
-            d.power_out[0] = a * d.pw_s;
-            d.power_out[1] = b * d.pw_p;
+            cluster_sync();
+            if (crank == 0 && warp == 0 && d.power_out) {
+                for (int f = 0; f < 2; ++f) {
+                    const double a = sum_rows<N>([&](int y) {
+                        const double* pr = rows;
+                        if constexpr (C > 1) pr = cg::this_cluster().map_shared_rank(rows, y % C);
+                        return pr[f * Cfg::RL + y / C];
+                    }, lane);
+                    if (lane == 0) d.power_out[f] = a * (f ? d.pw_p : d.pw_s);
+                }
+            }
         }
         cluster_sync();
         if (!queue) break;

@@ -42,13 +42,18 @@ const PlainVariant* find_plain_variant(int precision, int n, int thermal, int ma
     });
     if (march == SHG_MARCH_FUSED) return fused;
     if (march == SHG_MARCH_MULTIPASS) return multi;
-    // automatic: a thermal run marches on the multi-pass kernels where they are built.  One
-    // thermal instance's fused cluster holds 1-16 SMs for every optical pass, which lies on the
-    // run's critical path between two heat solves; the multi-pass launches spread each step
-    // over the GPU (the optical passes of a 128 x 128 x 200 FP64 run: 47.6 -> 21.3 ms).  Plain runs, which
-    // come in batches that fill the GPU with clusters, keep the fused march.
+    // automatic, for batches too large for the wide march (wide_variant_for): thermal runs on
+    // the multi-pass kernels where they are built, whose launches spread each step over the GPU;
+    // plain runs, which fill it with clusters, on the fused march
     if (th && multi) return multi;
     return fused ? fused : multi;
+}
+
+bool has_plain_choice(int precision, int n, int thermal) {
+    std::lock_guard<std::mutex> lk(g_mu);
+    for (const PlainVariant* v : g_chosen)
+        if (v->precision == precision && v->n == n && v->thermal == (thermal ? 1 : 0)) return true;
+    return false;
 }
 
 int plain_candidates(int precision, int n, const PlainVariant** out, int max) {

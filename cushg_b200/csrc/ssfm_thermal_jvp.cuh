@@ -100,7 +100,7 @@ __device__ __forceinline__ void thermal_coef_jvp(const InstDesc& d, double dki, 
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
             const double inc = j == 0 ? 0.0 : (j == 1 ? 0.25 : 0.5);
-            const double zj = d.dz * inc + sr * d.dz;
+            const double zj = fma_r(sr, d.dz, mul_r(d.dz, inc));
             const double phi = q * zj;
             const float r = (float)fma(-two_pi, rint(phi * inv_two_pi), phi);
             const float phid = (float)(qd * zj);
@@ -118,7 +118,7 @@ __device__ __forceinline__ void thermal_coef_jvp(const InstDesc& d, double dki, 
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
         const double inc = j == 0 ? 0.0 : (j == 1 ? 0.25 : 0.5);
-        const double w = (d.dz * inc + sr * d.dz) / b;
+        const double w = fma_r(sr, d.dz, mul_r(d.dz, inc)) / b;
         const double phi = dki * w, phid = dkid * w;
         double sn, cs;
         sincos(phi, &sn, &cs);

@@ -33,7 +33,8 @@ struct PlainVariant {
     int thermal;    // 1: thermal pass (per-voxel optics, Q emission)
     size_t smem;    // dynamic shared memory per CTA (multi-pass: of the row pass)
     PlainLaunch launch;  // fused cluster march, or null
-    MpLaunch mp;         // multi-pass march, or null
+    MpLaunch mp;         // multi-pass or wide march, or null
+    cudaError_t (*fit)(int* instances) = nullptr;  // wide march: instances resident at once
 };
 
 // Run `count` instances through variant v (either kind); queue as for PlainLaunch.
@@ -62,6 +63,11 @@ VariantTable variants_multipass();
 // (the first compiled fused variant, else the multi-pass one); fused / multi-pass = the
 // default of that kind.  Null if none is built.
 const PlainVariant* find_plain_variant(int precision, int n, int thermal = 0, int march = 0);
+// The wide march (ssfm_wide.cuh) of (precision, n, thermal) if it is the faster one for `count`
+// runs of one class that have the device to themselves, else null.
+const PlainVariant* wide_variant_for(int precision, int n, int thermal, int count);
+// Whether a tuner or shg_set_schedule chose a variant for (precision, n, thermal).
+bool has_plain_choice(int precision, int n, int thermal);
 // Every compiled plain variant of (precision, n), default first; returns how many.
 int plain_candidates(int precision, int n, const PlainVariant** out, int max);
 // Make v the variant find_plain_variant returns for its (precision, n, thermal).

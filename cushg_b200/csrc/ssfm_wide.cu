@@ -1,0 +1,109 @@
+// ssfm_wide.cu — variants and launch of the wide march (ssfm_wide.cuh).
+#include <cuda_runtime.h>
+
+#include "shg_host.h"
+#include "ssfm_variants.h"
+#include "ssfm_wide.cuh"
+
+namespace shg {
+
+namespace {
+
+// Kernel attributes, once per device, and the instances that fit on the device at once.
+template <typename T, int N, bool THERM>
+cudaError_t wide_fit(int* instances) {
+    using Cfg = WideCfg<T, N, THERM>;
+    auto kern = ssfm_wide_kernel<T, N, THERM>;
+    static PerDevice<int> state;
+    return state.get(
+        [&](int dev, int& res) {
+            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::smem_bytes);
+            int sms = 0, per_sm = 0;
+            if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+            if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, Cfg::NT, Cfg::smem_bytes);
+            res = sms * per_sm / Cfg::G;
+            return e == cudaSuccess && res < 1 ? cudaErrorCooperativeLaunchTooLarge : e;
+        },
+        instances);
+}
+
+template <typename T, int N, bool THERM>
+cudaError_t wide_march(const InstDesc* dev_descs, const InstDesc*, int count, cudaStream_t s) {
+    using Cfg = WideCfg<T, N, THERM>;
+    auto kern = ssfm_wide_kernel<T, N, THERM>;
+    int fit = 0;
+    const cudaError_t attr_err = wide_fit<T, N, THERM>(&fit);
+    if (attr_err != cudaSuccess) return attr_err;
+    if (count <= 0) return cudaSuccess;
+    auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
+    const size_t plane = up(sizeof(cx<T>) * (size_t)N * N);
+    WideWs ws;
+    ws.off_s = plane;
+    ws.off_part = 2 * plane;
+    ws.stride = 2 * plane + up(sizeof(double) * 2 * N);
+    ws.limit_ns = 2000000000ull;
+    const int batch = count < fit ? count : fit;
+    char* buf = nullptr;
+    const size_t bars = up(sizeof(unsigned) * 2 * (size_t)count);
+    cudaError_t e = dev_alloc((void**)&buf, bars + ws.stride * (size_t)batch, s);
+    if (e != cudaSuccess) return e;
+    ws.base = buf + bars;
+    e = cudaMemsetAsync(buf, 0, bars, s);
+    for (int i = 0; i < count && e == cudaSuccess; i += batch) {
+        ws.bar = reinterpret_cast<unsigned*>(buf) + 2 * (size_t)i;
+        const InstDesc* dd = dev_descs + i;
+        void* args[] = {&dd, &ws};
+        e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kern),
+                                        dim3(Cfg::G, (unsigned)(count - i < batch ? count - i : batch)), dim3(Cfg::NT), args,
+                                        Cfg::smem_bytes, s);
+    }
+    const cudaError_t ef = cudaFreeAsync(buf, s);
+    return e != cudaSuccess ? e : ef;
+}
+
+#define SHG_WIDE_VARIANT(T, PREC, N, THERM)                                                                          \
+    {PREC, N, 0, WideCfg<T, N, THERM>::NT, 1, THERM ? 1 : 0, WideCfg<T, N, THERM>::smem_bytes, nullptr, &wide_march<T, N, THERM>, \
+     &wide_fit<T, N, THERM>}
+
+const PlainVariant kTable[] = {
+    SHG_WIDE_VARIANT(float, 32, 32, false),  SHG_WIDE_VARIANT(float, 32, 48, false),
+    SHG_WIDE_VARIANT(double, 64, 32, false), SHG_WIDE_VARIANT(double, 64, 48, false),
+    SHG_WIDE_VARIANT(float, 32, 64, false),  SHG_WIDE_VARIANT(float, 32, 96, false),  SHG_WIDE_VARIANT(float, 32, 128, false),
+    SHG_WIDE_VARIANT(float, 32, 192, false), SHG_WIDE_VARIANT(float, 32, 256, false), SHG_WIDE_VARIANT(float, 32, 512, false),
+    SHG_WIDE_VARIANT(double, 64, 64, false), SHG_WIDE_VARIANT(double, 64, 96, false), SHG_WIDE_VARIANT(double, 64, 128, false),
+    SHG_WIDE_VARIANT(double, 64, 192, false), SHG_WIDE_VARIANT(double, 64, 256, false), SHG_WIDE_VARIANT(double, 64, 512, false),
+    SHG_WIDE_VARIANT(float, 32, 32, true),   SHG_WIDE_VARIANT(float, 32, 64, true),   SHG_WIDE_VARIANT(float, 32, 128, true),
+    SHG_WIDE_VARIANT(float, 32, 256, true),  SHG_WIDE_VARIANT(float, 32, 512, true),
+    SHG_WIDE_VARIANT(double, 64, 32, true),  SHG_WIDE_VARIANT(double, 64, 64, true),  SHG_WIDE_VARIANT(double, 64, 128, true),
+    SHG_WIDE_VARIANT(double, 64, 256, true), SHG_WIDE_VARIANT(double, 64, 512, true),
+};
+
+}  // namespace
+
+// When the wide march pays.  It takes the whole device for `fit` instances at a time, so its
+// time grows with the rounds of `fit`; the fused march's grows only when its clusters no longer
+// fit side by side, the multi-pass march's slowly with the count.  Measured per step (us), wide
+// against the march a batch takes (fused, or multi-pass for thermal sides 128-512 and 512):
+//   one plain run      FP32: 64 5.0 / 13.5, 128 5.6 / 29.1, 192 6.6 / 36.8, 256 7.7 / 20.5,
+//                      512 14.4 / 34.4; FP64: 64 5.4 / 14.8, 128 5.9 / 18.2, 256 9.0 / 33.8,
+//                      512 19.0 / 41.6
+//   thermal, 2 rounds  FP32: 64 x 16 21.4 / 40.6, 128 x 8 20.8 / 22.5, 256 x 4 26.0 / 30.7;
+//                      FP64: 64 x 16 23.3 / 56.8, 128 x 8 23.8 / 28.9, 256 x 4 33.7 / 45.8
+//   thermal, 4 rounds  FP32: 128 x 16 50.3 / 37.0, 256 x 8 51.0 / 52.7 (no longer)
+//   thermal at 512     FP32: 1 21.1 / 46.2, 4 83.6 / 87.1, 8 167 / 189; FP64: 1 32.4 / 56.6,
+//                      8 259 / 289 (at any count: both grow linearly)
+const PlainVariant* wide_variant_for(int precision, int n, int thermal, int count) {
+    for (const PlainVariant& v : kTable) {
+        if (v.precision != precision || v.n != n || v.thermal != (thermal ? 1 : 0)) continue;
+        int fit = 0;
+        if (v.fit(&fit) != cudaSuccess) {
+            cudaGetLastError();  // the device cannot hold the launch: the other marches can
+            return nullptr;
+        }
+        const int rounds = (count + fit - 1) / fit;
+        return rounds <= (thermal ? 2 : 1) || (thermal && n == 512) ? &v : nullptr;
+    }
+    return nullptr;
+}
+
+}  // namespace shg

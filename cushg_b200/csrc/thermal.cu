@@ -65,6 +65,36 @@ __global__ void optics_tangent_kernel(const R* __restrict__ T, const R* __restri
     }
 }
 
+// SH and pump power of thermal runs from the weighted |S|^2, |P|^2 their marches left in
+// w_out: a warp per row, its 32 lanes' columns added in order and the lanes by a shuffle tree,
+// then the rows the same way.  One order for every march, so an instance's powers do not
+// depend on which one ran it.
+__device__ __forceinline__ double lane_sum(const double* v, int n, int lane) {
+    double a = 0.0;
+    for (int i = lane; i < n; i += 32) a += v[i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    return a;
+}
+// grid (2 n / 8 row blocks, count) of 8 warps; the row sums replace each row's first element
+__global__ void __launch_bounds__(256) thermal_row_power_kernel(const InstDesc* __restrict__ descs) {
+    const InstDesc& d = descs[blockIdx.y];
+    const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31, n = d.n;
+    double* v = d.w_out + (size_t)row * n;
+    const double a = lane_sum(v, n, lane);
+    __syncwarp();
+    if (lane == 0) v[0] = a;
+}
+__global__ void thermal_power_kernel(const InstDesc* __restrict__ descs) {
+    const InstDesc& d = descs[blockIdx.x];
+    const int f = threadIdx.x >> 5, lane = threadIdx.x & 31, n = d.n;  // warp 0: SH, warp 1: pump
+    double a = 0.0;
+    for (int i = lane; i < n; i += 32) a += d.w_out[((size_t)f * n + i) * n];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    if (lane == 0 && d.power_out[f] >= 0.0) d.power_out[f] = a * (f ? d.pw_p : d.pw_s);  // < 0: the march gave up
+}
+
 template <typename R>
 __global__ void fill_kernel(R* __restrict__ a, size_t total, R v) {
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) a[i] = v;
@@ -344,6 +374,12 @@ template <typename R>
 cudaError_t launch_fill(R* a, size_t total, R v, cudaStream_t s) {
     const int blocks = (int)std::min<size_t>((total + 255) / 256, 148 * 16);
     fill_kernel<R><<<blocks, 256, 0, s>>>(a, total, v);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_thermal_power(const InstDesc* descs, int count, int n, cudaStream_t s) {
+    thermal_row_power_kernel<<<dim3(2 * n / 8, count), 256, 0, s>>>(descs);
+    thermal_power_kernel<<<count, 64, 0, s>>>(descs);
     return cudaGetLastError();
 }
 

@@ -30,6 +30,9 @@ template <typename R> cudaError_t launch_optics(const R* T, R* dk, R* np, R* ns,
 template <typename R>
 cudaError_t launch_optics_tangent(const R* T, const R* u, R* ddk, R* dnp, R* dns, const shg_params& p, cudaStream_t s);
 template <typename R> cudaError_t launch_fill(R* a, size_t total, R v, cudaStream_t s);
+// SH and pump power of `count` thermal runs of side n from their w_out, into their power_out
+struct InstDesc;
+cudaError_t launch_thermal_power(const InstDesc* descs, int count, int n, cudaStream_t s);
 // one sweep Ti -> Tf; with resid, also the convergence value of that sweep into *out
 template <typename R>
 cudaError_t launch_jacobi(const R* Ti, R* Tf, const R* Q, const JacobiCoef<R>& k, int boundary, bool resid, int rule,

@@ -82,7 +82,7 @@ struct ThermalInst {
     void *pump_out = nullptr, *signal_out = nullptr, *slices_p = nullptr, *slices_s = nullptr;
     char* buf = nullptr;
     R *Ta = nullptr, *Tb = nullptr, *Q = nullptr, *DK = nullptr, *NP = nullptr, *NS = nullptr;
-    double *partial = nullptr, *resid = nullptr, *power = nullptr;
+    double *partial = nullptr, *resid = nullptr, *power = nullptr, *w_out = nullptr;
     unsigned* tb_err = nullptr;
     R *cur = nullptr, *nxt = nullptr;  // cur holds the latest temperature (the reference's Tinic == Tfinal)
     SweepMaps<R> maps;
@@ -174,7 +174,8 @@ shg_status ti_alloc(ThermalInst<R>& t, cudaStream_t s) {
     const int n = p.nx, nz = p.nz;
     const size_t nt = (size_t)n * n * nz, arr = sizeof(R) * nt;
     const size_t npart = jacobi_partials(p);
-    const size_t bytes = 6 * arr + sizeof(double) * (npart + 4) + 256;
+    const size_t nw = 2 * (size_t)n * n;
+    const size_t bytes = 6 * arr + sizeof(double) * (npart + 4 + nw) + 256;
     cudaError_t e;
     if ((e = dev_alloc((void**)&t.buf, bytes, s)) != cudaSuccess) return cuda_fail(e, "cudaMallocAsync");
     t.Ta = reinterpret_cast<R*>(t.buf);
@@ -186,6 +187,7 @@ shg_status ti_alloc(ThermalInst<R>& t, cudaStream_t s) {
     t.partial = reinterpret_cast<double*>(t.NS + nt);
     t.resid = t.partial + npart;                            // [0] convergence value, [1] staging-error word
     t.power = t.resid + 2;                                  // [2]
+    t.w_out = t.power + 2;                                  // [2][n*n]
     t.tb_err = reinterpret_cast<unsigned*>(t.resid + 1);    // set by a blocked sweep whose staging timed out
     t.k = make_jacobi_coef<R>(p);
     // Solver.h:332: tol = 5e-4 / TSIZE in the working precision
@@ -204,7 +206,7 @@ shg_status ti_alloc(ThermalInst<R>& t, cudaStream_t s) {
 template <typename R>
 shg_status ti_init(ThermalInst<R>& t, cudaStream_t s) {
     cudaError_t e;
-    if ((e = cudaMemsetAsync(t.resid, 0, 2 * sizeof(double), s)) != cudaSuccess) return cuda_fail(e, "memset");
+    if ((e = cudaMemsetAsync(t.resid, 0, 4 * sizeof(double), s)) != cudaSuccess) return cuda_fail(e, "memset");
     if ((e = launch_thermal_init<R>(t.Ta, t.Tb, t.Q, *t.p, s)) != cudaSuccess) return cuda_fail(e, "thermal init");
     return SHG_OK;
 }
@@ -319,6 +321,7 @@ shg_status ti_optics(ThermalInst<R>& t, cudaStream_t s) {
     d.pump_out = t.pump_out;
     d.signal_out = t.signal_out;
     d.power_out = t.power;
+    d.w_out = t.w_out;
     d.slices_p = t.slices_p;
     d.slices_s = t.slices_s;
     d.nslices = (t.slices_p || t.slices_s) ? nz : 0;
@@ -402,7 +405,10 @@ shg_status thermal_batch_run(const shg_params* ps, int count, const void* const*
                 rc = cuda_fail(e, "descriptors");
                 break;
             }
-            if ((e = run_variant(v, dd, hd.data(), na, nullptr, s)) != cudaSuccess) { rc = cuda_fail(e, "thermal optical pass"); break; }
+            // the wide march while the instances still iterating are few enough for it (the
+            // marches agree bit for bit, so an instance's results do not depend on the choice)
+            const PlainVariant* w = p0.march == SHG_MARCH_AUTO ? wide_variant_for(p0.precision, p0.nx, 1, na) : nullptr;
+            if ((e = run_variant(w ? w : v, dd, hd.data(), na, nullptr, s)) != cudaSuccess) { rc = cuda_fail(e, "thermal optical pass"); break; }
             cudaEventRecord(ej[2], s);
             if ((e = cudaEventSynchronize(ej[2])) != cudaSuccess) { rc = cuda_fail(e, "thermal optical pass"); break; }
             float ms = 0.f;
@@ -428,6 +434,13 @@ shg_status thermal_batch_run(const shg_params* ps, int count, const void* const*
         if (rc != SHG_OK) break;
         cudaEventRecord(t1, s);
         if (stats) {
+            for (int i = 0; i < count; ++i) hd[i] = ti[i].d;  // each instance's last pass
+            if ((e = cudaMemcpyAsync(dd, hd.data(), sizeof(InstDesc) * (size_t)count, cudaMemcpyHostToDevice, s)) !=
+                    cudaSuccess ||
+                (e = launch_thermal_power(dd, count, p0.nx, s)) != cudaSuccess) {
+                rc = cuda_fail(e, "thermal powers");
+                break;
+            }
             std::vector<double> h(2 * (size_t)count);
             for (int i = 0; i < count && e == cudaSuccess; ++i)
                 e = cudaMemcpyAsync(&h[2 * (size_t)i], ti[i].power, 2 * sizeof(double), cudaMemcpyDeviceToHost, s);
@@ -449,6 +462,7 @@ shg_status thermal_batch_run(const shg_params* ps, int count, const void* const*
                 st.device_ms = ms;
                 st.jacobi_ms = ti[i].jacobi_ms;
                 st.optics_ms = ti[i].optics_ms;
+                if (rc == SHG_OK && st.sh_power < 0.0) rc = fail(SHG_ERR_CUDA, "a grid barrier of the march ran out");
                 if (rc == SHG_OK && (!std::isfinite(st.sh_power) || !std::isfinite(st.pump_power)))
                     rc = count > 1 ? fail(SHG_ERR_NONFINITE, "instance %d: SH / pump power %g / %g", i, st.sh_power,
                                           st.pump_power)

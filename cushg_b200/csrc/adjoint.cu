@@ -1,6 +1,9 @@
 // adjoint.cu — instantiations and host driver of the adjoint march (ssfm_adjoint.cuh):
 // shg_grad and shg_grad_batch of include/shg.h.  A batch is one launch with one cluster per
 // instance, each with its own checkpoints, segment buffers and accumulators.
+// The compiler chooses which product of a sum it fuses, as it did before the marches fixed the
+// choice: a derivative near its optimum is a small remainder, and keeps its bits this way.
+#define SHG_COMPILER_CONTRACTION
 #include <cuda_runtime.h>
 
 #include <algorithm>

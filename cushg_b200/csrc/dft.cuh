@@ -17,9 +17,9 @@ template <> struct cx_t<double> { using type = double2; };
 template <typename T> using cx = typename cx_t<T>::type;
 
 // Multiply, add and fused multiply-add with one rounding each, never contracted or split by
-// the compiler.  Everything a field value passes through is written with these, so that every
-// kernel that inlines it rounds alike: the fused, wide and multi-pass marches of one instance
-// give the same bits.
+// the compiler.  Everything a field value passes through in a march is written with these, so
+// that every kernel that inlines it rounds alike: the fused, wide and multi-pass marches of one
+// instance give the same bits.
 __device__ __forceinline__ float fma_r(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double fma_r(double a, double b, double c) { return __fma_rn(a, b, c); }
 __device__ __forceinline__ float mul_r(float a, float b) { return __fmul_rn(a, b); }
@@ -27,15 +27,37 @@ __device__ __forceinline__ double mul_r(double a, double b) { return __dmul_rn(a
 __device__ __forceinline__ float add_r(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ double add_r(double a, double b) { return __dadd_rn(a, b); }
 
+// a b + c d and a b - c d with one product fused into the add: the first, or with SECOND the
+// second.  Either is as good; each use below fuses the product that the compiler fused in the
+// fused march before this was written out, so the FP32 fields of plain runs kept their bits.
+// A source that defines SHG_COMPILER_CONTRACTION leaves the choice to the compiler (the adjoint
+// march, which shares no bits with the others).
+template <bool SECOND = false, typename T>
+__device__ __forceinline__ T dot2(T a, T b, T c, T d) {
+#ifdef SHG_COMPILER_CONTRACTION
+    return a * b + c * d;
+#else
+    return SECOND ? fma_r(c, d, mul_r(a, b)) : fma_r(a, b, mul_r(c, d));
+#endif
+}
+template <bool SECOND = false, typename T>
+__device__ __forceinline__ T det2(T a, T b, T c, T d) {
+#ifdef SHG_COMPILER_CONTRACTION
+    return a * b - c * d;
+#else
+    return SECOND ? fma_r(-c, d, mul_r(a, b)) : fma_r(a, b, mul_r(-c, d));
+#endif
+}
+
 template <typename T> __device__ __forceinline__ cx<T> mk(T re, T im) { cx<T> c; c.x = re; c.y = im; return c; }
 template <typename T> __device__ __forceinline__ cx<T> add(cx<T> a, cx<T> b) { return mk<T>(add_r(a.x, b.x), add_r(a.y, b.y)); }
 template <typename T> __device__ __forceinline__ cx<T> sub(cx<T> a, cx<T> b) { return mk<T>(add_r(a.x, -b.x), add_r(a.y, -b.y)); }
 template <typename T> __device__ __forceinline__ cx<T> mul(cx<T> a, cx<T> b) {
-    return mk<T>(fma_r(a.x, b.x, mul_r(-a.y, b.y)), fma_r(a.x, b.y, mul_r(a.y, b.x)));
+    return mk<T>(det2(a.x, b.x, a.y, b.y), dot2(a.x, b.y, a.y, b.x));
 }
 // a * conj(b)
 template <typename T> __device__ __forceinline__ cx<T> mulc(cx<T> a, cx<T> b) {
-    return mk<T>(fma_r(a.x, b.x, mul_r(a.y, b.y)), fma_r(a.y, b.x, mul_r(-a.x, b.y)));
+    return mk<T>(dot2(a.x, b.x, a.y, b.y), det2(a.y, b.x, a.x, b.y));
 }
 template <typename T> __device__ __forceinline__ cx<T> scale(cx<T> a, T s) { return mk<T>(mul_r(a.x, s), mul_r(a.y, s)); }
 
@@ -78,20 +100,12 @@ __host__ __device__ constexpr double sin32(int m) { return cos32((m + 24) & 31);
 // into hi + lo parts and applied with fused multiply-adds, so its rounding does not
 // bias the modulus of every transform by the same relative amount step after step (a
 // coherent error that would grow linearly with the number of SSFM steps).
-//
-// The sum of two products fuses one of them into the add; which one is a free choice, made
-// here (re2, im2: the second) as the compiler made it in the fused march before the choice was
-// written out, so the FP32 fields of a plain run kept their bits.
 template <typename T>
 __device__ __forceinline__ cx<T> rot_const(cx<T> v, double c, double s) {
     const bool diag = c == s, anti = c == -s;  // odd multiples of 45 degrees
     const bool re2 = sizeof(T) == 8 && diag, im2 = sizeof(T) == 8 ? !anti : !diag;
-    auto re = [&](T cc, T ss) {  // x c - y s
-        return re2 ? fma_r(-v.y, ss, mul_r(v.x, cc)) : fma_r(v.x, cc, mul_r(-v.y, ss));
-    };
-    auto im = [&](T cc, T ss) {  // x s + y c
-        return im2 ? fma_r(v.y, cc, mul_r(v.x, ss)) : fma_r(v.x, ss, mul_r(v.y, cc));
-    };
+    auto re = [&](T cc, T ss) { return re2 ? det2<true>(v.x, cc, v.y, ss) : det2(v.x, cc, v.y, ss); };
+    auto im = [&](T cc, T ss) { return im2 ? dot2<true>(v.x, ss, v.y, cc) : dot2(v.x, ss, v.y, cc); };
     if constexpr (sizeof(T) == 8) {
         return mk<T>(re(c, s), im(c, s));
     } else {
@@ -140,28 +154,25 @@ template <> __host__ __device__ __forceinline__ float4 make_mult<float>(double r
 
 // v * w
 __device__ __forceinline__ double2 mulw(double2 v, double2 w) {
-    return make_double2(fma_r(v.x, w.x, mul_r(-v.y, w.y)), fma_r(v.y, w.x, mul_r(v.x, w.y)));
+    return make_double2(det2(v.x, w.x, v.y, w.y), dot2<true>(v.x, w.y, v.y, w.x));
 }
 __device__ __forceinline__ float2 mulw(float2 v, float4 w) {
-    return make_float2(fma_r(v.x, w.x, fma_r(-v.y, w.y, fma_r(v.x, w.z, mul_r(-v.y, w.w)))),
-                       fma_r(v.x, w.y, fma_r(v.y, w.x, fma_r(v.y, w.z, mul_r(v.x, w.w)))));
+    return make_float2(fma_r(v.x, w.x, fma_r(-v.y, w.y, det2(v.x, w.z, v.y, w.w))),
+                       fma_r(v.x, w.y, fma_r(v.y, w.x, dot2<true>(v.x, w.w, v.y, w.z))));
 }
 // conj(v) * w
+#ifdef SHG_COMPILER_CONTRACTION
+__device__ __forceinline__ double2 mulw_cj(double2 v, double2 w) { return mulw(make_double2(v.x, -v.y), w); }
+__device__ __forceinline__ float2 mulw_cj(float2 v, float4 w) { return mulw(make_float2(v.x, -v.y), w); }
+#else
 __device__ __forceinline__ double2 mulw_cj(double2 v, double2 w) {
-    return make_double2(fma_r(v.x, w.x, mul_r(v.y, w.y)), fma_r(v.x, w.y, mul_r(-v.y, w.x)));
+    return make_double2(dot2(v.x, w.x, v.y, w.y), det2(v.x, w.y, v.y, w.x));
 }
 __device__ __forceinline__ float2 mulw_cj(float2 v, float4 w) {
-    return make_float2(fma_r(v.x, w.x, fma_r(v.y, w.y, fma_r(v.x, w.z, mul_r(v.y, w.w)))),
-                       fma_r(v.x, w.y, fma_r(-v.y, w.x, fma_r(v.x, w.w, mul_r(-v.y, w.z)))));
+    return make_float2(fma_r(v.x, w.x, fma_r(v.y, w.y, dot2(v.x, w.z, v.y, w.w))),
+                       fma_r(v.x, w.y, fma_r(-v.y, w.x, det2(v.x, w.w, v.y, w.z))));
 }
-// v * conj(w)
-__device__ __forceinline__ double2 mulwc(double2 v, double2 w) {
-    return make_double2(fma_r(v.x, w.x, mul_r(v.y, w.y)), fma_r(v.y, w.x, mul_r(-v.x, w.y)));
-}
-__device__ __forceinline__ float2 mulwc(float2 v, float4 w) {
-    return make_float2(fma_r(v.x, w.x, fma_r(v.y, w.y, fma_r(v.x, w.z, mul_r(v.y, w.w)))),
-                       fma_r(v.y, w.x, fma_r(-v.x, w.y, fma_r(v.y, w.z, mul_r(-v.x, w.w)))));
-}
+#endif
 
 template <int M, int SIGN, typename T> struct Dft;
 

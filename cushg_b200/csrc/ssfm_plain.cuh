@@ -74,9 +74,9 @@ __device__ __forceinline__ void dadz(cx<T> p, cx<T> s, cx<T> cP, cx<T> cS, T hap
                                      cx<T>& ds) {
     const cx<T> tp = mul<T>(cP, mulc<T>(s, p));
     dp = mk<T>(fma_r(-hap, p.x, tp.x), fma_r(-hap, p.y, tp.y));
-    const cx<T> pp = mk<T>(fma_r(p.x, p.x, mul_r(-p.y, p.y)), mul_r(add_r(p.x, p.x), p.y));
+    const cx<T> pp = mk<T>(det2(p.x, p.x, p.y, p.y), mul_r(add_r(p.x, p.x), p.y));
     const cx<T> ts = mul<T>(cS, pp);
-    const T g = fma_r(qs, fma_r(s.x, s.x, mul_r(s.y, s.y)), has);
+    const T g = fma_r(qs, dot2(s.x, s.x, s.y, s.y), has);
     ds = mk<T>(fma_r(-g, s.x, ts.x), fma_r(-g, s.y, ts.y));
 }
 

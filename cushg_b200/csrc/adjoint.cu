@@ -172,12 +172,12 @@ shg_status grad_batch(const shg_params* ps, int count, const double* const* poli
     }
     bool keep_all = false;
     if (checkpoint_every <= 0 && nsm > 0 && (size_t)count * C >= (size_t)nsm) {
-        size_t need = 0, fr = 0, tot = 0;
+        size_t need = 0, fr = 0;
         for (GradJob& J : jobs) {
             layout(J, J.nsteps);
             need += J.bytes;
         }
-        if (cudaMemGetInfo(&fr, &tot) == cudaSuccess) keep_all = need <= fr / 2;
+        if (dev_free_bytes(&fr) == cudaSuccess) keep_all = need <= fr / 2;
         else cudaGetLastError();
     }
     size_t total = 0;

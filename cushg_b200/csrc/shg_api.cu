@@ -72,7 +72,9 @@ cudaError_t dev_alloc(void** ptr, size_t bytes, cudaStream_t s) {
                 pools[dev] = nullptr;
                 return e;
             }
-            unsigned long long keep = kPoolKeepBytes;
+            size_t fr = 0, total = 0;
+            if (cudaMemGetInfo(&fr, &total) != cudaSuccess) cudaGetLastError();
+            unsigned long long keep = total / kPoolKeepFraction;
             if (const char* env = std::getenv("SHG_POOL_KEEP_MB")) {
                 char* end = nullptr;
                 const unsigned long long mb = std::strtoull(env, &end, 10);
@@ -83,6 +85,21 @@ cudaError_t dev_alloc(void** ptr, size_t bytes, cudaStream_t s) {
         pool = pools[dev];
     }
     return cudaMallocFromPoolAsync(ptr, bytes, pool, s);
+}
+
+cudaError_t dev_free_bytes(size_t* bytes) {
+    size_t fr = 0, total = 0;
+    cudaError_t e = cudaMemGetInfo(&fr, &total);
+    int dev = 0;
+    if (e != cudaSuccess || (e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    unsigned long long reserved = 0, used = 0;
+    if (dev >= 0 && dev < 64 && g_pools[dev] &&
+        cudaMemPoolGetAttribute(g_pools[dev], cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
+        cudaMemPoolGetAttribute(g_pools[dev], cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess && reserved > used)
+        fr += reserved - used;
+    *bytes = fr;
+    return cudaSuccess;
 }
 
 // Physical constants, src/headers/Crystal.h:19-21 (µm, ps, W, V).

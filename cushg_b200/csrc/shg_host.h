@@ -17,14 +17,19 @@ shg_status fail(shg_status st, const char* fmt, ...);
 shg_status cuda_fail(cudaError_t e, const char* what);
 void clear_error();
 
-// Stream-ordered device memory from the library's own pool on the current device, which keeps
-// up to kPoolKeepBytes (or SHG_POOL_KEEP_MB megabytes from the environment, read when the
-// pool is created) between calls instead of handing it back at every synchronisation (the
-// default pool's release threshold is 0, so a repeated call would map its workspace again
-// each time).
-constexpr unsigned long long kPoolKeepBytes = 2ull << 30;
+// Stream-ordered device memory from the library's own pool on the current device.  The pool
+// keeps up to a quarter of the device's memory (or SHG_POOL_KEEP_MB megabytes from the
+// environment, read when the pool is created) between calls instead of handing it back at every
+// synchronisation: mapping new memory takes 13-40 ms per GB, and a gradient batch that keeps
+// every step's fields (42 GB for 18 FP64 256 x 256 x 400 instances) spent 570 ms and more of
+// each call on it, against 115 ms of kernels.  What the pool holds unused is not lost to the
+// process: the driver hands it to any other allocation (cudaMalloc and everything built on it)
+// that would fail without it.
+constexpr unsigned long long kPoolKeepFraction = 4;
 // Inside a stream capture it falls back to cudaMallocAsync (a graph memory node).
 cudaError_t dev_alloc(void** ptr, size_t bytes, cudaStream_t s);
+// Device memory dev_alloc can still hand out: what is free, and what the pool holds unused.
+cudaError_t dev_free_bytes(size_t* bytes);
 
 double sellmeier(int crystal, double L, double T);
 double delta_k(const shg_params& p, double T);

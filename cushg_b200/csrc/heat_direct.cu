@@ -366,15 +366,26 @@ __global__ void rhs_kernel(const R* __restrict__ T, const R* __restrict__ Q, dou
     }
 }
 
-// A block computes a 128 x 128 tile of C with eight warps, each a 64 x 32 part of it as 4 x 4
-// FP64 tensor-core products (mma.sync m16n8k4); k runs in 32-wide slices through a
-// three-stage ring of cp.async copies.  Row pitches: A slices 36 doubles, B slices 132, so
+// A block computes a BM x BN tile of C with WR x WC warps, each a 16 MI x 8 NJ part of it as
+// MI x NJ FP64 tensor-core products (mma.sync m16n8k4); k runs in 32-wide slices through a
+// three-stage ring of cp.async copies.  Row pitches: A slices 36 doubles, B slices BN + 4, so
 // that the fragment reads of a half-warp (4 rows x 4 columns of A, 4 rows x 4 columns of B)
 // fall in 16 different 8-byte bank pairs; every row starts on 16 bytes.
-constexpr int kGemmBM = 128, kGemmBN = 128, kGemmBK = 32, kGemmThreads = 256, kGemmStages = 3;
-constexpr int kGemmALd = kGemmBK + 4, kGemmBLd = kGemmBN + 4;
-constexpr int kGemmStageDoubles = kGemmBM * kGemmALd + kGemmBK * kGemmBLd;
-constexpr size_t kGemmSmem = sizeof(double) * kGemmStageDoubles * kGemmStages;  // 207 KB
+//   128 x 128 (eight 64 x 32 warps) has the fewest shared-memory reads per product and runs the
+// FP64 pipe at 82-85 % of its peak, but leaves the device idle where it cuts a product into few
+// tiles: 96 x 96 x 37 has 28, of 25 k cycles each.  32 x 32 (four 16 x 16 warps) and 64 x 64 (four
+// 32 x 32 warps) are for those (gemm picks).
+template <int MI_, int NJ_, int WR_, int WC_, int MINB_>
+struct GemmCfg {
+    static constexpr int MI = MI_, NJ = NJ_, WR = WR_, WC = WC_, MINB = MINB_;
+    static constexpr int BM = 16 * MI * WR, BN = 8 * NJ * WC, BK = 32, THREADS = 32 * WR * WC, STAGES = 3;
+    static constexpr int ALD = BK + 4, BLD = BN + 4;
+    static constexpr int STAGE = BM * ALD + BK * BLD;  // doubles
+    static constexpr size_t SMEM = sizeof(double) * STAGE * STAGES;
+};
+using GemmBig = GemmCfg<4, 4, 2, 4, 1>;    // 128 x 128, 207 KB
+using GemmMid = GemmCfg<2, 4, 2, 2, 2>;    // 64 x 64, 107 KB
+using GemmSmall = GemmCfg<1, 2, 2, 2, 4>;  // 32 x 32, 54 KB
 
 // 16 bytes from global to shared memory, asynchronously; the bytes past `valid` (0..16) are
 // zero-filled and not read.
@@ -395,86 +406,89 @@ __device__ __forceinline__ void mma_f64(double (&c)[4], double a0, double a1, do
 // 2, 4. C[b] = A[b] B[b] in FP64 for row-major A (M x K, lda), B (K x N, ldb) and C (M x N, ldc),
 // batch b = blockIdx.z at element strides sA, sB, sC.  lda, ldb, ldc, the strides and the three
 // base addresses are even (16-byte rows).  Copies past M, N and K are zero-filled.
-__global__ void __launch_bounds__(kGemmThreads, 1) dgemm_kernel(const double* __restrict__ A, const double* __restrict__ B,
-                                                             double* __restrict__ C, int M, int N, int K, int lda,
-                                                             int ldb, int ldc, long long sA, long long sB, long long sC) {
+template <class Cfg>
+__global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB)
+    dgemm_kernel(const double* __restrict__ A, const double* __restrict__ B, double* __restrict__ C, int M, int N, int K,
+                 int lda, int ldb, int ldc, long long sA, long long sB, long long sC) {
+    constexpr int MI = Cfg::MI, NJ = Cfg::NJ, BM = Cfg::BM, BN = Cfg::BN, BK = Cfg::BK, STAGES = Cfg::STAGES;
+    constexpr int ALD = Cfg::ALD, BLD = Cfg::BLD;
     extern __shared__ __align__(16) double gsm[];
     A += blockIdx.z * sA;
     B += blockIdx.z * sB;
     C += blockIdx.z * sC;
-    const int m0 = blockIdx.y * kGemmBM, n0 = blockIdx.x * kGemmBN;
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
-    const int wm = (warp & 1) * 64, wn = (warp >> 1) * 32;  // this warp's 64 x 32 part of the tile
-    // k slice `tile` into stage st: A 128 x 32 and B 32 x 128, 2048 chunks of 16 bytes each
+    const int wm = (warp % Cfg::WR) * 16 * MI, wn = (warp / Cfg::WR) * 8 * NJ;  // this warp's part of the tile
+    // k slice `tile` into stage st, in chunks of 16 bytes
     auto load = [&](int tile, int st) {
-        double* As = gsm + st * kGemmStageDoubles;
-        double* Bs = As + kGemmBM * kGemmALd;
-        const int k0 = tile * kGemmBK;
+        double* As = gsm + st * Cfg::STAGE;
+        double* Bs = As + BM * ALD;
+        const int k0 = tile * BK;
 #pragma unroll
-        for (int j = 0; j < kGemmBM * kGemmBK / 2 / kGemmThreads; ++j) {
-            const int c = tid + j * kGemmThreads;
-            const int row = c / (kGemmBK / 2), col = (c % (kGemmBK / 2)) * 2;
+        for (int j = 0; j < BM * BK / 2 / Cfg::THREADS; ++j) {
+            const int c = tid + j * Cfg::THREADS;
+            const int row = c / (BK / 2), col = (c % (BK / 2)) * 2;
             const int gr = m0 + row, gc = k0 + col;
             const int valid = gr < M ? 8 * max(0, min(2, K - gc)) : 0;
-            cp_async16(As + row * kGemmALd + col, valid ? A + (size_t)gr * lda + gc : A, valid);
+            cp_async16(As + row * ALD + col, valid ? A + (size_t)gr * lda + gc : A, valid);
         }
 #pragma unroll
-        for (int j = 0; j < kGemmBK * kGemmBN / 2 / kGemmThreads; ++j) {
-            const int c = tid + j * kGemmThreads;
-            const int row = c / (kGemmBN / 2), col = (c % (kGemmBN / 2)) * 2;
+        for (int j = 0; j < BK * BN / 2 / Cfg::THREADS; ++j) {
+            const int c = tid + j * Cfg::THREADS;
+            const int row = c / (BN / 2), col = (c % (BN / 2)) * 2;
             const int gr = k0 + row, gc = n0 + col;
             const int valid = gr < K ? 8 * max(0, min(2, N - gc)) : 0;
-            cp_async16(Bs + row * kGemmBLd + col, valid ? B + (size_t)gr * ldb + gc : B, valid);
+            cp_async16(Bs + row * BLD + col, valid ? B + (size_t)gr * ldb + gc : B, valid);
         }
     };
-    double acc[4][4][4];
+    double acc[MI][NJ][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < MI; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
+        for (int j = 0; j < NJ; ++j)
 #pragma unroll
             for (int r = 0; r < 4; ++r) acc[i][j][r] = 0.0;
-    const int tiles = (K + kGemmBK - 1) / kGemmBK;
+    const int tiles = (K + BK - 1) / BK;
 #pragma unroll
-    for (int st = 0; st < kGemmStages - 1; ++st) {
+    for (int st = 0; st < STAGES - 1; ++st) {
         if (st < tiles) load(st, st);
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
     for (int tl = 0; tl < tiles; ++tl) {
         // this thread's copies of slice tl have landed; the barrier makes everyone's visible and
         // ends every read of the stage the next load overwrites (slice tl - 1's)
-        asm volatile("cp.async.wait_group %0;" ::"n"(kGemmStages - 2) : "memory");
+        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
         __syncthreads();
-        if (tl + kGemmStages - 1 < tiles) load(tl + kGemmStages - 1, (tl + kGemmStages - 1) % kGemmStages);
+        if (tl + STAGES - 1 < tiles) load(tl + STAGES - 1, (tl + STAGES - 1) % STAGES);
         asm volatile("cp.async.commit_group;" ::: "memory");
-        const double* As = gsm + (tl % kGemmStages) * kGemmStageDoubles;
-        const double* Bs = As + kGemmBM * kGemmALd;
+        const double* As = gsm + (tl % STAGES) * Cfg::STAGE;
+        const double* Bs = As + BM * ALD;
 #pragma unroll
-        for (int kk = 0; kk < kGemmBK; kk += 4) {
-            double a[4][2], b[4];
+        for (int kk = 0; kk < BK; kk += 4) {
+            double a[MI][2], b[NJ];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                a[i][0] = As[(wm + 16 * i + g) * kGemmALd + kk + t];
-                a[i][1] = As[(wm + 16 * i + g + 8) * kGemmALd + kk + t];
+            for (int i = 0; i < MI; ++i) {
+                a[i][0] = As[(wm + 16 * i + g) * ALD + kk + t];
+                a[i][1] = As[(wm + 16 * i + g + 8) * ALD + kk + t];
             }
 #pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = Bs[(kk + t) * kGemmBLd + wn + 8 * j + g];
+            for (int j = 0; j < NJ; ++j) b[j] = Bs[(kk + t) * BLD + wn + 8 * j + g];
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < MI; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) mma_f64(acc[i][j], a[i][0], a[i][1], b[j]);
+                for (int j = 0; j < NJ; ++j) mma_f64(acc[i][j], a[i][0], a[i][1], b[j]);
         }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < MI; ++i)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int row = m0 + wm + 16 * i + g + 8 * h;
             if (row >= M) continue;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
+            for (int j = 0; j < NJ; ++j) {
                 const int col = n0 + wn + 8 * j + 2 * t;  // even: 16-byte aligned in C
                 double* out = C + (size_t)row * ldc + col;
                 if (col + 1 < N) *reinterpret_cast<double2*>(out) = make_double2(acc[i][j][2 * h], acc[i][j][2 * h + 1]);
@@ -563,22 +577,29 @@ __global__ void unfold_kernel(const double* __restrict__ pq, double* __restrict_
 // [1] sum (J(u) - u)^2 for one FP64 Jacobi sweep J of u (jacobi_point, coefficients in FP64),
 // [2] max |u - T_before| and [3] sum (u - T_before)^2.  Maxima are kept as the bits of
 // non-negative doubles (ordered like unsigned integers; a NaN wins).  A thread walks
-// kFinishZ planes of one (x, y) column with u's z neighbours in registers, so every load of a
+// zc planes (finish_planes) of one (x, y) column with u's z neighbours in registers, so every load of a
 // plane is independent of the arithmetic; neighbours outside the unknowns are Dirichlet
 // voxels of T, which nothing writes.
 constexpr int kFinishZ = 16;
 
+// Planes per thread: 16, or fewer (at least 2) where that would leave SMs without three blocks.
+int finish_planes(size_t plane, int nz) {
+    int zc = kFinishZ;
+    while (zc > 2 && plane * ((nz + zc - 1) / zc) < (size_t)148 * 3 * 256) zc /= 2;
+    return zc;
+}
+
 template <typename R, int BOUND>
 __global__ void __launch_bounds__(256, 3) finish_kernel(R* __restrict__ T, const R* __restrict__ Q, const double* __restrict__ u,
-                                                     const HeatArgs a, const JacobiCoef<double> k, double* __restrict__ out) {
+                                                     const HeatArgs a, const JacobiCoef<double> k, int zc, double* __restrict__ out) {
     auto U = [&](size_t rowbase, int col) -> double { return u[rowbase + col]; };  // the solution
     const size_t plane = (size_t)a.mx * a.my, nn = (size_t)a.n, tplane = nn * nn;
-    const int chunks = (a.nz + kFinishZ - 1) / kFinishZ;
+    const int chunks = (a.nz + zc - 1) / zc;
     const size_t items = plane * chunks;
     double rmax = 0.0, rsum = 0.0, cmax = 0.0, csum = 0.0;
     for (size_t it = blockIdx.x * (size_t)blockDim.x + threadIdx.x; it < items; it += (size_t)gridDim.x * blockDim.x) {
         const size_t t = it % plane;
-        const int z0 = (int)(it / plane) * kFinishZ, z1 = min(a.nz, z0 + kFinishZ);
+        const int z0 = (int)(it / plane) * zc, z1 = min(a.nz, z0 + zc);
         const int i = (int)(t % a.mx), j = (int)(t / a.mx);
         const int x = a.x0 + i, y = a.y0 + j;
         const bool uxm = i > 0, uxp = i + 1 < a.mx, uym = j > 0, uyp = j + 1 < a.my;
@@ -644,23 +665,40 @@ __global__ void __launch_bounds__(256, 3) finish_kernel(R* __restrict__ T, const
 
 // C = A B over `batch` matrices (see dgemm_kernel); M is split into launches of at most 65535
 // row tiles.
-cudaError_t gemm(const double* A, const double* B, double* C, int M, int N, int K, int lda, int ldb, int ldc, int batch,
-                 long long sA, long long sB, long long sC, cudaStream_t s) {
+template <class Cfg>
+cudaError_t gemm_tiles(const double* A, const double* B, double* C, int M, int N, int K, int lda, int ldb, int ldc,
+                       int batch, long long sA, long long sB, long long sC, cudaStream_t s) {
+    auto kern = dgemm_kernel<Cfg>;
     static PerDevice<int> attr;  // the kernel's dynamic shared memory, once per device
-    const cudaError_t ae = attr.get([](int, int&) {
-        return cudaFuncSetAttribute(dgemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem);
+    const cudaError_t ae = attr.get([&](int, int&) {
+        return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM);
     });
     if (ae != cudaSuccess) return ae;
-    const int max_rows = 65535 * kGemmBM;
+    const int max_rows = 65535 * Cfg::BM;
     for (int r0 = 0; r0 < M; r0 += max_rows) {
         const int rows = std::min(M - r0, max_rows);
-        const dim3 grid((unsigned)((N + kGemmBN - 1) / kGemmBN), (unsigned)((rows + kGemmBM - 1) / kGemmBM), (unsigned)batch);
-        dgemm_kernel<<<grid, kGemmThreads, kGemmSmem, s>>>(A + (size_t)r0 * lda, B, C + (size_t)r0 * ldc, rows, N, K, lda, ldb,
-                                                   ldc, sA, sB, sC);
+        const dim3 grid((unsigned)((N + Cfg::BN - 1) / Cfg::BN), (unsigned)((rows + Cfg::BM - 1) / Cfg::BM), (unsigned)batch);
+        kern<<<grid, Cfg::THREADS, Cfg::SMEM, s>>>(A + (size_t)r0 * lda, B, C + (size_t)r0 * ldc, rows, N, K, lda, ldb, ldc,
+                                                   sA, sB, sC);
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
+}
+
+// Which tile: the one whose busiest SM has the least to do, counting its tiles' products (padding
+// included) at the share of the FP64 pipe the tile reaches.
+cudaError_t gemm(const double* A, const double* B, double* C, int M, int N, int K, int lda, int ldb, int ldc, int batch,
+                 long long sA, long long sB, long long sC, cudaStream_t s) {
+    auto cost = [&](int bm, int bn, double share) {
+        const double tiles = (double)((M + bm - 1) / bm) * ((N + bn - 1) / bn) * batch;
+        return std::ceil(tiles / 148.0) * bm * bn / share;
+    };
+    const double big = cost(GemmBig::BM, GemmBig::BN, 0.84), mid = cost(GemmMid::BM, GemmMid::BN, 0.7),
+                 small = cost(GemmSmall::BM, GemmSmall::BN, 0.5);
+    if (big <= mid && big <= small) return gemm_tiles<GemmBig>(A, B, C, M, N, K, lda, ldb, ldc, batch, sA, sB, sC, s);
+    if (mid <= small) return gemm_tiles<GemmMid>(A, B, C, M, N, K, lda, ldb, ldc, batch, sA, sB, sC, s);
+    return gemm_tiles<GemmSmall>(A, B, C, M, N, K, lda, ldb, ldc, batch, sA, sB, sC, s);
 }
 
 int grid_for(size_t work, int threads) {
@@ -754,7 +792,8 @@ shg_status HeatDirect::solve(const shg_params& p, R* T, const R* Q, double t_inf
         e = gemm(Y, ox->GT, X, nz * my, mx, mx, mx, ox->ld, mx, 1, 0, 0, 0, s);
     }
     if (e != cudaSuccess) return cuda_fail(e, "heat transform");
-    const size_t fitems = (size_t)pl * ((nz + kFinishZ - 1) / kFinishZ);
+    const int zc = finish_planes((size_t)pl, nz);
+    const size_t fitems = (size_t)pl * ((nz + zc - 1) / zc);
     const int fb = grid_for(fitems, 256);
     const double* u = X;
     if (fold) {
@@ -763,9 +802,9 @@ shg_status HeatDirect::solve(const shg_params& p, R* T, const R* Q, double t_inf
         u = Y;
     }
     if (p.boundary == SHG_BOUNDARY_TOP_OPEN)
-        finish_kernel<R, SHG_BOUNDARY_TOP_OPEN><<<fb, 256, 0, s>>>(T, Q, u, a, k, out);
+        finish_kernel<R, SHG_BOUNDARY_TOP_OPEN><<<fb, 256, 0, s>>>(T, Q, u, a, k, zc, out);
     else
-        finish_kernel<R, SHG_BOUNDARY_OVEN_SURROUNDED><<<fb, 256, 0, s>>>(T, Q, u, a, k, out);
+        finish_kernel<R, SHG_BOUNDARY_OVEN_SURROUNDED><<<fb, 256, 0, s>>>(T, Q, u, a, k, zc, out);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "heat solution");
     return SHG_OK;
 }

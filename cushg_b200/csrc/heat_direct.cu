@@ -15,15 +15,20 @@
 // the reference reduce exactly to these: e.g. the vertical edge's 0.5 (Bix + Biz) times
 // 4/(dx dz) is 2 Bix / dx^2 + 2 Biz / dz^2.)  So A = Ax (+) Ay (+) Az, a Kronecker sum.
 //
-// The solve.  Ax and Ay are tridiagonal and similar to symmetric matrices (a diagonal scaling
-// of the Robin end rows), whose eigendecomposition the host computes once per operator and
-// device (implicit QL).  With the forward transforms F = V^T S and the inverse G = S^{-1} V:
-//   1. b (FP64) from Q, the Dirichlet voxels and T_inf                        rhs_kernel
-//   2. b <- b Fx^T (along x), then Fy b (along y)                            dgemm_kernel x2
-//   3. for every mode (ky, kx): (Az + lambda_x + lambda_y) v = b along z       thomas_kernel
-//   4. v <- Gy v, then v Gx^T                                                dgemm_kernel x2
-//      (folded x transform: v's rows from their even and odd halves)           unfold_kernel
+// The solve.  Two of the three operators are diagonalised by dense transforms (F = V^T S forward,
+// G = S^{-1} V back, of the symmetric form S M S^{-1} = V diag(lambda) V^T) and the third direction
+// is solved by elimination.  x is always transformed.  Of y and z the cheaper one is (axis_of):
+// a direction with the same kind of end at both sides has modes of exact parity, and its
+// transform folds into two of half the size, so z (Robin at both ends) costs nz / 2 products
+// per point against ny for TOP_OPEN's y (Dirichlet and Robin).  With t the transformed one of the
+// two and s the other:
+//   1. b (FP64) from Q, the Dirichlet voxels and T_inf, folded               rhs_kernel
+//   2. b <- b Fx^T (along x), then Ft b (along t)                            dgemm_kernel
+//   3. for every mode (kt, kx): (As + lambda_x + lambda_t) v = b along s     thomas_kernel
+//   4. v <- Gt v, then v Gx^T; unfolded                                      dgemm_kernel, unfold_kernel
 //   5. T <- v, with the FP64 residual of one Jacobi sweep of v and the change  finish_kernel
+// The x and y modes come from the host (implicit QL, once per operator and device), the z modes
+// from their closed form on the device in every solve (z_modes_kernel, microseconds).
 // Unknowns: TOP_OPEN, x 0..n-1 (Robin both ends), y 1..n-1 (y = 0 Dirichlet, Robin at n-1),
 // z 0..nz-1 (Robin); OVEN_SURROUNDED, x and y 1..n-2 (Dirichlet both ends), z as above.
 #include <cuda_runtime.h>
@@ -203,6 +208,12 @@ struct OpMats {
     // laid out for C = A B like FT and GT; lamf the eigenvalues, even modes first.
     bool fold = false;
     double *FeT = nullptr, *FoT = nullptr, *GeT = nullptr, *GoT = nullptr, *lamf = nullptr;
+    // The same halves as left factors (rows modes for F, rows points for G), for a symmetric
+    // operator with m even, as the y direction of OVEN_SURROUNDED has; rows of ldl = h rounded up
+    // to even doubles.
+    bool fold_left = false;
+    int ldl = 0;
+    double *Fe = nullptr, *Fo = nullptr, *Ge = nullptr, *Go = nullptr;
 };
 
 // Process-wide cache of operator transforms, per device (an operator's eigendecomposition
@@ -250,9 +261,20 @@ shg_status get_op(const Op1D& op, const OpMats** out) {
             GoT[(size_t)a * h + i] = G[(size_t)i * m + ko];
         }
     }
+    const bool fold_left = op.lo_robin == op.hi_robin && m % 2 == 0;
+    const int ldl = h + (h & 1);
+    const size_t hl = fold_left ? (size_t)h * ldl : 0;
+    std::vector<double> Fe(hl, 0.0), Fo(hl, 0.0), Ge(hl, 0.0), Go(hl, 0.0);
+    for (int a = 0; fold_left && a < h; ++a)
+        for (int i = 0; i < h; ++i) {
+            Fe[(size_t)a * ldl + i] = F[(size_t)a * m + i];
+            Fo[(size_t)a * ldl + i] = F[(size_t)(h + a) * m + i];
+            Ge[(size_t)i * ldl + a] = G[(size_t)i * m + a];
+            Go[(size_t)i * ldl + a] = G[(size_t)i * m + h + a];
+        }
     if (g_ops.size() >= kMaxCachedOps) return fail(SHG_ERR_UNSUPPORTED, "more than %d heat operators cached", (int)kMaxCachedOps);
     double* buf = nullptr;
-    if ((e = cudaMalloc((void**)&buf, sizeof(double) * (4 * mm + (m + (m & 1)) + 4 * hh + lamf.size()))) != cudaSuccess)
+    if ((e = cudaMalloc((void**)&buf, sizeof(double) * (4 * mm + (m + (m & 1)) + 4 * hh + lamf.size() + 4 * hl))) != cudaSuccess)
         return cuda_fail(e, "cudaMalloc");
     OpMats* c = new OpMats;
     c->op = op;
@@ -272,11 +294,20 @@ shg_status get_op(const Op1D& op, const OpMats** out) {
         c->GoT = fb + 3 * hh;
         c->lamf = fb + 4 * hh;
     }
-    const double* src[10] = {Fp.data(), Gp.data(), FT.data(), GT.data(), lam.data(),
-                             FeT.data(), FoT.data(), GeT.data(), GoT.data(), lamf.data()};
-    double* dst[10] = {c->F, c->G, c->FT, c->GT, c->lam, c->FeT, c->FoT, c->GeT, c->GoT, c->lamf};
-    const size_t cnt[10] = {mm, mm, mm, mm, (size_t)m, hh, hh, hh, hh, lamf.size()};
-    for (int k = 0; k < 10 && e == cudaSuccess; ++k)
+    c->fold_left = fold_left;
+    c->ldl = ldl;
+    if (fold_left) {
+        c->Fe = fb + 4 * hh + lamf.size();  // even offsets: 4 hh, and m with the fold
+        c->Fo = c->Fe + hl;
+        c->Ge = c->Fe + 2 * hl;
+        c->Go = c->Fe + 3 * hl;
+    }
+    const double* src[14] = {Fp.data(),  Gp.data(),  FT.data(),   GT.data(), lam.data(), FeT.data(), FoT.data(),
+                             GeT.data(), GoT.data(), lamf.data(), Fe.data(), Fo.data(),  Ge.data(),  Go.data()};
+    double* dst[14] = {c->F,   c->G,   c->FT,  c->GT, c->lam, c->FeT, c->FoT,
+                       c->GeT, c->GoT, c->lamf, c->Fe, c->Fo,  c->Ge,  c->Go};
+    const size_t cnt[14] = {mm, mm, mm, mm, (size_t)m, hh, hh, hh, hh, lamf.size(), hl, hl, hl, hl};
+    for (int k = 0; k < 14 && e == cudaSuccess; ++k)
         if (cnt[k]) e = cudaMemcpy(dst[k], src[k], sizeof(double) * cnt[k], cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         cudaFree(buf);
@@ -348,21 +379,139 @@ __device__ __forceinline__ double rhs_value(const R* __restrict__ T, const R* __
     return s;
 }
 
-// FOLD: each row holds s_i = b_i + b_{mx-1-i} at i < mx/2 and d_i = b_i - b_{mx-1-i} at mx/2 + i.
-template <typename R, bool FOLD>
-__global__ void rhs_kernel(const R* __restrict__ T, const R* __restrict__ Q, double* __restrict__ b, const HeatArgs a) {
-    const int w = FOLD ? a.mx / 2 : a.mx;  // work items per row
-    const size_t plane = (size_t)w * a.my, total = plane * a.nz;
+// Which directions the transforms fold: fx the x direction, ft the other transformed one (0 none,
+// 1 y, 2 z); wx, wy, wz the half counts along the folded directions.  A folded direction of m
+// points holds the sums v_q + v_{m-1-q} (the middle point alone where m is odd) in its first
+// ceil(m/2) places and the differences v_q - v_{m-1-q} in the others.
+struct Fold {
+    int fx, ft, wx, wy, wz;
+};
+struct FoldItem {
+    int i, j, z;    // the item's point
+    int j2, z2;     // its mirror image along the folded y or z (equal: none, or the middle)
+    int jd, zd;     // where the differences go
+    bool pair;
+};
+__device__ __forceinline__ FoldItem fold_item(const Fold& f, const HeatArgs& a, size_t c) {
+    FoldItem t;
+    t.i = (int)(c % f.wx);
+    const size_t r = c / f.wx;
+    t.j = (int)(r % f.wy);
+    t.z = (int)(r / f.wy);
+    t.j2 = f.ft == 1 ? a.my - 1 - t.j : t.j;
+    t.z2 = f.ft == 2 ? a.nz - 1 - t.z : t.z;
+    t.jd = f.ft == 1 ? f.wy + t.j : t.j;
+    t.zd = f.ft == 2 ? f.wz + t.z : t.z;
+    t.pair = t.j2 != t.j || t.z2 != t.z;
+    return t;
+}
+
+template <typename R, bool FX>
+__global__ void rhs_kernel(const R* __restrict__ T, const R* __restrict__ Q, double* __restrict__ b, const HeatArgs a,
+                           const Fold f) {
+    const size_t total = (size_t)f.wx * f.wy * f.wz;
     for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < total; c += (size_t)gridDim.x * blockDim.x) {
-        const int i = (int)(c % w), j = (int)((c / w) % a.my), z = (int)(c / plane);
-        const size_t row = ((size_t)z * a.my + j) * a.mx;
-        if (FOLD) {
-            const double b1 = rhs_value<R>(T, Q, a, i, j, z), b2 = rhs_value<R>(T, Q, a, a.mx - 1 - i, j, z);
-            b[row + i] = b1 + b2;
-            b[row + w + i] = b1 - b2;
+        const FoldItem t = fold_item(f, a, c);
+        auto put = [&](int j, int z, double v0, double v1) {  // a row's entries of points i and mx-1-i
+            double* row = b + ((size_t)z * a.my + j) * a.mx;
+            row[t.i] = FX ? v0 + v1 : v0;
+            if (FX) row[f.wx + t.i] = v0 - v1;
+        };
+        const double e0 = rhs_value<R>(T, Q, a, t.i, t.j, t.z);
+        const double e1 = FX ? rhs_value<R>(T, Q, a, a.mx - 1 - t.i, t.j, t.z) : 0.0;
+        if (t.pair) {
+            const double m0 = rhs_value<R>(T, Q, a, t.i, t.j2, t.z2);
+            const double m1 = FX ? rhs_value<R>(T, Q, a, a.mx - 1 - t.i, t.j2, t.z2) : 0.0;
+            put(t.j, t.z, e0 + m0, e1 + m1);
+            put(t.jd, t.zd, e0 - m0, e1 - m1);
         } else {
-            b[row + i] = rhs_value<R>(T, Q, a, i, j, z);
+            put(t.j, t.z, e0, e1);
         }
+    }
+}
+
+// The modes of the z operator (m = nz points, Robin at both ends with Biot number bi), one block
+// per mode.  With c = (m-1)/2 the eigenvectors are v_i = cos(theta (i-c)) (even) and
+// sin(theta (i-c)) (odd), eigenvalue 4 sin^2(theta/2) / dz^2; the end rows give
+//   sin(theta) tan(e) = bi,  theta c = k pi + e (even, k = 0..) or (k + 1/2) pi + e (odd),
+// with 0 <= e < pi/2, except for the mode with theta = pi at bi = 0, which becomes
+// v_i = (-1)^i cosh(eta (i-c)), sinh(eta) tanh(eta c) = bi, eigenvalue 4 cosh^2(eta/2) / dz^2.
+// The phase k pi (i-c)/c is reduced in integers, so the entries are good to rounding.  In the
+// weights s_i^2 = 1, 2, .., 2, 1 of the symmetric form, F[k][i] = s_i^2 v_i / |v| and
+// G[i][k] = v_i / |v| with |v|^2 = sum s_i^2 v_i^2.  Even modes first; halves as in OpMats.
+__global__ void __launch_bounds__(128) z_modes_kernel(int m, double bi, double idz2, double* __restrict__ lam,
+                                                      double* __restrict__ Fe, double* __restrict__ Fo,
+                                                      double* __restrict__ Ge, double* __restrict__ Go, int lde, int ldo) {
+    const int he = (m + 1) / 2, mode = blockIdx.x, odd = mode >= he, k = odd ? mode - he : mode;
+    const int h = odd ? m / 2 : he;                  // points of the half
+    const bool top = mode == (m & 1 ? he - 1 : m - 1);  // the last mode of the parity that holds (-1)^i
+    const double c = 0.5 * (m - 1), half_pi = 1.57079632679489661923, pi = 3.14159265358979323846;
+    // root of an increasing function on (lo, hi) by Newton steps kept inside the bracket
+    double root, lo = 0.0, hi;
+    if (top) {
+        hi = 2.0 * (asinh(bi) + sqrt(bi / c));  // above the root
+        root = bi > 0.0 ? fmin(hi, fmax(asinh(bi), sqrt(bi / c))) : 0.0;
+    } else {
+        hi = half_pi;
+        const double th0 = (k + 0.5 * odd) * pi / c;
+        root = th0 > 0.0 ? atan(bi / sin(th0)) : fmin(sqrt(bi * c), 1.5);
+    }
+    for (int it = 0; it < 80 && bi > 0.0; ++it) {
+        double g, dg;
+        if (top) {
+            const double t = tanh(root * c);
+            g = sinh(root) * t - bi;
+            dg = cosh(root) * t + sinh(root) * c * (1.0 - t * t);
+        } else {
+            double sn, cs, se, ce;
+            sincos(((k + 0.5 * odd) * pi + root) / c, &sn, &cs);
+            sincos(root, &se, &ce);
+            g = sn * se - bi * ce;
+            dg = cs * se / c + sn * ce + bi * se;
+        }
+        if (g > 0.0) hi = root;
+        else lo = root;
+        double next = dg > 0.0 ? root - g / dg : 0.5 * (lo + hi);
+        if (!(next >= lo && next <= hi)) next = 0.5 * (lo + hi);
+        const double step = fabs(next - root);
+        root = next;
+        if (step <= 2e-16 * root) break;
+    }
+    const int n1 = m - 1;
+    auto value = [&](int i) -> double {  // v_i
+        const int r = 2 * i - n1;        // (i - c) / c = r / n1
+        if (top) {
+            const double x = fabs(0.5 * r) * root;  // eta |i - c|; cosh over cosh(eta c), no overflow
+            const double v = exp(x - root * c) * (1.0 + exp(-2.0 * x)) / (1.0 + exp(-2.0 * root * c));
+            return (i & 1) ? -v : v;
+        }
+        const long long q = ((long long)(2 * k + odd) * r) % (4ll * n1);  // phase = pi q / (2 n1) + e r / n1
+        const double ph = (double)q / (2.0 * n1) + root / pi * ((double)r / n1);
+        return odd ? sinpi(ph) : cospi(ph);
+    };
+    double sum = 0.0;
+    for (int i = threadIdx.x; i < m; i += 128) {
+        const double v = value(i);
+        sum += (i == 0 || i == n1 ? 1.0 : 2.0) * v * v;
+    }
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    __shared__ double part[4];
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = sum;
+    __syncthreads();
+    const double nrm = 1.0 / sqrt(part[0] + part[1] + part[2] + part[3]);
+    double* F = odd ? Fo : Fe;
+    double* G = odd ? Go : Ge;
+    const int ld = odd ? ldo : lde;
+    for (int i = threadIdx.x; i < ld; i += 128) {
+        const double v = i < h ? value(i) * nrm : 0.0;  // zero in the row's padding
+        F[(size_t)k * ld + i] = (i == 0 || i == n1 ? 1.0 : 2.0) * v;
+        if (i < h) G[(size_t)i * ld + k] = v;
+    }
+    if (k == h - 1 && ld > h)  // and the padding column of G
+        for (int i = threadIdx.x; i < h; i += 128) G[(size_t)i * ld + h] = 0.0;
+    if (threadIdx.x == 0) {
+        const double q = top ? cosh(0.5 * root) : sin(0.5 * ((k + 0.5 * odd) * pi + root) / c);
+        lam[mode] = 4.0 * q * q * idz2;
     }
 }
 
@@ -416,7 +565,8 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB)
     A += blockIdx.z * sA;
     B += blockIdx.z * sB;
     C += blockIdx.z * sC;
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    // the few tiles of the short side run side by side and share the long operand's slices in L2
+    const int m0 = (M < N ? blockIdx.x : blockIdx.y) * BM, n0 = (M < N ? blockIdx.y : blockIdx.x) * BN;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
     const int wm = (warp % Cfg::WR) * 16 * MI, wn = (warp / Cfg::WR) * 8 * NJ;  // this warp's part of the tile
@@ -497,50 +647,61 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MINB)
         }
 }
 
-// 3. For every mode t = j * mx + i: (Az + lambda_x[i] + lambda_y[j]) u = f along z, Thomas
-// elimination (the system is diagonally dominant: lambda_x + lambda_y > 0 whenever a direction
-// has a Dirichlet end or a Robin end with Bi > 0, which every boundary model has).  f and then
-// u in v; the eliminated upper diagonal in cp.  Both sweeps load kThomasChunk planes ahead of
-// the dependent recurrence, so each thread keeps that many loads in flight.
-constexpr int kThomasChunk = 4;
+// 3. For every pair of modes (a, b), a = kx: (As + la[a] + lb[b]) u = f along s, Thomas elimination
+// (diagonally dominant: the eigenvalues' sum is positive whenever a transformed direction has a
+// Dirichlet end or a Robin end with Bi > 0; along the eliminated one the rows are dominant by
+// themselves).  Line (a, b) starts at b * stride_b + a and has `len` points `stride` apart; each
+// end is next to a Dirichlet voxel or a Robin face.  f and then u in v; the eliminated upper
+// diagonal in cp.  Both sweeps load kThomasChunk points ahead of the dependent recurrence, so
+// each thread keeps that many loads in flight.
+constexpr int kThomasChunk = 8;
 
-__global__ void thomas_kernel(double* __restrict__ v, double* __restrict__ cp, const double* __restrict__ lx,
-                              const double* __restrict__ ly, int mx, int my, int nz, double idz2, double biz) {
-    const size_t plane = (size_t)mx * my;
-    for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < plane; t += (size_t)gridDim.x * blockDim.x) {
-        const double lam = lx[t % mx] + ly[t / mx];
-        const double a_end = 2.0 * (1.0 + biz) * idz2 + lam;  // Robin rows z = 0, nz - 1
-        const double a_in = 2.0 * idz2 + lam;
+struct ThomasArgs {
+    int na, nb, len, lo_robin, hi_robin;
+    size_t stride_b, stride;
+    double id2, bi;
+};
+
+__global__ void thomas_kernel(double* __restrict__ v, double* __restrict__ cp, const double* __restrict__ la,
+                              const double* __restrict__ lb, const ThomasArgs p) {
+    const size_t lines = (size_t)p.na * p.nb;
+    const int len = p.len;
+    for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < lines; t += (size_t)gridDim.x * blockDim.x) {
+        const int a = (int)(t % p.na), b = (int)(t / p.na);
+        const double lam = la[a] + lb[b];
+        const double a_in = 2.0 * p.id2 + lam, a_rob = 2.0 * (1.0 + p.bi) * p.id2 + lam;
+        const size_t base = (size_t)b * p.stride_b + a;
         double c = 0.0, d = 0.0;
-        for (int z0 = 0; z0 < nz; z0 += kThomasChunk) {
+        for (int z0 = 0; z0 < len; z0 += kThomasChunk) {
             double f[kThomasChunk];
 #pragma unroll
             for (int q = 0; q < kThomasChunk; ++q)
-                if (z0 + q < nz) f[q] = v[(size_t)(z0 + q) * plane + t];
+                if (z0 + q < len) f[q] = v[base + (size_t)(z0 + q) * p.stride];
 #pragma unroll
             for (int q = 0; q < kThomasChunk; ++q) {
                 const int z = z0 + q;
-                if (z >= nz) break;
-                const bool first = z == 0, last = z == nz - 1;
-                const double lo = first ? 0.0 : (last ? -2.0 * idz2 : -idz2);
-                const double up = last ? 0.0 : (first ? -2.0 * idz2 : -idz2);
-                const double r = 1.0 / ((first || last ? a_end : a_in) - lo * c);
+                if (z >= len) break;
+                const bool first = z == 0, last = z == len - 1;
+                const bool rob = (first && p.lo_robin) || (last && p.hi_robin);
+                const double lo = first ? 0.0 : (last && p.hi_robin ? -2.0 * p.id2 : -p.id2);
+                const double up = last ? 0.0 : (first && p.lo_robin ? -2.0 * p.id2 : -p.id2);
+                const double r = 1.0 / ((rob ? a_rob : a_in) - lo * c);
                 c = up * r;
                 d = (f[q] - lo * d) * r;
-                const size_t o = (size_t)z * plane + t;
+                const size_t o = base + (size_t)z * p.stride;
                 cp[o] = c;
                 v[o] = d;
             }
         }
-        double u = d;  // u at z = nz - 1
-        for (int z1 = nz - 1; z1 > 0; z1 -= kThomasChunk) {  // z = z1 - 1 down to z1 - kThomasChunk
+        double u = d;  // u at the last point
+        for (int z1 = len - 1; z1 > 0; z1 -= kThomasChunk) {  // points z1 - 1 down to z1 - kThomasChunk
             double dv[kThomasChunk], cv[kThomasChunk];
 #pragma unroll
             for (int q = 0; q < kThomasChunk; ++q) {
                 const int z = z1 - 1 - q;
                 if (z >= 0) {
-                    dv[q] = v[(size_t)z * plane + t];
-                    cv[q] = cp[(size_t)z * plane + t];
+                    dv[q] = v[base + (size_t)z * p.stride];
+                    cv[q] = cp[base + (size_t)z * p.stride];
                 }
             }
 #pragma unroll
@@ -548,7 +709,7 @@ __global__ void thomas_kernel(double* __restrict__ v, double* __restrict__ cp, c
                 const int z = z1 - 1 - q;
                 if (z < 0) break;
                 u = dv[q] - cv[q] * u;
-                v[(size_t)z * plane + t] = u;
+                v[base + (size_t)z * p.stride] = u;
             }
         }
     }
@@ -556,20 +717,31 @@ __global__ void thomas_kernel(double* __restrict__ v, double* __restrict__ cp, c
 
 __device__ __forceinline__ double nan_max(double a, double b) { return (b > a || b != b) ? b : a; }
 
-// 4'. Folded x transform: each row of the inverse transform's output holds P at i < mx/2 and Q
-// at mx/2 + i; the solution row is u_i = P_i + Q_i, u_{mx-1-i} = P_i - Q_i.  One streaming pass
-// into the other volume, so that the finishing pass reads one value per neighbour.
-__global__ void unfold_kernel(const double* __restrict__ pq, double* __restrict__ u, size_t rows, int mx) {
-    const int h = mx / 2;
-    const size_t items = rows * (size_t)h;
-    for (size_t it = blockIdx.x * (size_t)blockDim.x + threadIdx.x; it < items; it += (size_t)gridDim.x * blockDim.x) {
-        const size_t r = it / h;
-        const int i = (int)(it % h);
-        const double* src = pq + r * mx;
-        double* dst = u + r * mx;
-        const double pv = src[i], qv = src[h + i];
-        dst[i] = pv + qv;
-        dst[mx - 1 - i] = pv - qv;
+// 4'. From the folded transforms' output (a folded direction holds its even part P in the places
+// of the sums and its odd part Q in those of the differences: u_q = P + Q, u_{m-1-q} = P - Q) to
+// the solution, in one streaming pass into the other volume, so that the finishing pass reads
+// one value per neighbour.
+template <bool FX>
+__global__ void unfold_kernel(const double* __restrict__ pq, double* __restrict__ u, const HeatArgs a, const Fold f) {
+    const size_t total = (size_t)f.wx * f.wy * f.wz;
+    for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < total; c += (size_t)gridDim.x * blockDim.x) {
+        const FoldItem t = fold_item(f, a, c);
+        auto at = [&](int j, int z) { return ((size_t)z * a.my + j) * a.mx; };
+        auto put = [&](int j, int z, double p, double q) {
+            double* row = u + at(j, z);
+            row[t.i] = FX ? p + q : p;
+            if (FX) row[a.mx - 1 - t.i] = p - q;
+        };
+        const size_t re = at(t.j, t.z);
+        const double pe = pq[re + t.i], qe = FX ? pq[re + f.wx + t.i] : 0.0;
+        if (t.pair) {
+            const size_t rd = at(t.jd, t.zd);
+            const double pd = pq[rd + t.i], qd = FX ? pq[rd + f.wx + t.i] : 0.0;
+            put(t.j, t.z, pe + pd, qe + qd);
+            put(t.j2, t.z2, pe - pd, qe - qd);
+        } else {
+            put(t.j, t.z, pe, qe);
+        }
     }
 }
 
@@ -663,8 +835,8 @@ __global__ void __launch_bounds__(256, 3) finish_kernel(R* __restrict__ T, const
     }
 }
 
-// C = A B over `batch` matrices (see dgemm_kernel); M is split into launches of at most 65535
-// row tiles.
+// C = A B over `batch` matrices (see dgemm_kernel); the longer side is split into launches of at
+// most 65535 tiles.
 template <class Cfg>
 cudaError_t gemm_tiles(const double* A, const double* B, double* C, int M, int N, int K, int lda, int ldb, int ldc,
                        int batch, long long sA, long long sB, long long sC, cudaStream_t s) {
@@ -674,12 +846,14 @@ cudaError_t gemm_tiles(const double* A, const double* B, double* C, int M, int N
         return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM);
     });
     if (ae != cudaSuccess) return ae;
-    const int max_rows = 65535 * Cfg::BM;
-    for (int r0 = 0; r0 < M; r0 += max_rows) {
-        const int rows = std::min(M - r0, max_rows);
-        const dim3 grid((unsigned)((N + Cfg::BN - 1) / Cfg::BN), (unsigned)((rows + Cfg::BM - 1) / Cfg::BM), (unsigned)batch);
-        kern<<<grid, Cfg::THREADS, Cfg::SMEM, s>>>(A + (size_t)r0 * lda, B, C + (size_t)r0 * ldc, rows, N, K, lda, ldb, ldc,
-                                                   sA, sB, sC);
+    const bool wide = M < N;
+    const int span = 65535 * (wide ? Cfg::BN : Cfg::BM), total = wide ? N : M;
+    for (int o = 0; o < total; o += span) {
+        const int part = std::min(total - o, span), m = wide ? M : part, n = wide ? part : N;
+        const unsigned mt = (unsigned)((m + Cfg::BM - 1) / Cfg::BM), nt = (unsigned)((n + Cfg::BN - 1) / Cfg::BN);
+        const dim3 grid(wide ? mt : nt, wide ? nt : mt, (unsigned)batch);
+        kern<<<grid, Cfg::THREADS, Cfg::SMEM, s>>>(A + (wide ? 0 : (size_t)o * lda), B + (wide ? o : 0),
+                                                   C + (wide ? o : (size_t)o * ldc), m, n, K, lda, ldb, ldc, sA, sB, sC);
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
@@ -701,6 +875,30 @@ cudaError_t gemm(const double* A, const double* B, double* C, int M, int N, int 
     return gemm_tiles<GemmSmall>(A, B, C, M, N, K, lda, ldb, ldc, batch, sA, sB, sC, s);
 }
 
+// Microseconds that `products` products per point (4 flops each, there and back) take at the
+// 28 TFLOP/s the large tiles reach.
+double transform_us(double vol, double products) { return 4.0 * vol * products / 28e6; }
+
+// Whether y's transform is folded (a symmetric operator): half the products, but two launches for
+// one and smaller tiles, so only where the products saved take 50 us.  126x126x200 measured 301 us
+// whole, 313 us folded (29 us of products saved), 94x94x37 92 / 103 us.
+bool folds_y(const HeatGrid& g) {
+    return g.oy.lo_robin == g.oy.hi_robin && g.my % 2 == 0 &&
+           transform_us((double)g.mx * g.my * g.nz, 0.5 * g.my) >= 50.0;
+}
+
+// The direction transformed beside x: 1 y, 2 z, by modelled time: the transform's products, and the
+// elimination's dependent rows along the other direction, about 0.25 us each however many
+// lines run side by side; z where that takes less than 0.7 of it.  Measured solves, y against z
+// transformed: 512x512x501 16.5 / 12.7 ms, 512x512x64 2145 / 1289 us, 256x256x60 401 / 327 us,
+// and where y is kept 192x192x60 217 / 212 us, 128x128x100 156 / 159 us, 126x126x200 301 / 317 us.
+int axis_of(const HeatGrid& g) {
+    const double vol = (double)g.mx * g.my * g.nz;
+    const double ty = transform_us(vol, folds_y(g) ? 0.5 * g.my : g.my) + 0.25 * g.nz;
+    const double tz = transform_us(vol, 0.5 * g.nz) + 0.25 * g.my;
+    return tz < 0.7 * ty ? 2 : 1;
+}
+
 int grid_for(size_t work, int threads) {
     return (int)std::max<size_t>(1, std::min<size_t>((work + threads - 1) / threads, (size_t)148 * 16));
 }
@@ -714,26 +912,32 @@ HeatDirect::~HeatDirect() {
 void HeatDirect::release(cudaStream_t s) {
     if (ws_) cudaFreeAsync(ws_, s);
     ws_ = nullptr;
-    cap_ = 0;
+    cap_ = size_ = 0;
 }
 
 template <typename R>
 shg_status HeatDirect::solve(const shg_params& p, R* T, const R* Q, double t_inf, cudaStream_t s) {
     const HeatGrid g = heat_grid(p);
     if (g.nz > 65535) return fail(SHG_ERR_UNSUPPORTED, "direct heat solve: nz = %d above 65535", g.nz);
+    const int axis = axis_of(g);
     const OpMats *ox = nullptr, *oy = nullptr;
     shg_status rc;
-    if ((rc = get_op(g.ox, &ox)) != SHG_OK || (rc = get_op(g.oy, &oy)) != SHG_OK) return rc;
+    if ((rc = get_op(g.ox, &ox)) != SHG_OK || (axis == 1 && (rc = get_op(g.oy, &oy)) != SHG_OK)) return rc;
     const size_t vol = (size_t)g.mx * g.my * g.nz;
+    // z modes: even and odd halves of F and G, eigenvalues
+    const int he = (g.nz + 1) / 2, ho = g.nz / 2, lde = he + (he & 1), ldo = ho + (ho & 1);
+    const size_t zmodes = axis == 2 ? 2 * ((size_t)he * lde + (size_t)ho * ldo) + g.nz : 0;
+    const size_t need = 2 * (vol + (vol & 1)) + 4 + zmodes;
     cudaError_t e;
-    if (vol > cap_) {
+    if (need > size_) {
         release(s);
-        if ((e = dev_alloc((void**)&ws_, sizeof(double) * (2 * vol + 4), s)) != cudaSuccess) {
+        if ((e = dev_alloc((void**)&ws_, sizeof(double) * need, s)) != cudaSuccess) {
             ws_ = nullptr;
             return cuda_fail(e, "cudaMallocAsync");
         }
-        cap_ = vol;
+        size_ = need;
     }
+    cap_ = vol + (vol & 1);
     nt_ = (size_t)g.n * g.n * g.nz;
     double* X = ws_;
     double* Y = ws_ + cap_;
@@ -763,44 +967,73 @@ shg_status HeatDirect::solve(const shg_params& p, R* T, const R* Q, double t_inf
     const int mx = g.mx, my = g.my, nz = g.nz;
     const long long pl = (long long)mx * my;
     if ((e = cudaMemsetAsync(out, 0, 4 * sizeof(double), s)) != cudaSuccess) return cuda_fail(e, "memset");
-    const bool fold = ox->fold;
+    const bool fx = ox->fold;
     const int h = mx / 2;
-    if (fold) rhs_kernel<R, true><<<grid_for(vol / 2, 256), 256, 0, s>>>(T, Q, X, a);
-    else rhs_kernel<R, false><<<grid_for(vol, 256), 256, 0, s>>>(T, Q, X, a);
+    Fold f;
+    f.fx = fx;
+    f.ft = axis == 2 ? 2 : folds_y(g) ? 1 : 0;
+    f.wx = fx ? h : mx;
+    f.wy = f.ft == 1 ? my / 2 : my;
+    f.wz = f.ft == 2 ? he : nz;
+    const size_t fitems = (size_t)f.wx * f.wy * f.wz;
+    if (fx) rhs_kernel<R, true><<<grid_for(fitems, 256), 256, 0, s>>>(T, Q, X, a, f);
+    else rhs_kernel<R, false><<<grid_for(fitems, 256), 256, 0, s>>>(T, Q, X, a, f);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "heat right-hand side");
-    // into mode space: along x (rows of X; folded, the even modes from the sums and the odd
-    // ones from the differences, half the work), then along y (one product per z plane)
-    // (folded: the even and odd halves as a batch of two, FoT = FeT + h*h)
+    double *zFe = out + 4, *zFo = zFe + (size_t)he * lde, *zGe = zFo + (size_t)ho * ldo, *zGo = zGe + (size_t)he * lde,
+           *zlam = zGo + (size_t)ho * ldo;
+    if (axis == 2) {
+        z_modes_kernel<<<nz, 128, 0, s>>>(nz, a.biz, a.idz2, zlam, zFe, zFo, zGe, zGo, lde, ldo);
+        if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "heat z modes");
+    }
+    // the transforms: along x from rows, folded as a batch of two halves (FoT = FeT + h*h); along y
+    // one product per z plane, along z one over all columns, each half by itself when folded
     const long long hh = (long long)h * h;
-    if (fold) {
-        e = gemm(X, ox->FeT, Y, nz * my, h, h, mx, h, mx, 2, h, hh, h, s);
-    } else {
-        e = gemm(X, ox->FT, Y, nz * my, mx, mx, mx, ox->ld, mx, 1, 0, 0, 0, s);
-    }
-    if (e != cudaSuccess || (e = gemm(oy->F, Y, X, my, mx, my, oy->ld, mx, mx, nz, 0, pl, pl, s)) != cudaSuccess)
+    auto along_x = [&](const double* eT, const double* full, const double* from, double* to) {
+        return fx ? gemm(from, eT, to, nz * my, h, h, mx, h, mx, 2, h, hh, h, s)
+                  : gemm(from, full, to, nz * my, mx, mx, mx, ox->ld, mx, 1, 0, 0, 0, s);
+    };
+    auto along_t = [&](const double* full, const double* even, const double* odd, const double* from, double* to) {
+        if (axis == 2) {
+            if (he == ho)
+                return gemm(even, from, to, he, (int)pl, he, lde, (int)pl, (int)pl, 2, odd - even, he * pl, he * pl, s);
+            const cudaError_t e1 = gemm(even, from, to, he, (int)pl, he, lde, (int)pl, (int)pl, 1, 0, 0, 0, s);
+            return e1 != cudaSuccess ? e1
+                                     : gemm(odd, from + he * pl, to + he * pl, ho, (int)pl, ho, ldo, (int)pl, (int)pl, 1, 0, 0, 0, s);
+        }
+        if (f.ft == 0) return gemm(full, from, to, my, mx, my, oy->ld, mx, mx, nz, 0, pl, pl, s);
+        const int w = my / 2;
+        const size_t off = (size_t)w * mx;
+        const cudaError_t e1 = gemm(even, from, to, w, mx, w, oy->ldl, mx, mx, nz, 0, pl, pl, s);
+        return e1 != cudaSuccess ? e1 : gemm(odd, from + off, to + off, w, mx, w, oy->ldl, mx, mx, nz, 0, pl, pl, s);
+    };
+    if ((e = along_x(ox->FeT, ox->FT, X, Y)) != cudaSuccess ||
+        (e = axis == 2 ? along_t(nullptr, zFe, zFo, Y, X) : along_t(oy->F, oy->Fe, oy->Fo, Y, X)) != cudaSuccess)
         return cuda_fail(e, "heat transform");
-    thomas_kernel<<<grid_for((size_t)pl, 128), 128, 0, s>>>(X, Y, fold ? ox->lamf : ox->lam, oy->lam, mx, my, nz, a.idz2,
-                                                             a.biz);
+    ThomasArgs ta;
+    ta.na = mx;
+    ta.nb = axis == 2 ? nz : my;
+    ta.len = axis == 2 ? my : nz;
+    ta.stride_b = axis == 2 ? (size_t)pl : (size_t)mx;
+    ta.stride = axis == 2 ? (size_t)mx : (size_t)pl;
+    ta.lo_robin = axis == 2 ? g.oy.lo_robin : 1;
+    ta.hi_robin = axis == 2 ? g.oy.hi_robin : 1;
+    ta.id2 = axis == 2 ? a.idy2 : a.idz2;
+    ta.bi = axis == 2 ? a.biy : a.biz;
+    thomas_kernel<<<grid_for((size_t)ta.na * ta.nb, 128), 128, 0, s>>>(X, Y, fx ? ox->lamf : ox->lam,
+                                                                        axis == 2 ? zlam : oy->lam, ta);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "heat tridiagonal solve");
-    // back to voxels: along y, then along x (folded: P from the even modes, Q from the odd;
-    // the finishing pass combines them)
-    if ((e = gemm(oy->G, X, Y, my, mx, my, oy->ld, mx, mx, nz, 0, pl, pl, s)) != cudaSuccess)
+    if ((e = axis == 2 ? along_t(nullptr, zGe, zGo, X, Y) : along_t(oy->G, oy->Ge, oy->Go, X, Y)) != cudaSuccess ||
+        (e = along_x(ox->GeT, ox->GT, Y, X)) != cudaSuccess)
         return cuda_fail(e, "heat transform");
-    if (fold) {
-        e = gemm(Y, ox->GeT, X, nz * my, h, h, mx, h, mx, 2, h, hh, h, s);
-    } else {
-        e = gemm(Y, ox->GT, X, nz * my, mx, mx, mx, ox->ld, mx, 1, 0, 0, 0, s);
-    }
-    if (e != cudaSuccess) return cuda_fail(e, "heat transform");
-    const int zc = finish_planes((size_t)pl, nz);
-    const size_t fitems = (size_t)pl * ((nz + zc - 1) / zc);
-    const int fb = grid_for(fitems, 256);
     const double* u = X;
-    if (fold) {
-        unfold_kernel<<<grid_for((size_t)nz * my * h, 256), 256, 0, s>>>(X, Y, (size_t)nz * my, mx);
+    if (fx || f.ft) {
+        if (fx) unfold_kernel<true><<<grid_for(fitems, 256), 256, 0, s>>>(X, Y, a, f);
+        else unfold_kernel<false><<<grid_for(fitems, 256), 256, 0, s>>>(X, Y, a, f);
         if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "heat solution");
         u = Y;
     }
+    const int zc = finish_planes((size_t)pl, nz);
+    const int fb = grid_for((size_t)pl * ((nz + zc - 1) / zc), 256);
     if (p.boundary == SHG_BOUNDARY_TOP_OPEN)
         finish_kernel<R, SHG_BOUNDARY_TOP_OPEN><<<fb, 256, 0, s>>>(T, Q, u, a, k, zc, out);
     else

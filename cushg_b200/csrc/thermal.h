@@ -76,8 +76,9 @@ class HeatDirect {
     void release(cudaStream_t s);
 
   private:
-    double* ws_ = nullptr;  // two compact FP64 volumes, then the four reduction slots
-    size_t cap_ = 0;        // doubles per volume
+    double* ws_ = nullptr;  // two compact FP64 volumes, the four reduction slots, the z modes
+    size_t size_ = 0;       // doubles allocated
+    size_t cap_ = 0;        // doubles per volume of the latest solve
     size_t nt_ = 0;         // voxels of the latest solve
 };
 

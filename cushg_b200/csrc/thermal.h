@@ -39,6 +39,15 @@ cudaError_t launch_jacobi(const R* Ti, R* Tf, const R* Q, const JacobiCoef<R>& k
                           double* partial, double* out, cudaStream_t s);
 size_t jacobi_partials(const shg_params& p);
 
+// `count` unchecked sweeps in one cooperative launch with T in shared memory (jacobi_resident.cu),
+// for grids that fit: from Ta, which with Tb holds the faces between tiles meanwhile, into Ta
+// (count even) or Tb (odd).  Arrays 2-real aligned; bar: a scratch word; *err is set to 1 if a
+// barrier wait ran out.
+template <typename R> bool jacobi_resident_fits(const JacobiCoef<R>& k);
+template <typename R>
+cudaError_t launch_jacobi_resident(R* Ta, R* Tb, const R* Q, const JacobiCoef<R>& k, int boundary, int count, unsigned* bar,
+                                   unsigned* err, cudaStream_t s);
+
 // Temporally blocked sweeps (jacobi_tb.cu): `depth` (2..4) sweeps Ti -> Tf in one launch,
 // with Ti and Q read through 3D TMA maps made by make_tb_map.  *err is set to 1 if a
 // staged plane never arrived.

@@ -74,6 +74,30 @@ cudaError_t run_sweeps(R*& cur, R*& nxt, const R* Ta, const SweepMaps<R>& m, con
     return cudaSuccess;
 }
 
+// Whether `count` unchecked sweeps run in one launch of the resident kernel: the automatic depth,
+// a grid that fits, and enough sweeps to pay for reading and writing T once and a cooperative
+// launch.
+constexpr int64_t kResidentMin = 8;
+template <typename R>
+bool resident(const shg_params& p, const JacobiCoef<R>& k, int64_t count) {
+    return p.jacobi_block == 0 && count >= kResidentMin && jacobi_resident_fits<R>(k);
+}
+
+// `count` unchecked sweeps on the resident kernel; cur / nxt as run_sweeps leaves them.  err[1] is
+// the kernel's barrier word.
+template <typename R>
+cudaError_t run_resident(R*& cur, R*& nxt, const R* Q, const JacobiCoef<R>& k, int boundary, int64_t count, unsigned* err,
+                         cudaStream_t s) {
+    while (count > 0) {
+        const int t = (int)std::min<int64_t>(count, 1 << 24);
+        const cudaError_t e = launch_jacobi_resident<R>(cur, nxt, Q, k, boundary, t, err + 1, err, s);
+        if (e != cudaSuccess) return e;
+        if (t & 1) std::swap(cur, nxt);
+        count -= t;
+    }
+    return cudaSuccess;
+}
+
 // One instance of a thermal run: its buffers, its Jacobi state and its latest optical pass.
 template <typename R>
 struct ThermalInst {
@@ -116,6 +140,7 @@ constexpr int64_t kSweepGraphMin = 64;
 template <typename R>
 cudaError_t run_sweeps_graphed(ThermalInst<R>& t, int64_t count, cudaStream_t s) {
     const shg_params& p = *t.p;
+    if (resident<R>(p, t.k, count)) return run_resident<R>(t.cur, t.nxt, t.Q, t.k, p.boundary, count, t.tb_err, s);
     if (t.depth > 1 || count < kSweepGraphMin)
         return run_sweeps<R>(t.cur, t.nxt, t.Ta, t.maps, t.Q, t.k, p.boundary, t.depth, count, t.tb_err, s);
     const int parity = t.cur == t.Ta ? 0 : 1;
@@ -253,7 +278,7 @@ shg_status ti_jacobi(ThermalInst<R>& t, HeatDirect* heat, cudaStream_t s) {
             return cuda_fail(e, "jacobi residual");
         unsigned staged_err = 0;
         std::memcpy(&staged_err, &h[1], sizeof(staged_err));
-        if (staged_err) return fail(SHG_ERR_CUDA, "blocked Jacobi sweep: a staged plane did not arrive");
+        if (staged_err) return fail(SHG_ERR_CUDA, "Jacobi sweeps: a bounded wait (staged plane or grid barrier) ran out");
         *out = h[0];
         return SHG_OK;
     };
@@ -501,16 +526,20 @@ shg_status heat_run(const shg_params& p, R* T, const R* Q, int64_t sweeps, cudaS
     do {
         SweepMaps<R> maps;
         if (depth > 1 && (rc = make_sweep_maps<R>(T, other, Q, n, nz, &maps)) != SHG_OK) break;
-        // both buffers start alike, so the voxels no sweep writes (Dirichlet faces) agree
-        if ((e = cudaMemcpyAsync(other, T, arr, cudaMemcpyDeviceToDevice, s)) != cudaSuccess ||
+        const JacobiCoef<R> k = make_jacobi_coef<R>(p);
+        const bool res = resident<R>(p, k, sweeps);
+        // both buffers start alike, so the voxels no sweep writes (Dirichlet faces) agree (the
+        // resident kernel writes them too)
+        if ((!res && (e = cudaMemcpyAsync(other, T, arr, cudaMemcpyDeviceToDevice, s)) != cudaSuccess) ||
             (e = cudaMemsetAsync(tb_err, 0, sizeof(unsigned), s)) != cudaSuccess) {
             rc = cuda_fail(e, "heat sweeps set-up");
             break;
         }
-        const JacobiCoef<R> k = make_jacobi_coef<R>(p);
         R* cur = T;
         R* nxt = other;
-        if ((e = run_sweeps<R>(cur, nxt, T, maps, Q, k, p.boundary, depth, sweeps, tb_err, s)) != cudaSuccess) {
+        e = res ? run_resident<R>(cur, nxt, Q, k, p.boundary, sweeps, tb_err, s)
+                : run_sweeps<R>(cur, nxt, T, maps, Q, k, p.boundary, depth, sweeps, tb_err, s);
+        if (e != cudaSuccess) {
             rc = cuda_fail(e, "jacobi sweep");
             break;
         }
@@ -524,7 +553,7 @@ shg_status heat_run(const shg_params& p, R* T, const R* Q, int64_t sweeps, cudaS
             rc = cuda_fail(e, "heat sweeps");
             break;
         }
-        if (h) rc = fail(SHG_ERR_CUDA, "blocked Jacobi sweep: a staged plane did not arrive");
+        if (h) rc = fail(SHG_ERR_CUDA, "Jacobi sweeps: a bounded wait (staged plane or grid barrier) ran out");
     } while (0);
     cudaFreeAsync(buf, s);
     e = cudaGetLastError();

@@ -191,39 +191,25 @@ __global__ void __launch_bounds__(MpCfg<T, N>::row_threads(THERM))
             if (d.slices_p) reinterpret_cast<V*>(d.slices_p)[(size_t)y * N + x] = p0;
             if (d.slices_s) reinterpret_cast<V*>(d.slices_s)[(size_t)y * N + x] = s0;
         }
-    } else {
-        for (int e = tid; e < RB * N; e += NT) {
-            const int lr = e / N, x = e % N;
-            const size_t g = (size_t)(y0 + lr) * N + x;
-            Ps[sidx<N, R2, SW>(lr, x)] = gP[g];
-            Ss[sidx<N, R2, SW>(lr, x)] = gS[g];
+    }
+
+    // 16-point stage over n1 of every (row, k2) of both fields: inverse, straight from global
+    // memory (position n1 + 16 k2 is stored at n1 * R2 + k2, so the lanes' loads are contiguous)
+    if (mode != 0) {
+        for (int j = tid; j < 2 * RB * R2; j += NT) {
+            const int k2 = j % R2, lr = (j / R2) % RB;
+            const bool f = j >= RB * R2;
+            V* F = f ? Ss : Ps;
+            const V* row = (f ? gS : gP) + (size_t)(y0 + lr) * N + k2;
+            V u[16];
+#pragma unroll
+            for (int n = 0; n < 16; ++n) u[n] = cj(__ldcg(row + n * R2));
+            Dft<16, -1, T>::run(u);
+#pragma unroll
+            for (int n = 0; n < 16; ++n) F[sidx<N, R2, SW>(lr, n + 16 * k2)] = cj(u[n]);
         }
     }
     __syncthreads();
-
-    // 16-point stage over n1 of every (row, k2), both fields
-    auto n1_pass = [&](bool inv) {
-        for (int j = tid; j < RB * R2; j += NT) {
-            const int k2 = j % R2, lr = j / R2;
-#pragma unroll 1
-            for (int f = 0; f < 2; ++f) {
-                V* F = f ? Ss : Ps;
-                V u[16];
-#pragma unroll
-                for (int n = 0; n < 16; ++n) {
-                    u[n] = F[sidx<N, R2, SW>(lr, n + 16 * k2)];
-                    if (inv) u[n] = cj(u[n]);
-                }
-                Dft<16, -1, T>::run(u);
-#pragma unroll
-                for (int n = 0; n < 16; ++n) F[sidx<N, R2, SW>(lr, n + 16 * k2)] = inv ? cj(u[n]) : u[n];
-            }
-        }
-    };
-    if (mode != 0) {
-        n1_pass(true);
-        __syncthreads();
-    }
 
     const T hap = (T)d.hap, has = (T)d.has, qs = (T)d.qs, dz6 = (T)(d.dz / 6.0);
     {
@@ -308,14 +294,18 @@ __global__ void __launch_bounds__(MpCfg<T, N>::row_threads(THERM))
             if ((tid & 31) == 0) part[(r < RB ? 0 : N) + y0 + r % RB] = a;
         }
     }
-    if (mode != 2) {
-        n1_pass(false);
-        __syncthreads();
-        for (int e = tid; e < RB * N; e += NT) {
-            const int lr = e / N, x = e % N;
-            const size_t g = (size_t)(y0 + lr) * N + x;
-            gP[g] = Ps[sidx<N, R2, SW>(lr, x)];
-            gS[g] = Ss[sidx<N, R2, SW>(lr, x)];
+    if (mode != 2) {  // and forward, straight to global memory
+        for (int j = tid; j < 2 * RB * R2; j += NT) {
+            const int k2 = j % R2, lr = (j / R2) % RB;
+            const bool f = j >= RB * R2;
+            const V* F = f ? Ss : Ps;
+            V* row = (f ? gS : gP) + (size_t)(y0 + lr) * N + k2;
+            V u[16];
+#pragma unroll
+            for (int n = 0; n < 16; ++n) u[n] = F[sidx<N, R2, SW>(lr, n + 16 * k2)];
+            Dft<16, -1, T>::run(u);
+#pragma unroll
+            for (int n = 0; n < 16; ++n) __stcg(row + n * R2, u[n]);
         }
     }
 }
@@ -347,22 +337,23 @@ __global__ void __launch_bounds__(MpCfg<T, N>::CNT)
         tw[j] = gtab[j];
         py[j] = gtab[(f ? 4 : 3) * N + j];
     }
-    if (tid < CW) px[tid] = gtab[(f ? 2 : 1) * N + x0 + tid];
-    for (int e = tid; e < N * CW; e += NT) {
-        const int y = e / CW, c = e % CW;
-        tile[e] = F[(size_t)y * N + x0 + c];
+    if (tid < CW) {
+        const int q = x0 + tid;  // stored column q holds position q / R2 + 16 (q mod R2)
+        px[tid] = gtab[(f ? 2 : 1) * N + q / R2 + 16 * (q % R2)];
     }
-    __syncthreads();
-    auto col_stage = [&](bool inv) {  // R2-point stage over n2 of every (column, n1)
-        const int c = tid % CW, n1 = tid / CW;
+    // R2-point stage over n2 of every (column, n1): from global memory to the tile (the loads are
+    // under way while the tables settle), and at the end back
+    const int sc = tid % CW, sn1 = tid / CW;
+    V* col = F + (size_t)sn1 * N + x0 + sc;
+    {
         V v[R2];
 #pragma unroll
-        for (int k = 0; k < R2; ++k) v[k] = tile[(n1 + 16 * k) * CW + c];
-        r2_stage<T, R2>(v, tw, n1, inv);
+        for (int k = 0; k < R2; ++k) v[k] = __ldcg(col + (size_t)16 * k * N);
+        __syncthreads();
+        r2_stage<T, R2>(v, tw, sn1, false);
 #pragma unroll
-        for (int k = 0; k < R2; ++k) tile[(n1 + 16 * k) * CW + c] = v[k];
-    };
-    col_stage(false);
+        for (int k = 0; k < R2; ++k) tile[(sn1 + 16 * k) * CW + sc] = v[k];
+    }
     __syncthreads();
     // 16-point DFT over n1 of every (column, k2), propagator by frequency, inverse DFT
     for (int j = tid; j < R2 * CW; j += NT) {
@@ -389,12 +380,12 @@ __global__ void __launch_bounds__(MpCfg<T, N>::CNT)
         for (int n = 0; n < 16; ++n) tile[(n + 16 * k2) * CW + c] = u[n];
     }
     __syncthreads();
-    col_stage(true);
-    __syncthreads();
-    for (int e = tid; e < N * CW; e += NT) {
-        const int y = e / CW, c = e % CW;
-        F[(size_t)y * N + x0 + c] = tile[e];
-    }
+    V v[R2];
+#pragma unroll
+    for (int k = 0; k < R2; ++k) v[k] = tile[(sn1 + 16 * k) * CW + sc];
+    r2_stage<T, R2>(v, tw, sn1, true);
+#pragma unroll
+    for (int k = 0; k < R2; ++k) __stcg(col + (size_t)16 * k * N, v[k]);
 }
 
 // SH and pump power of each plain instance from its row sums (one warp).

@@ -21,7 +21,7 @@ namespace {
 // captured into a CUDA graph.  Instances with fewer steps drop out of later launches.
 template <typename T, int N, bool THERM>
 cudaError_t mp_march(const InstDesc* dev_descs, const InstDesc* host_descs, int count, cudaStream_t s) {
-    using Cfg = MpCfg<T, N>;
+    using Cfg = MpCfg<T, N, THERM>;
     static PerDevice<int> state;  // kernel attributes, once per device
     const cudaError_t attr_err = state.get([](int, int&) {
         cudaError_t e = cudaFuncSetAttribute(mp_row_kernel<T, N, THERM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -39,10 +39,10 @@ cudaError_t mp_march(const InstDesc* dev_descs, const InstDesc* host_descs, int 
     if (e != cudaSuccess) return e;
     const dim3 rgrid(Cfg::RPART, count), cgrid(N / Cfg::CW, 2, count);
     mp_setup_kernel<T, N><<<count, 256, 0, s>>>(dev_descs, L);
-    mp_row_kernel<T, N, THERM><<<rgrid, Cfg::row_threads(THERM), Cfg::row_smem, s>>>(dev_descs, L, -1);
+    mp_row_kernel<T, N, THERM><<<rgrid, Cfg::RNT, Cfg::row_smem, s>>>(dev_descs, L, -1);
     for (int st = 0; st < max_steps; ++st) {
         mp_col_kernel<T, N><<<cgrid, Cfg::CNT, Cfg::col_smem, s>>>(dev_descs, L, st);
-        mp_row_kernel<T, N, THERM><<<rgrid, Cfg::row_threads(THERM), Cfg::row_smem, s>>>(dev_descs, L, st);
+        mp_row_kernel<T, N, THERM><<<rgrid, Cfg::RNT, Cfg::row_smem, s>>>(dev_descs, L, st);
     }
     if (!THERM) mp_power_kernel<T, N><<<count, 32, 0, s>>>(dev_descs, L);
     e = cudaGetLastError();
@@ -51,7 +51,7 @@ cudaError_t mp_march(const InstDesc* dev_descs, const InstDesc* host_descs, int 
 }
 
 #define SHG_MP_VARIANT(T, PREC, N, THERM) \
-    {PREC, N, 0, MpCfg<T, N>::row_threads(THERM), 1, THERM ? 1 : 0, MpCfg<T, N>::row_smem, nullptr, &mp_march<T, N, THERM>}
+    {PREC, N, 0, MpCfg<T, N, THERM>::RNT, 1, THERM ? 1 : 0, MpCfg<T, N, THERM>::row_smem, nullptr, &mp_march<T, N, THERM>}
 
 const PlainVariant kTable[] = {
     SHG_MP_VARIANT(float, 32, 512, false),  SHG_MP_VARIANT(double, 64, 512, false),

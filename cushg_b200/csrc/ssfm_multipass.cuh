@@ -23,12 +23,20 @@
 
 namespace shg {
 
-template <typename T, int N>
+template <typename T, int N, bool THERM = false>
 struct MpCfg {
     static constexpr int R2 = N / 16;
     static constexpr int SW = sizeof(T) == 4 ? 16 : 8;  // complex slots per 128 B
-    static constexpr int RB = sizeof(T) == 4 ? 8 : 4;   // rows per row-pass CTA
-    static constexpr int RNT = RB * 16;                  // row-pass threads: one (row, n1) job each
+    // Rows per row-pass CTA and threads per (row, n1) job in its pointwise work.  The thermal pass
+    // is bound by the dependent chains of its per-voxel coefficients and RK4, so it takes small
+    // CTAs of four threads a job, four to an SM (FP32: 128 registers): four 512 x 512 instances,
+    // 8 rows x 4 threads 42 us, 2 x 4 36 us in FP32; 4 x 2 81 us, 2 x 4 63 us in FP64.  A plain
+    // pass is bound by the FMA pipe and runs a job on one thread (8 rows: 44 us for eight
+    // instances, 4 rows or two threads a job 44-45 us).
+    static constexpr int RB = THERM ? 2 : sizeof(T) == 4 ? 8 : 4;
+    static constexpr int PX = THERM ? 4 : 1;
+    static constexpr int JOBS = RB * 16, RNT = JOBS * PX;  // row-pass jobs and threads
+    static constexpr int MINB = THERM ? 4 : 1;
     static constexpr int CW = SW;                        // columns per column-pass CTA: one 128 B row segment
     static constexpr int CNT = 16 * CW;                  // column-pass threads: one (column, n1) job each
     static constexpr int RPART = N / RB;                 // row-pass CTAs per instance
@@ -36,27 +44,21 @@ struct MpCfg {
     static constexpr size_t row_smem = sizeof(cx<T>) * (2 * (size_t)RB * N + 12) + sizeof(mult<T>) * N +
                                        (sizeof(T) == 4 ? 6 * sizeof(Rk4Pack) : 0);
     static constexpr size_t col_smem = sizeof(cx<T>) * (size_t)N * CW + sizeof(mult<T>) * (2 * (size_t)N + CW);
-    // The thermal row pass gives each (row, n1) job several threads in its pointwise work (the
-    // RK4 half steps with per-voxel coefficients, by far its longest part): a single instance
-    // has only N x 16 jobs, and the pass otherwise lasts one thread's chain of R2 points.  Four
-    // in FP32 (the kernel fits the 128 registers of a 512-thread block), two in FP64.
-    __host__ __device__ static constexpr int row_px(bool therm) { return therm ? (sizeof(T) == 4 ? 4 : 2) : 1; }
-    __host__ __device__ static constexpr int row_threads(bool therm) { return RNT * row_px(therm); }
     static_assert(N % 16 == 0 && RB * RPART == N && N % CW == 0, "bad multi-pass split");
 };
 
 // Per-instance workspace in global memory, at base + inst * stride: the two field planes,
 // the multiplier tables (twiddles tw, propagator factors pxp, pxs, pyp, pys: N each), the
-// row-pass power partials, the running Δk prefix (thermal) and the step positions z_s.
+// rows' power sums, the running Δk prefix and the latest slice's phase cosines and sines (thermal)
+// and the step positions z_s.
 struct MpLayout {
     char* base;
     size_t stride;
-    size_t off_s, off_tab, off_part, off_dk, off_zs;
+    size_t off_s, off_tab, off_part, off_dk, off_ph, off_zs;
 };
 
 template <typename T, int N>
 __host__ __device__ inline MpLayout mp_layout(char* base, int max_steps, bool thermal) {
-    using Cfg = MpCfg<T, N>;
     auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
     MpLayout L;
     L.base = base;
@@ -65,7 +67,8 @@ __host__ __device__ inline MpLayout mp_layout(char* base, int max_steps, bool th
     L.off_tab = L.off_s + up(plane);
     L.off_part = L.off_tab + up(sizeof(mult<T>) * 5 * (size_t)N);
     L.off_dk = L.off_part + up(sizeof(double) * 2 * N);
-    L.off_zs = L.off_dk + (thermal ? up(sizeof(double) * (size_t)N * N) : 0);
+    L.off_ph = L.off_dk + (thermal ? up(sizeof(double) * (size_t)N * N) : 0);
+    L.off_zs = L.off_ph + (thermal ? up(3 * plane) : 0);
     L.stride = L.off_zs + up(sizeof(double) * ((size_t)max_steps + 1));
     return L;
 }
@@ -125,11 +128,11 @@ __device__ __forceinline__ void l2_prefetch(const void* p, size_t bytes, int i, 
 // s + 1 = out_after writes the outputs and this CTA's power partials; s = nsteps-1 is the
 // last).  Grid (N / RB, count).
 template <typename T, int N, bool THERM>
-__global__ void __launch_bounds__(MpCfg<T, N>::row_threads(THERM))
+__global__ void __launch_bounds__(MpCfg<T, N, THERM>::RNT, MpCfg<T, N, THERM>::MINB)
     mp_row_kernel(const InstDesc* __restrict__ descs, MpLayout L, int s) {
-    using Cfg = MpCfg<T, N>;
+    using Cfg = MpCfg<T, N, THERM>;
     constexpr int R2 = Cfg::R2, RB = Cfg::RB, SW = Cfg::SW;
-    constexpr int JOBS = Cfg::RNT, PX = Cfg::row_px(THERM), NT = JOBS * PX;
+    constexpr int JOBS = Cfg::JOBS, PX = Cfg::PX, NT = Cfg::RNT;
     using V = cx<T>;
     using W = mult<T>;
     const InstDesc d = descs[blockIdx.y];
@@ -253,25 +256,84 @@ __global__ void __launch_bounds__(MpCfg<T, N>::row_threads(THERM))
                 k0 = R2 & ~1;
             }
         }
-        // thermal: each point's optics and Δk prefix are loaded before the previous point's
-        // arithmetic (thermal_pre one point ahead)
-        auto pre_of = [&](int k) {
-            const size_t g = (size_t)(y0 + lr) * N + n1 + 16 * k;
-            return thermal_pre<T, THERM>(d, mode, s, g, (size_t)N * N, THERM ? dkint + g : nullptr);
-        };
-        ThermPre<T> nxt = pre_of(k0 + part < R2 ? k0 + part : 0);
+        if constexpr (THERM) {
+            // boundary_point with the phases' cosines and sines kept from the first half of a step
+            // for its second half; each point's values are loaded one point ahead
+            const T* tnp = reinterpret_cast<const T*>(d.t_np);
+            const T* tns = reinterpret_cast<const T*>(d.t_ns);
+            const T* tdk = reinterpret_cast<const T*>(d.t_dk);
+            V* phs = reinterpret_cast<V*>(wbase + L.off_ph);
+            constexpr size_t nn = (size_t)N * N;
+            struct Pre {
+                T np0, ns0, np1, ns1, dk;  // slices s and s + 1
+                double dki;
+                V cs[3];  // of slice s
+            };
+            auto fetch = [&](int k) {
+                const size_t g = (size_t)(y0 + lr) * N + n1 + 16 * k, g0 = (size_t)s * nn + g;
+                Pre f{};
+                if (mode != 0) {
+                    f.np0 = __ldg(tnp + g0);
+                    f.ns0 = __ldg(tns + g0);
+                    f.dki = dkint[g];
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) f.cs[j] = phs[j * nn + g];
+                }
+                if (mode != 2) {
+                    f.np1 = __ldg(tnp + g0 + nn);
+                    f.ns1 = __ldg(tns + g0 + nn);
+                    f.dk = __ldg(tdk + g0 + nn);
+                }
+                return f;
+            };
+            Pre nxt = fetch(part);
 #pragma unroll 1
-        for (int k = k0 + part; k < R2; k += PX) {
-            const int x = n1 + 16 * k;
-            const int o = sidx<N, R2, SW>(lr, x);
-            const size_t g = (size_t)(y0 + lr) * N + x;
-            const ThermPre<T> cur = nxt;
-            if (k + PX < R2) nxt = pre_of(k + PX);
-            V p = Ps[o], q = Ss[o];
-            boundary_point<T, THERM>(d, mode, s, g, (size_t)N * N, p, q, coef, coef + 6, hap, has, qs, dz6,
-                                     THERM ? dkint + g : nullptr, cur);
-            Ps[o] = p;
-            Ss[o] = q;
+            for (int k = part; k < R2; k += PX) {
+                const int x = n1 + 16 * k, o = sidx<N, R2, SW>(lr, x);
+                const size_t g = (size_t)(y0 + lr) * N + x;
+                const Pre c = nxt;
+                if (k + PX < R2) nxt = fetch(k + PX);
+                V p = Ps[o], q = Ss[o], cf[6];
+                if (mode != 0) {
+                    thermal_cf<T>(d, c.np0, c.ns0, c.cs, cf);
+                    rk4_point<T>(p, q, cf, hap, has, thermal_qs<T>(d, c.ns0), dz6);
+                    if (d.t_q) reinterpret_cast<T*>(d.t_q)[(size_t)s * nn + g] = thermal_q<T>(d, c.np0, c.ns0, p, q);
+                    if (s + 1 < d.nslices) {
+                        const size_t gs = (size_t)(s + 1) * nn + g;
+                        if (d.slices_p) put_field<T>(d, d.slices_p, gs, p);
+                        if (d.slices_s) put_field<T>(d, d.slices_s, gs, q);
+                    }
+                    if (s + 1 == d.out_after) {
+                        if (d.pump_out) put_field<T>(d, d.pump_out, g, p);
+                        if (d.signal_out) put_field<T>(d, d.signal_out, g, q);
+                        d.w_out[g] = weighted_abs2<T>((double)c.ns1, q);
+                        d.w_out[nn + g] = weighted_abs2<T>((double)c.np1, p);
+                    }
+                }
+                if (mode != 2) {
+                    const double dki = add_r(c.dki, (double)c.dk);
+                    dkint[g] = dki;
+                    V cs[3];
+                    thermal_phase<T>(d, dki, s + 1, cs);
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) phs[j * nn + g] = cs[j];
+                    thermal_cf<T>(d, c.np1, c.ns1, cs, cf);
+                    rk4_point<T>(p, q, cf, hap, has, thermal_qs<T>(d, c.ns1), dz6);
+                    Ps[o] = p;
+                    Ss[o] = q;
+                }
+            }
+        } else {
+#pragma unroll 1
+            for (int k = k0 + part; k < R2; k += PX) {
+                const int x = n1 + 16 * k;
+                const int o = sidx<N, R2, SW>(lr, x);
+                const size_t g = (size_t)(y0 + lr) * N + x;
+                V p = Ps[o], q = Ss[o];
+                boundary_point<T, false>(d, mode, s, g, (size_t)N * N, p, q, coef, coef + 6, hap, has, qs, dz6, nullptr, {});
+                Ps[o] = p;
+                Ss[o] = q;
+            }
         }
         if constexpr (PX > 1) __syncthreads();
 #pragma unroll 1

@@ -83,57 +83,53 @@ __device__ __forceinline__ void rk4_jvp(cx<T>& P, cx<T>& S, cx<T>& Pd, cx<T>& Sd
     Sd = mk<T>(sd.x + asd.x * dz6, sd.y + asd.y * dz6);
 }
 
-// Thermal stage coefficients (thermal_coef) and their tangents from the voxel's tangents
-// of DKint, n_p and n_s.
+// Thermal stage coefficients (thermal_coef) and their tangents from the voxel's tangents of
+// DKint, n_p and n_s, in two parts: the three phases' cosines and sines and the phases' tangents
+// (JvpPhase, which a slice's two half steps share), and the coefficients.
 template <typename T>
-__device__ __forceinline__ void thermal_coef_jvp(const InstDesc& d, double dki, double dkid, int sl, double np,
-                                                 double ns, double npd, double nsd, cx<T>* cf, cx<T>* cfd) {
-    const double sr = (double)sl, b = sr + 1.0;
-    if constexpr (sizeof(T) == 4) {
-        // FP32 run: cf exactly as thermal_coef computes it (FP64 phase and reduction, FP32
-        // sine, cosine and κ/n), so the tangent march's forward part repeats the forward
-        // march; the tangents in FP32
-        const double q = dki / b, qd = dkid / b, two_pi = 6.283185307179586476925,
-                     inv_two_pi = 0.159154943091895335769;
-        const float kp = (float)d.kf_p / (float)np, ks = (float)d.kf_s / (float)ns;
-        const float kpd = -kp * (float)npd / (float)np, ksd = -ks * (float)nsd / (float)ns;
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            const double inc = j == 0 ? 0.0 : (j == 1 ? 0.25 : 0.5);
-            const double zj = fma_r(sr, d.dz, mul_r(d.dz, inc));
-            const double phi = q * zj;
-            const float r = (float)fma(-two_pi, rint(phi * inv_two_pi), phi);
-            const float phid = (float)(qd * zj);
-            float sn, cs;
-            sincosf(r, &sn, &cs);
-            cf[j] = mk<T>(kp * sn, kp * cs);
-            cf[3 + j] = mk<T>(-ks * sn, ks * cs);
-            cfd[j] = mk<T>(kpd * sn + kp * cs * phid, kpd * cs - kp * sn * phid);
-            cfd[3 + j] = mk<T>(-ksd * sn - ks * cs * phid, ksd * cs - ks * sn * phid);
-        }
-        return;
-    }
-    const double kp = d.kf_p / np, ks = d.kf_s / ns;
-    const double kpd = -kp * npd / np, ksd = -ks * nsd / ns;
+struct JvpPhase {
+    cx<T> cs[3];
+    T d[3];
+};
+template <typename T>
+__device__ __forceinline__ JvpPhase<T> thermal_phase_jvp(const InstDesc& d, double dki, double dkid, int sl) {
+    JvpPhase<T> f;
+    thermal_phase<T>(d, dki, sl, f.cs);
+    const double sr = (double)sl, qd = dkid / (sr + 1.0);
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
         const double inc = j == 0 ? 0.0 : (j == 1 ? 0.25 : 0.5);
-        const double w = fma_r(sr, d.dz, mul_r(d.dz, inc)) / b;
-        const double phi = dki * w, phid = dkid * w;
-        double sn, cs;
-        sincos(phi, &sn, &cs);
+        f.d[j] = (T)(qd * fma_r(sr, d.dz, mul_r(d.dz, inc)));
+    }
+    return f;
+}
+template <typename T>
+__device__ __forceinline__ void thermal_coef_jvp(const InstDesc& d, const JvpPhase<T>& f, T np, T ns, T npd, T nsd, cx<T>* cf,
+                                                 cx<T>* cfd) {
+    thermal_cf<T>(d, np, ns, f.cs, cf);
+    const T rp = -npd / np, rs = -nsd / ns;  // κ̇ / κ
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
         // cP = κp (sin φ, cos φ), cS = κs (-sin φ, cos φ)
-        cf[j] = mk<T>((T)(kp * sn), (T)(kp * cs));
-        cf[3 + j] = mk<T>((T)(-ks * sn), (T)(ks * cs));
-        cfd[j] = mk<T>((T)(kpd * sn + kp * cs * phid), (T)(kpd * cs - kp * sn * phid));
-        cfd[3 + j] = mk<T>((T)(-ksd * sn - ks * cs * phid), (T)(ksd * cs - ks * sn * phid));
+        const cx<T> a = cf[j], b = cf[3 + j];
+        cfd[j] = mk<T>(rp * a.x + a.y * f.d[j], rp * a.y - a.x * f.d[j]);
+        cfd[3 + j] = mk<T>(rs * b.x - b.y * f.d[j], rs * b.y + b.x * f.d[j]);
     }
 }
 
-// Offsets of the tangent planes and the tangent Δk prefix in a multi-pass workspace laid
-// out by mp_layout plus jvp_extra_bytes.
+// Rows per row-pass CTA, threads per (row, n1) job and CTAs per SM of the tangent row pass: small
+// CTAs of four threads a job at 128 registers (FP32), so that an SM holds 16 warps.  With 8 rows
+// (4 in FP64) and two threads a job, one CTA of 8 warps per SM, the pass waited on its dependent
+// chains: four 512 x 512 instances 144 us (FP32) and 291 us (FP64), now 96 and 172.
+template <typename T>
+struct JvpCfg {
+    static constexpr int RB = 2, PX = 4, JOBS = RB * 16, NT = JOBS * PX, MINB = sizeof(T) == 4 ? 4 : 1;
+};
+
+// Offsets of the tangent planes, the tangent Δk prefix and the phases of the latest slice (nine
+// planes of T: JvpPhase) in a multi-pass workspace laid out by mp_layout.
 struct JvpLayout {
-    size_t off_pd, off_sd, off_dkd, stride;
+    size_t off_pd, off_sd, off_dkd, off_ph, stride;
 };
 
 template <typename T, int N>
@@ -144,13 +140,10 @@ __host__ __device__ inline JvpLayout jvp_layout(const MpLayout& L) {
     J.off_pd = L.stride;
     J.off_sd = J.off_pd + up(plane);
     J.off_dkd = J.off_sd + up(plane);
-    J.stride = J.off_dkd + up(sizeof(double) * (size_t)N * N);
+    J.off_ph = J.off_dkd + up(sizeof(double) * (size_t)N * N);
+    J.stride = J.off_ph + up(9 * sizeof(T) * (size_t)N * N);
     return J;
 }
-
-// Threads per (row, n1) job in the tangent row pass's pointwise work, as in the thermal row
-// pass (two: the tangent RK4 needs more registers than a 512-thread block allows).
-constexpr int kJvpPX = 2;
 
 // Row pass of the tangent march (grid (N / RB, instances); the workspace of instance i at
 // L.base + i * L.stride, L.stride covering the tangent planes of JL): as mp_row_kernel's thermal
@@ -158,12 +151,12 @@ constexpr int kJvpPX = 2;
 // s + 1 = out_after sums this CTA's SH power and its derivative into the partials
 // (part[2 r], part[2 r + 1]).
 template <typename T, int N>
-__global__ void __launch_bounds__(MpCfg<T, N>::RNT * kJvpPX)
+__global__ void __launch_bounds__(JvpCfg<T>::NT, JvpCfg<T>::MINB)
     mp_row_jvp_kernel(const InstDesc* __restrict__ descs, MpLayout L, JvpLayout JL, const JvpDesc* __restrict__ jds,
                       int s) {
     using Cfg = MpCfg<T, N>;
-    constexpr int R2 = Cfg::R2, RB = Cfg::RB, SW = Cfg::SW;
-    constexpr int JOBS = Cfg::RNT, PX = kJvpPX, NT = JOBS * PX;
+    constexpr int R2 = Cfg::R2, SW = Cfg::SW;
+    constexpr int RB = JvpCfg<T>::RB, JOBS = JvpCfg<T>::JOBS, PX = JvpCfg<T>::PX, NT = JvpCfg<T>::NT;
     using V = cx<T>;
     using W = mult<T>;
     using R = T;
@@ -177,6 +170,7 @@ __global__ void __launch_bounds__(MpCfg<T, N>::RNT * kJvpPX)
     const W* gtab = reinterpret_cast<const W*>(wbase + L.off_tab);
     double* dkint = reinterpret_cast<double*>(wbase + L.off_dk);
     double* dkind = reinterpret_cast<double*>(wbase + JL.off_dkd);
+    T* phs = reinterpret_cast<T*>(wbase + JL.off_ph);
 
     extern __shared__ __align__(16) unsigned char smem_raw[];
     V* F4[4];
@@ -209,33 +203,37 @@ __global__ void __launch_bounds__(MpCfg<T, N>::RNT * kJvpPX)
             F4[2][o] = mk<T>((T)((pp.x - pm.x) * jd.pump_scale), (T)((pp.y - pm.y) * jd.pump_scale));
             F4[3][o] = mk<T>((T)0, (T)0);
         }
-    } else {
-        for (int e = tid; e < RB * N; e += NT) {
-            const int lr = e / N, x = e % N;
-            const size_t gi = (size_t)(y0 + lr) * N + x;
-#pragma unroll
-            for (int f = 0; f < 4; ++f) F4[f][sidx<N, R2, SW>(lr, x)] = g[f][gi];
-        }
     }
-    __syncthreads();
-    auto n1_pass = [&](bool inv) {
-        for (int j = tid; j < RB * R2; j += NT) {
-            const int k2 = j % R2, lr = j / R2;
-#pragma unroll 1
-            for (int f = 0; f < 4; ++f) {
-                V* F = F4[f];
-                V u[16];
+    // 16-point stage over n1 of every (row, k2) of the four planes: inverse from global memory,
+    // forward to it, in the forward march's storage order (mp_row_kernel)
+    auto n1_in = [&]() {
+        for (int j = tid; j < 4 * RB * R2; j += NT) {
+            const int k2 = j % R2, lr = (j / R2) % RB, f = j / (R2 * RB);
+            V* F = F4[0] + f * RB * N;
+            const V* row = g[f] + (size_t)(y0 + lr) * N + k2;
+            V u[16];
 #pragma unroll
-                for (int n = 0; n < 16; ++n) {
-                    u[n] = F[sidx<N, R2, SW>(lr, n + 16 * k2)];
-                    if (inv) u[n] = cj(u[n]);
-                }
-                Dft<16, -1, T>::run(u);
+            for (int n = 0; n < 16; ++n) u[n] = cj(__ldcg(row + n * R2));
+            Dft<16, -1, T>::run(u);
 #pragma unroll
-                for (int n = 0; n < 16; ++n) F[sidx<N, R2, SW>(lr, n + 16 * k2)] = inv ? cj(u[n]) : u[n];
-            }
+            for (int n = 0; n < 16; ++n) F[sidx<N, R2, SW>(lr, n + 16 * k2)] = cj(u[n]);
         }
     };
+    auto n1_out = [&]() {
+        for (int j = tid; j < 4 * RB * R2; j += NT) {
+            const int k2 = j % R2, lr = (j / R2) % RB, f = j / (R2 * RB);
+            const V* F = F4[0] + f * RB * N;
+            V* row = g[f] + (size_t)(y0 + lr) * N + k2;
+            V u[16];
+#pragma unroll
+            for (int n = 0; n < 16; ++n) u[n] = F[sidx<N, R2, SW>(lr, n + 16 * k2)];
+            Dft<16, -1, T>::run(u);
+#pragma unroll
+            for (int n = 0; n < 16; ++n) __stcg(row + n * R2, u[n]);
+        }
+    };
+    if (mode != 0) n1_in();
+    __syncthreads();
     // the R2 stages of planes [f0, f1) of job (lr, n1)
     auto r2_pass = [&](int n1, int lr, bool inv, int f0, int f1) {
 #pragma unroll 1
@@ -248,10 +246,6 @@ __global__ void __launch_bounds__(MpCfg<T, N>::RNT * kJvpPX)
             for (int k = 0; k < R2; ++k) F4[f][sidx<N, R2, SW>(lr, n1 + 16 * k)] = v[k];
         }
     };
-    if (mode != 0) {
-        n1_pass(true);
-        __syncthreads();
-    }
     const R* tnp = reinterpret_cast<const R*>(d.t_np);
     const R* tns = reinterpret_cast<const R*>(d.t_ns);
     const R* tdk = reinterpret_cast<const R*>(d.t_dk);
@@ -277,6 +271,7 @@ __global__ void __launch_bounds__(MpCfg<T, N>::RNT * kJvpPX)
         struct Pre {
             R np[2], ns[2], dnp[2], dns[2], dk, ddk;
             double dki, dkid;
+            JvpPhase<T> ph;  // of slice s, left there by the previous pass
         };
         auto fetch = [&](int k) {
             Pre f;
@@ -295,6 +290,13 @@ __global__ void __launch_bounds__(MpCfg<T, N>::RNT * kJvpPX)
             f.ddk = h1 == 2 ? __ldg(ddk + (size_t)(s + 1) * nn + gi) : (R)0;
             f.dki = mode == 0 ? 0.0 : dkint[gi];
             f.dkid = mode == 0 ? 0.0 : dkind[gi];
+            if (mode != 0) {
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+                    f.ph.cs[j] = mk<T>(phs[(3 * j) * nn + gi], phs[(3 * j + 1) * nn + gi]);
+                    f.ph.d[j] = phs[(3 * j + 2) * nn + gi];
+                }
+            }
             return f;
         };
         Pre nxt;
@@ -309,6 +311,7 @@ __global__ void __launch_bounds__(MpCfg<T, N>::RNT * kJvpPX)
             V p = F4[0][o], q = F4[1][o], pd = F4[2][o], qd = F4[3][o];
             const R pdk = cur.dk, pddk = cur.ddk;
             double dki = cur.dki, dkid = cur.dkid;
+            JvpPhase<T> ph = cur.ph;
 #pragma unroll 1
             for (int h = h0; h < h1; ++h) {
                 const int sl = s + h;
@@ -318,13 +321,20 @@ __global__ void __launch_bounds__(MpCfg<T, N>::RNT * kJvpPX)
                     dkid += (double)pddk;
                     dkint[gi] = dki;
                     dkind[gi] = dkid;
+                    ph = thermal_phase_jvp<T>(d, dki, dkid, sl);
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) {
+                        phs[(3 * j) * nn + gi] = ph.cs[j].x;
+                        phs[(3 * j + 1) * nn + gi] = ph.cs[j].y;
+                        phs[(3 * j + 2) * nn + gi] = ph.d[j];
+                    }
                 }
                 // this half step's values (selects, so that the rolled loop indexes no array)
                 const double np = (double)(h ? cur.np[1] : cur.np[0]), ns = (double)(h ? cur.ns[1] : cur.ns[0]);
                 const double npd = (double)(h ? cur.dnp[1] : cur.dnp[0]), nsd = (double)(h ? cur.dns[1] : cur.dns[0]);
                 V cf[6], cfd[6];
-                thermal_coef_jvp<T>(d, dki, dkid, sl, np, ns, npd, nsd, cf, cfd);
-                rk4_jvp<T>(p, q, pd, qd, cf, cfd, hap, has, (T)(0.5 * (d.bf_s * ns)), (T)(0.5 * (d.bf_s * nsd)), dz6);
+                thermal_coef_jvp<T>(d, ph, (T)np, (T)ns, (T)npd, (T)nsd, cf, cfd);
+                rk4_jvp<T>(p, q, pd, qd, cf, cfd, hap, has, thermal_qs<T>(d, (T)ns), thermal_qs<T>(d, (T)nsd), dz6);
                 if (h == 0 && jd.q_dot) {
                     // tangent of kernelSetQ for slice s after its step:
                     // Q = q_p n_p |P|^2 + q_s n_s |S|^2 + βs (q_h n_s |S|^2)^2
@@ -378,16 +388,7 @@ __global__ void __launch_bounds__(MpCfg<T, N>::RNT * kJvpPX)
             part[2 * blockIdx.x + 1] = b;
         }
     }
-    if (mode != 2) {
-        n1_pass(false);
-        __syncthreads();
-        for (int e = tid; e < RB * N; e += NT) {
-            const int lr = e / N, x = e % N;
-            const size_t gi = (size_t)(y0 + lr) * N + x;
-#pragma unroll
-            for (int f = 0; f < 4; ++f) g[f][gi] = F4[f][sidx<N, R2, SW>(lr, x)];
-        }
-    }
+    if (mode != 2) n1_out();
 }
 
 // Column pass of the tangent march: the diffraction of one field (blockIdx.y) and of its
@@ -422,28 +423,27 @@ __global__ void __launch_bounds__(MpCfg<T, N>::CNT)
         tw[j] = gtab[j];
         py[j] = gtab[(f ? 4 : 3) * N + j];
     }
-    if (tid < CW) px[tid] = gtab[(f ? 2 : 1) * N + x0 + tid];
-    for (int e = tid; e < N * CW; e += NT) {
-        const int y = e / CW, c = e % CW;
-        tile[e] = F[(size_t)y * N + x0 + c];
-        tiled[e] = Fd[(size_t)y * N + x0 + c];
-    }
+    auto stored = [&](int q) { return q / R2 + 16 * (q % R2); };  // position that stored column q holds
+    if (tid < CW) px[tid] = gtab[(f ? 2 : 1) * N + stored(x0 + tid)];
+    // R2-point stages from global memory to the tiles, and at the end back (mp_col_kernel)
+    const int sc = tid % CW, sn1 = tid / CW;
+    const size_t co = (size_t)sn1 * N + x0 + sc;
     __syncthreads();
-    auto col_stage = [&](V* tl, bool inv) {
-        const int c = tid % CW, n1 = tid / CW;
+#pragma unroll 1
+    for (int t = 0; t < 2; ++t) {
+        const V* src = (t ? Fd : F) + co;
+        V* tl = t ? tiled : tile;
         V v[R2];
 #pragma unroll
-        for (int k = 0; k < R2; ++k) v[k] = tl[(n1 + 16 * k) * CW + c];
-        r2_stage<T, R2>(v, tw, n1, inv);
+        for (int k = 0; k < R2; ++k) v[k] = __ldcg(src + (size_t)16 * k * N);
+        r2_stage<T, R2>(v, tw, sn1, false);
 #pragma unroll
-        for (int k = 0; k < R2; ++k) tl[(n1 + 16 * k) * CW + c] = v[k];
-    };
-    col_stage(tile, false);
-    col_stage(tiled, false);
+        for (int k = 0; k < R2; ++k) tl[(sn1 + 16 * k) * CW + sc] = v[k];
+    }
     __syncthreads();
     for (int j = tid; j < R2 * CW; j += NT) {
         const int c = j % CW, k2 = j / CW;
-        const int x = x0 + c;
+        const int x = stored(x0 + c);
         const int fx = (x >> 4) + R2 * (x & 15);
         const double sx = (double)(fx < N / 2 ? fx : fx - N);
         V u[16], ud[16];
@@ -478,13 +478,16 @@ __global__ void __launch_bounds__(MpCfg<T, N>::CNT)
         }
     }
     __syncthreads();
-    col_stage(tile, true);
-    col_stage(tiled, true);
-    __syncthreads();
-    for (int e = tid; e < N * CW; e += NT) {
-        const int y = e / CW, c = e % CW;
-        F[(size_t)y * N + x0 + c] = tile[e];
-        Fd[(size_t)y * N + x0 + c] = tiled[e];
+#pragma unroll 1
+    for (int t = 0; t < 2; ++t) {
+        V* dst = (t ? Fd : F) + co;
+        const V* tl = t ? tiled : tile;
+        V v[R2];
+#pragma unroll
+        for (int k = 0; k < R2; ++k) v[k] = tl[(sn1 + 16 * k) * CW + sc];
+        r2_stage<T, R2>(v, tw, sn1, true);
+#pragma unroll
+        for (int k = 0; k < R2; ++k) __stcg(dst + (size_t)16 * k * N, v[k]);
     }
 }
 
@@ -496,7 +499,7 @@ __global__ void mp_jvp_sum_kernel(const InstDesc* __restrict__ descs, MpLayout L
     const int i = blockIdx.x;
     const double* part = reinterpret_cast<const double*>(L.base + (size_t)i * L.stride + L.off_part);
     double a = 0.0, b = 0.0;
-    for (int r = 0; r < MpCfg<T, N>::RPART; ++r) {
+    for (int r = 0; r < N / JvpCfg<T>::RB; ++r) {
         a += part[2 * r];
         b += part[2 * r + 1];
     }

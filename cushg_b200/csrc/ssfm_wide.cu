@@ -87,11 +87,11 @@ const PlainVariant kTable[] = {
 //   one plain run      FP32: 64 5.0 / 13.5, 128 5.6 / 29.1, 192 6.6 / 36.8, 256 7.7 / 20.5,
 //                      512 14.4 / 34.4; FP64: 64 5.4 / 14.8, 128 5.9 / 18.2, 256 9.0 / 33.8,
 //                      512 19.0 / 41.6
-//   thermal, 2 rounds  FP32: 64 x 16 21.4 / 40.6, 128 x 8 20.8 / 22.5, 256 x 4 26.0 / 30.7;
-//                      FP64: 64 x 16 23.3 / 56.8, 128 x 8 23.8 / 28.9, 256 x 4 33.7 / 45.8
-//   thermal, 4 rounds  FP32: 128 x 16 50.3 / 37.0, 256 x 8 51.0 / 52.7 (no longer)
-//   thermal at 512     FP32: 1 21.1 / 46.2, 4 83.6 / 87.1, 8 167 / 189; FP64: 1 32.4 / 56.6,
-//                      8 259 / 289 (at any count: both grow linearly)
+//   thermal, 1 round   FP32: 128 x 4 10.6 / 15.6, 256 x 2 13.0 / 18.6, 512 21.4 / 29.8;
+//                      FP64: 128 x 4 11.7 / 17.5, 256 x 2 17.0 / 22.8, 512 33.0 / 38.0
+//   thermal, 2 rounds  FP32: 64 x 16 21.4 / 40.6, but 128 x 8 20.8 / 19.2, 256 x 4 25.6 / 24.5,
+//                      512 x 2 42.3 / 38.6; FP64: 64 x 16 23.3 / 56.8, but 128 x 8 23.1 / 22.7,
+//                      256 x 4 33.1 / 33.0, 512 x 2 65.4 / 57.8
 const PlainVariant* wide_variant_for(int precision, int n, int thermal, int count) {
     for (const PlainVariant& v : kTable) {
         if (v.precision != precision || v.n != n || v.thermal != (thermal ? 1 : 0)) continue;
@@ -101,7 +101,7 @@ const PlainVariant* wide_variant_for(int precision, int n, int thermal, int coun
             return nullptr;
         }
         const int rounds = (count + fit - 1) / fit;
-        return rounds <= (thermal ? 2 : 1) || (thermal && n == 512) ? &v : nullptr;
+        return rounds <= (thermal && n < 128 ? 2 : 1) ? &v : nullptr;
     }
     return nullptr;
 }

@@ -45,8 +45,9 @@ namespace {
 template <typename T, int N>
 cudaError_t jvp_march(const InstDesc* hdescs, const InstDesc* d_dev, const JvpDesc* jds_dev, int count, cudaStream_t s) {
     using Cfg = MpCfg<T, N>;
-    constexpr int row_nt = Cfg::RNT * kJvpPX;
-    const size_t row_smem = sizeof(cx<T>) * 4 * (size_t)Cfg::RB * N + sizeof(mult<T>) * N + sizeof(double) * 2 * (row_nt / 32);
+    using JCfg = JvpCfg<T>;
+    constexpr int row_nt = JCfg::NT;
+    const size_t row_smem = sizeof(cx<T>) * 4 * (size_t)JCfg::RB * N + sizeof(mult<T>) * N + sizeof(double) * 2 * (row_nt / 32);
     const size_t col_smem = sizeof(cx<T>) * 2 * (size_t)N * Cfg::CW + sizeof(mult<T>) * (2 * (size_t)N + Cfg::CW);
     static PerDevice<int> state;  // kernel attributes, once per device
     const cudaError_t attr_err = state.get([&](int, int&) {
@@ -66,10 +67,10 @@ cudaError_t jvp_march(const InstDesc* hdescs, const InstDesc* d_dev, const JvpDe
     cudaError_t e = dev_alloc((void**)&L.base, JL.stride * (size_t)count, s);
     if (e != cudaSuccess) return e;
     mp_setup_kernel<T, N><<<count, 256, 0, s>>>(d_dev, L);
-    mp_row_jvp_kernel<T, N><<<dim3(Cfg::RPART, count), row_nt, row_smem, s>>>(d_dev, L, JL, jds_dev, -1);
+    mp_row_jvp_kernel<T, N><<<dim3(N / JCfg::RB, count), row_nt, row_smem, s>>>(d_dev, L, JL, jds_dev, -1);
     for (int st = 0; st < max_steps; ++st) {
         mp_col_jvp_kernel<T, N><<<dim3(N / Cfg::CW, 2, count), Cfg::CNT, col_smem, s>>>(d_dev, L, JL, jds_dev, st);
-        mp_row_jvp_kernel<T, N><<<dim3(Cfg::RPART, count), row_nt, row_smem, s>>>(d_dev, L, JL, jds_dev, st);
+        mp_row_jvp_kernel<T, N><<<dim3(N / JCfg::RB, count), row_nt, row_smem, s>>>(d_dev, L, JL, jds_dev, st);
     }
     mp_jvp_sum_kernel<T, N><<<count, 32, 0, s>>>(d_dev, L, jds_dev);
     e = cudaGetLastError();

@@ -86,7 +86,7 @@ def test_batches_on_either_side_of_the_rule(precision, sides):
 @pytest.mark.parametrize("n,precision,count", [(32, 64, 1), (64, 32, 1), (128, 64, 1), (128, 32, 9), (256, 32, 1),
                                                (256, 64, 5), (512, 32, 2), (512, 64, 1)])
 def test_thermal_equals_batch_march(n, precision, count):
-    """A thermal batch's optical passes on the wide march (few instances, or side 512) and on
+    """A thermal batch's optical passes on the wide march (few instances) and on
     the march of large batches."""
     import torch
     ps = []

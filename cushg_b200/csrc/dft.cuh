@@ -104,13 +104,23 @@ template <typename T>
 __device__ __forceinline__ cx<T> rot_const(cx<T> v, double c, double s) {
     const bool diag = c == s, anti = c == -s;  // odd multiples of 45 degrees
     const bool re2 = sizeof(T) == 8 && diag, im2 = sizeof(T) == 8 ? !anti : !diag;
-    auto re = [&](T cc, T ss) { return re2 ? det2<true>(v.x, cc, v.y, ss) : det2(v.x, cc, v.y, ss); };
-    auto im = [&](T cc, T ss) { return im2 ? dot2<true>(v.x, ss, v.y, cc) : dot2(v.x, ss, v.y, cc); };
+    // a factor of zero takes no product: the real rotation of radix 3, the low part of cos 60
+    auto re = [&](T cc, T ss) {
+        if (ss == (T)0) return mul_r(v.x, cc);
+        if (cc == (T)0) return mul_r(-v.y, ss);
+        return re2 ? det2<true>(v.x, cc, v.y, ss) : det2(v.x, cc, v.y, ss);
+    };
+    auto im = [&](T cc, T ss) {
+        if (ss == (T)0) return mul_r(v.y, cc);
+        if (cc == (T)0) return mul_r(v.x, ss);
+        return im2 ? dot2<true>(v.x, ss, v.y, cc) : dot2(v.x, ss, v.y, cc);
+    };
     if constexpr (sizeof(T) == 8) {
         return mk<T>(re(c, s), im(c, s));
     } else {
         const float ch = (float)c, sh = (float)s;
         const float cl = (float)(c - (double)ch), sl = (float)(s - (double)sh);
+        if (s == 0.0) return mk<T>(fma_r(v.x, ch, re(cl, sl)), fma_r(v.y, ch, im(cl, sl)));
         return mk<T>(fma_r(v.x, ch, fma_r(-v.y, sh, re(cl, sl))), fma_r(v.x, sh, fma_r(v.y, ch, im(cl, sl))));
     }
 }

@@ -165,7 +165,7 @@ static BatchLayout batch_layout(const shg_params* params, int count, void* const
         const PlainVariant* w = wide_choice(params[i], items[i].v, 1);
         if (!w || w->fit(&fit) != cudaSuccess) break;
         wide.push_back(w);
-        share += 1.0 / fit;
+        share += 1.0 / (fit * w->rounds);
     }
     if ((int)wide.size() == count && share < 1.0 + 1e-9)
         for (int i = 0; i < count; ++i) items[i].v = wide[i];

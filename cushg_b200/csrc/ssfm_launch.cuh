@@ -13,10 +13,11 @@
 
 namespace shg {
 
-template <typename T, int N, int C, int NT, bool THERM, int MINB>
-cudaError_t launch_plain(const InstDesc* descs, int count, int* queue, cudaStream_t stream) {
+// (resident, if given: the clusters that fit on the device at once)
+template <typename T, int N, int C, int NT, bool THERM, int MINB, bool SPLIT = false>
+cudaError_t launch_plain_fit(const InstDesc* descs, int count, int* queue, cudaStream_t stream, int* fit) {
     using Cfg = PlainCfg<T, N, C, NT, THERM>;
-    auto kern = ssfm_plain_kernel<T, N, C, NT, THERM, MINB>;
+    auto kern = ssfm_plain_kernel<T, N, C, NT, THERM, MINB, SPLIT>;
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(NT, 1, 1);
     cfg.dynamicSmemBytes = Cfg::smem_bytes;
@@ -52,10 +53,20 @@ cudaError_t launch_plain(const InstDesc* descs, int count, int* queue, cudaStrea
         },
         &resident);
     if (attr_err != cudaSuccess) return attr_err;
+    if (fit) *fit = resident;
     if (count <= 0) return cudaSuccess;
     const int clusters = queue ? std::min(count, resident) : count;
     cfg.gridDim = dim3((unsigned)(clusters * C), 1, 1);
     return cudaLaunchKernelEx(&cfg, kern, descs, count, queue);
+}
+
+template <typename T, int N, int C, int NT, bool THERM, int MINB, bool SPLIT = false>
+cudaError_t launch_plain(const InstDesc* descs, int count, int* queue, cudaStream_t stream) {
+    return launch_plain_fit<T, N, C, NT, THERM, MINB, SPLIT>(descs, count, queue, stream, nullptr);
+}
+template <typename T, int N, int C, int NT, bool THERM, int MINB, bool SPLIT>
+cudaError_t plain_fit(int* instances) {
+    return launch_plain_fit<T, N, C, NT, THERM, MINB, SPLIT>(nullptr, 0, nullptr, nullptr, instances);
 }
 
 #define SHG_VARIANT(T, PREC, N, C, NT, MINB, THERM)                                                  \

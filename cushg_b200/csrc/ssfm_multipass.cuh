@@ -92,26 +92,6 @@ __global__ void __launch_bounds__(256) mp_setup_kernel(const InstDesc* __restric
     }
 }
 
-// The R2-point stage of the four-step transform on the elements n2 = 0..R2-1 of one n1:
-// forward = DFT, then twiddle W_N^{n1 k}; inverse = conj(DFT(conj(x) W)).
-template <typename T, int R2>
-__device__ __forceinline__ void r2_stage(cx<T> (&v)[R2], const mult<T>* tw, int n1, bool inv) {
-    auto cj = [](cx<T> a) { return mk<T>(a.x, -a.y); };
-    if (inv) {
-        v[0] = cj(v[0]);
-#pragma unroll
-        for (int k = 1; k < R2; ++k) v[k] = mulw_cj(v[k], tw[k * 16 + n1]);
-    }
-    Dft<R2, -1, T>::run(v);
-    if (inv) {
-#pragma unroll
-        for (int k = 0; k < R2; ++k) v[k] = cj(v[k]);
-    } else {
-#pragma unroll
-        for (int k = 1; k < R2; ++k) v[k] = mulw(v[k], tw[k * 16 + n1]);
-    }
-}
-
 // L2 prefetch of `bytes` of global memory from p, in 4 KB bulk prefetches issued by threads
 // i, i + n, ... of the block; nothing when p or bytes is not a multiple of 16 (a bulk
 // prefetch needs both).  A prefetch only warms L2: it never changes what a load returns.

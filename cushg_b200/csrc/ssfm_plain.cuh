@@ -432,6 +432,26 @@ __device__ __forceinline__ void boundary_point(const InstDesc& d, int mode, int 
     }
 }
 
+// The R2-point stage of the four-step transform on the elements n2 = 0..R2-1 of one n1:
+// forward = DFT, then twiddle W_N^{n1 k}; inverse = conj(DFT(conj(x) W)).
+template <typename T, int R2>
+__device__ __forceinline__ void r2_stage(cx<T> (&v)[R2], const mult<T>* tw, int n1, bool inv) {
+    auto cj = [](cx<T> a) { return mk<T>(a.x, -a.y); };
+    if (inv) {
+        v[0] = cj(v[0]);
+#pragma unroll
+        for (int k = 1; k < R2; ++k) v[k] = mulw_cj(v[k], tw[k * 16 + n1]);
+    }
+    Dft<R2, -1, T>::run(v);
+    if (inv) {
+#pragma unroll
+        for (int k = 0; k < R2; ++k) v[k] = cj(v[k]);
+    } else {
+#pragma unroll
+        for (int k = 1; k < R2; ++k) v[k] = mulw(v[k], tw[k * 16 + n1]);
+    }
+}
+
 // Sum of |v|^2 over one row of a plane in shared memory, by a warp: each lane's columns in
 // order, then the lanes by a shuffle tree.  The plain marches add a row's points like this and
 // then the rows like this (sum_rows), so an instance's powers do not depend on the march or on
@@ -458,7 +478,14 @@ __device__ __forceinline__ double sum_rows(Get&& row, int lane) {
 // atomic counter the host zeroes before the launch, instances in the descriptor order the
 // host chose: longest march first) until the queue is empty.  queue == nullptr: one
 // instance per cluster, instance = cluster index.
-template <typename T, int N, int C, int NT, bool THERM, int MINB = 1>
+//
+// SPLIT (16-CTA clusters): for one run on its own, whose step lasts as long as a thread's chain.
+// Each field's stages and each RK4 point pair get threads of their own, with a CTA barrier between
+// the parts, instead of one thread running a job's two fields and R2 points after each other.
+// Per step, one run alone, this / the wide march / without SPLIT: FP32 32 x 32 2.5 / 4.9 / 6.8 us,
+// 64 x 64 3.1 / 5.0 / 13.1, 96 x 96 4.9 / 5.3 / 42.8, 128 x 128 6.5 / 5.6 / 29.6 (not built); FP64
+// 32 x 32 2.7 / 5.4 / 9.1, 64 x 64 4.2 / 5.3 / 15.2, 96 x 96 7.5 / 5.7 / 35.9 (not built).
+template <typename T, int N, int C, int NT, bool THERM, int MINB = 1, bool SPLIT = false>
 __global__ void __launch_bounds__(NT, MINB)
     ssfm_plain_kernel(const InstDesc* __restrict__ descs, int count, int* __restrict__ queue) {
     using Cfg = PlainCfg<T, N, C, NT, THERM>;
@@ -722,6 +749,113 @@ __global__ void __launch_bounds__(NT, MINB)
             }
         };
 
+        // ---- the same passes with a thread per field (SPLIT) -------------------------------
+        auto split_r2 = [&](bool inv) {
+            for (int j = tid; j < 2 * JA; j += NT) {
+                const int n1 = j & 15, lr = (j >> 4) % Cfg::RL;
+                V* F = j >= JA ? Ss : Ps;
+                V v[R2];
+#pragma unroll
+                for (int k = 0; k < R2; ++k) v[k] = F[sidx<N, R2, SW>(lr, n1 + 16 * k)];
+                r2_stage<T, R2>(v, tw, n1, inv);
+#pragma unroll
+                for (int k = 0; k < R2; ++k) F[sidx<N, R2, SW>(lr, n1 + 16 * k)] = v[k];
+            }
+        };
+        auto split_points = [&](int mode, int s, const V* cf_prev, const V* cf_next) {
+            if constexpr (PACK) {
+                if (mode == 1 && s + 1 >= d.nslices) {
+                    const Rk4Pack* kprev = kpk + 3 * (s & 1);
+                    const Rk4Pack* knext = kpk + 3 * ((s + 1) & 1);
+                    const float2 nhap = bc2(-hap), nhas = bc2(-has), nqs = bc2(-qs), dzz = bc2(dz6);
+                    for (int j = tid; j < Cfg::RL * 16 * (R2 / 2); j += NT) {
+                        const int n1 = j & 15, kk = (j >> 4) % (R2 / 2), lr = (j >> 4) / (R2 / 2);
+                        const int o0 = sidx<N, R2, SW>(lr, n1 + 32 * kk), o1 = sidx<N, R2, SW>(lr, n1 + 32 * kk + 16);
+                        const V p0 = Ps[o0], q0 = Ss[o0], p1 = Ps[o1], q1 = Ss[o1];
+                        Cx2 P{make_float2(p0.x, p1.x), make_float2(p0.y, p1.y)};
+                        Cx2 S{make_float2(q0.x, q1.x), make_float2(q0.y, q1.y)};
+                        rk4_pair(P, S, kprev, nhap, nhas, nqs, dzz);
+                        rk4_pair(P, S, knext, nhap, nhas, nqs, dzz);
+                        Ps[o0] = make_float2(P.r.x, P.i.x);
+                        Ps[o1] = make_float2(P.r.y, P.i.y);
+                        Ss[o0] = make_float2(S.r.x, S.i.x);
+                        Ss[o1] = make_float2(S.r.y, S.i.y);
+                    }
+                    if constexpr (R2 & 1) {  // the odd one out
+                        for (int j = tid; j < JA; j += NT) {
+                            const int o = sidx<N, R2, SW>(j >> 4, (j & 15) + 16 * (R2 - 1));
+                            V p = Ps[o], q = Ss[o];
+                            rk4_point<T>(p, q, cf_prev, hap, has, qs, dz6);
+                            rk4_point<T>(p, q, cf_next, hap, has, qs, dz6);
+                            Ps[o] = p;
+                            Ss[o] = q;
+                        }
+                    }
+                    return;
+                }
+            }
+            for (int e = tid; e < Cfg::PLANE; e += NT) {
+                const int lr = e / N, x = e % N, o = sidx<N, R2, SW>(lr, x);
+                const size_t g = (size_t)(crank + C * lr) * N + x;
+                V p = Ps[o], q = Ss[o];
+                boundary_point<T, false>(d, mode, s, g, (size_t)N * N, p, q, cf_prev, cf_next, hap, has, qs, dz6, nullptr, {});
+                Ps[o] = p;
+                Ss[o] = q;
+            }
+        };
+        auto split_rb = [&](bool inv) {
+            for (int j = tid; j < 2 * JB; j += NT) {
+                const int k2 = j % R2, lr = (j / R2) % Cfg::RL;
+                V* F = j >= JB ? Ss : Ps;
+                V u[16];
+#pragma unroll
+                for (int n = 0; n < 16; ++n) {
+                    u[n] = F[sidx<N, R2, SW>(lr, n + 16 * k2)];
+                    if (inv) u[n] = cj(u[n]);
+                }
+                Dft<16, -1, T>::run(u);
+#pragma unroll
+                for (int n = 0; n < 16; ++n) F[sidx<N, R2, SW>(lr, n + 16 * k2)] = inv ? cj(u[n]) : u[n];
+            }
+        };
+        auto split_ca = [&](bool inv) {
+            for (int j = tid; j < 2 * JCA; j += NT) {
+                const int x = j % N, n1l = (j / N) % CPR;
+                V* F = j >= JCA ? Ss : Ps;
+                V v[R2];
+#pragma unroll
+                for (int k = 0; k < R2; ++k) v[k] = F[sidx<N, R2, SW>(n1l + CPR * k, x)];
+                r2_stage<T, R2>(v, tw, crank + C * n1l, inv);
+#pragma unroll
+                for (int k = 0; k < R2; ++k) F[sidx<N, R2, SW>(n1l + CPR * k, x)] = v[k];
+            }
+        };
+        auto split_cb = [&]() {
+            for (int j = tid; j < 2 * JCB; j += NT) {
+                const int xl = j % (N / C), k2 = (j / (N / C)) % R2;
+                const bool f = j >= JCB;
+                const int x = crank * (N / C) + xl;
+                V* const mine = f ? Ss : Ps;
+                const W px = f ? pxs[x] : pxp[x];
+                const W* py = f ? pys : pyp;
+                V* at[16];
+                V u[16];
+#pragma unroll
+                for (int n = 0; n < 16; ++n) {
+                    V* base = mine;
+                    if constexpr (C > 1) base = cg::this_cluster().map_shared_rank(mine, n % C);
+                    at[n] = base + sidx<N, R2, SW>(n / C + CPR * k2, x);
+                    u[n] = *at[n];
+                }
+                Dft<16, -1, T>::run(u);
+#pragma unroll
+                for (int k1 = 0; k1 < 16; ++k1) u[k1] = cj(mulw(mulw(u[k1], py[k2 + R2 * k1]), px));
+                Dft<16, -1, T>::run(u);
+#pragma unroll
+                for (int n = 0; n < 16; ++n) *at[n] = cj(u[n]);
+            }
+        };
+
         // Between the two row passes a CTA-wide barrier is needed only where a warp's RA jobs
         // and RB jobs touch different rows.  With R2 == 16 both passes give job j the row j / 16
         // and every thread the same jobs, so each warp owns its rows for RB, RA and RB' / RA'
@@ -731,13 +865,48 @@ __global__ void __launch_bounds__(NT, MINB)
             else __syncthreads();
         };
 
-        pass_ra(0, -1, coef, coef);
-        row_sync();
+        auto ra = [&](int mode, int s, const V* cf_prev, const V* cf_next) {
+            if constexpr (SPLIT) {
+                if (mode != 0) {
+                    split_r2(true);
+                    __syncthreads();
+                }
+                split_points(mode, s, cf_prev, cf_next);
+                if (mode != 2) {
+                    __syncthreads();
+                    split_r2(false);
+                }
+                __syncthreads();
+            } else {
+                pass_ra(mode, s, cf_prev, cf_next);
+                row_sync();
+            }
+        };
+        ra(0, -1, coef, coef);
 
         double z = 0.0;
         for (int s = 0; s < nsteps; ++s) {
             V* cf_cur = coef + 6 * (s & 1);
             V* cf_nxt = coef + 6 * ((s + 1) & 1);
+            if constexpr (SPLIT) {
+                split_rb(false);
+                __syncthreads();
+                split_ca(false);
+                cluster_sync();
+                if (tid >= NT - 3 && s + 1 < nsteps) {
+                    stage_coef<T>(d, s + 1, add_r(z, d.dz), tid - (NT - 3), cf_nxt);
+                    if constexpr (PACK) stage_pack(cf_nxt, tid - (NT - 3), kpk + 3 * ((s + 1) & 1));
+                }
+                split_cb();
+                cluster_sync();
+                split_ca(true);
+                __syncthreads();
+                split_rb(true);
+                __syncthreads();
+                ra(s + 1 < nsteps ? 1 : 2, s, cf_cur, cf_nxt);
+                z = add_r(z, d.dz);
+                continue;
+            }
             pass_rb(false);
             __syncthreads();
             pass_ca(false);
@@ -752,8 +921,7 @@ __global__ void __launch_bounds__(NT, MINB)
             __syncthreads();
             pass_rb(true);
             row_sync();
-            pass_ra(s + 1 < nsteps ? 1 : 2, s, cf_cur, cf_nxt);
-            row_sync();
+            ra(s + 1 < nsteps ? 1 : 2, s, cf_cur, cf_nxt);
             z += d.dz;
         }
 

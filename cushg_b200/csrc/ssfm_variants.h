@@ -34,7 +34,8 @@ struct PlainVariant {
     size_t smem;    // dynamic shared memory per CTA (multi-pass: of the row pass)
     PlainLaunch launch;  // fused cluster march, or null
     MpLaunch mp;         // multi-pass or wide march, or null
-    cudaError_t (*fit)(int* instances) = nullptr;  // wide march: instances resident at once
+    cudaError_t (*fit)(int* instances) = nullptr;  // marches for few runs: instances resident at once
+    int rounds = 1;  // marches for few runs: rounds of `fit` up to which they are the faster march
 };
 
 // Run `count` instances through variant v (either kind); queue as for PlainLaunch.
@@ -57,6 +58,7 @@ VariantTable variants_f64_small();
 VariantTable variants_f64_large();
 VariantTable variants_thermal();
 VariantTable variants_multipass();
+VariantTable variants_split();  // not among the batch tuner's choices
 
 // The variant the drivers use for (precision, n, thermal) under march preference `march`
 // (SHG_MARCH_*): automatic = the tuned one if shg_autotune chose one, else the default

@@ -117,7 +117,7 @@ typedef struct shg_params {
     int32_t jacobi_block;
     /* Which SSFM march to run (SHG_MARCH_*).  Automatic: a single run, or a batch few enough to
      * fit on the device side by side, takes the wide march (one instance spread over the whole
-     * GPU by a cooperative launch); larger batches of plain runs take the fused cluster march
+     * GPU by a cooperative launch; small sides a 16-CTA cluster); larger batches of plain runs take the fused cluster march
      * where one is built for the grid side (planes in shared memory, sides <= 256) and the
      * multi-pass march otherwise (planes in global memory, side 512); larger batches of thermal
      * runs the multi-pass march where one is built (sides 128, 256) and the fused one otherwise.

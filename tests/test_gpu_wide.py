@@ -1,5 +1,5 @@
-"""The wide SSFM march (one instance over the whole GPU, the automatic march of single runs and
-small batches) against the fused and multi-pass marches of the same instance, through the C ABI.
+"""The marches of single runs and small batches (one instance over the whole GPU, or for small sides
+over a 16-CTA cluster with a thread per field) against the fused and multi-pass marches of the same instance, through the C ABI.
 
 All marches write every operation a field value passes through with explicit rounding, so the
 fields and powers must be the same bits; no tolerance is involved."""

@@ -53,11 +53,13 @@ cudaError_t fork_streams(int dev, ForkStreams** out) {
     return cudaSuccess;
 }
 
-// The wide march for `count` plain runs p of variant v's class on their own; null where the
-// caller or a tuner chose the march, or the wide one is not faster.
-const PlainVariant* wide_choice(const shg_params& p, const PlainVariant* v, int count) {
+constexpr int kFewLevels = 5;  // at most so many variants for few runs per class
+
+// The level-th variant for few plain runs of variant v's class (few_runs_variant); null past the
+// last and where the caller or a tuner chose the march.
+const PlainVariant* few_choice(const shg_params& p, const PlainVariant* v, int level, int* upto) {
     if (p.march != SHG_MARCH_AUTO || has_plain_choice(v->precision, v->n, 0)) return nullptr;
-    return wide_variant_for(v->precision, v->n, 0, count);
+    return few_runs_variant(v->precision, v->n, level, upto);
 }
 
 // The descriptor of one run, as a kernel argument: no copy from the caller's stack.
@@ -73,7 +75,8 @@ shg_status plain_solve_device(const shg_params& p, const void* signal_in, void* 
     int out32 = 0;
     const PlainVariant* v = plain_variant_of(p, &out32);
     if (!v) return fail(SHG_ERR_UNSUPPORTED, "no kernel for grid side %d", p.nx);
-    if (const PlainVariant* w = wide_choice(p, v, 1)) v = w;
+    int upto = 0;
+    if (const PlainVariant* w = few_choice(p, v, 0, &upto)) v = w;
     InstDesc d = make_plain_desc(p, p.temp, p.temp);
     d.out32 = out32;
     d.signal_in = signal_in;
@@ -156,19 +159,23 @@ static BatchLayout batch_layout(const shg_params* params, int count, void* const
         const PlainVariant* v = plain_variant_of(params[i], &out32);
         items[i] = {v, i, (double)params[i].nx * params[i].nx * shg_steps(&params[i]), out32};
     }
-    // A batch small enough to march side by side on the wide march takes it: the classes share
-    // the device, so the parts of it that they fill must add up to at most one.
-    std::vector<const PlainVariant*> wide;
-    double share = 0.0;
-    for (int i = 0; i < count && share < 1.0 + 1e-9; ++i) {
-        int fit = 0;
-        const PlainVariant* w = wide_choice(params[i], items[i].v, 1);
-        if (!w || w->fit(&fit) != cudaSuccess) break;
-        wide.push_back(w);
-        share += 1.0 / (fit * w->rounds);
+    // A small batch takes the variants for few runs, each class from its widest on until the batch
+    // fits: the classes share the device, so the parts of it that they fill must add up to at most one.
+    for (int level = 0; level < kFewLevels; ++level) {
+        std::vector<const PlainVariant*> few;
+        double share = 0.0;
+        for (int i = 0; i < count && share < 1.0 + 1e-9; ++i) {
+            const PlainVariant* w = nullptr;
+            int upto = 0;
+            for (int l = level; l >= 0 && !w; --l) w = few_choice(params[i], items[i].v, l, &upto);  // its last, if fewer
+            if (!w) break;
+            few.push_back(w);
+            share += 1.0 / upto;
+        }
+        if ((int)few.size() < count || share >= 1.0 + 1e-9) continue;
+        for (int i = 0; i < count; ++i) items[i].v = few[i];
+        break;
     }
-    if ((int)wide.size() == count && share < 1.0 + 1e-9)
-        for (int i = 0; i < count; ++i) items[i].v = wide[i];
     std::stable_sort(items.begin(), items.end(), [](const Item& a, const Item& b) {
         if (a.v != b.v) return a.v < b.v;
         return a.cost > b.cost;

@@ -479,12 +479,15 @@ __device__ __forceinline__ double sum_rows(Get&& row, int lane) {
 // host chose: longest march first) until the queue is empty.  queue == nullptr: one
 // instance per cluster, instance = cluster index.
 //
-// SPLIT (16-CTA clusters): for one run on its own, whose step lasts as long as a thread's chain.
-// Each field's stages and each RK4 point pair get threads of their own, with a CTA barrier between
-// the parts, instead of one thread running a job's two fields and R2 points after each other.
-// Per step, one run alone, this / the wide march / without SPLIT: FP32 32 x 32 2.5 / 4.9 / 6.8 us,
-// 64 x 64 3.1 / 5.0 / 13.1, 96 x 96 4.9 / 5.3 / 42.8, 128 x 128 6.5 / 5.6 / 29.6 (not built); FP64
-// 32 x 32 2.7 / 5.4 / 9.1, 64 x 64 4.2 / 5.3 / 15.2, 96 x 96 7.5 / 5.7 / 35.9 (not built).
+// SPLIT: each field's stages and each RK4 point pair get threads of their own, with a CTA barrier
+// between the parts, instead of one thread running a job's two fields and R2 points after each
+// other.  Where a step lasts as long as a thread's chain this wins: for one run on its own over 16
+// CTAs, and on the small sides, whose planes leave room for few threads, on a full device too.
+// Per step, one run over 16 CTAs / the wide march / the default without SPLIT: FP32 32 x 32 2.5 /
+// 4.9 / 6.8 us, 64 x 64 3.1 / 5.0 / 13.1, 96 x 96 4.9 / 5.3 / 42.8, 128 x 128 6.5 / 5.6 / 29.6; FP64
+// 32 x 32 2.7 / 5.4 / 9.1, 64 x 64 4.2 / 5.3 / 15.2, 96 x 96 7.5 / 5.7 / 35.9, 128 x 128 9.4 / 5.9 /
+// 18.2.  148 runs: FP32 96 x 96 32.5 / - / 45.0, FP64 32 x 32 9.0 / - / 12.1.  From 192 the jobs of
+// the two fields fill the threads anyway and the extra barriers cost: 192 x 192 FP32 41.2 / - / 38.2.
 template <typename T, int N, int C, int NT, bool THERM, int MINB = 1, bool SPLIT = false>
 __global__ void __launch_bounds__(NT, MINB)
     ssfm_plain_kernel(const InstDesc* __restrict__ descs, int count, int* __restrict__ queue) {

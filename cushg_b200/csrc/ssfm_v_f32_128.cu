@@ -4,9 +4,9 @@
 namespace shg {
 
 static const PlainVariant kTable[] = {
-    SHG_VARIANT(float, 32, 128, 2, 512, 1, false),  // default
+    SHG_SPLIT_VARIANT(float, 32, 128, 2, 512, 1),  // default
     SHG_VARIANT(float, 32, 128, 2, 256, 1, false),
-    SHG_VARIANT(float, 32, 128, 4, 256, 2, false),
+    SHG_SPLIT_VARIANT(float, 32, 128, 4, 256, 2),
 };
 
 VariantTable variants_f32_128() { return {kTable, (int)(sizeof(kTable) / sizeof(kTable[0]))}; }

@@ -34,8 +34,7 @@ struct PlainVariant {
     size_t smem;    // dynamic shared memory per CTA (multi-pass: of the row pass)
     PlainLaunch launch;  // fused cluster march, or null
     MpLaunch mp;         // multi-pass or wide march, or null
-    cudaError_t (*fit)(int* instances) = nullptr;  // marches for few runs: instances resident at once
-    int rounds = 1;  // marches for few runs: rounds of `fit` up to which they are the faster march
+    cudaError_t (*fit)(int* instances) = nullptr;  // instances resident on the device at once
 };
 
 // Run `count` instances through variant v (either kind); queue as for PlainLaunch.
@@ -58,16 +57,21 @@ VariantTable variants_f64_small();
 VariantTable variants_f64_large();
 VariantTable variants_thermal();
 VariantTable variants_multipass();
-VariantTable variants_split();  // not among the batch tuner's choices
+VariantTable variants_split();  // this and the next two: not among the batch tuner's choices
+VariantTable variants_split64();
+VariantTable variants_wide();
 
 // The variant the drivers use for (precision, n, thermal) under march preference `march`
 // (SHG_MARCH_*): automatic = the tuned one if shg_autotune chose one, else the default
 // (the first compiled fused variant, else the multi-pass one); fused / multi-pass = the
 // default of that kind.  Null if none is built.
 const PlainVariant* find_plain_variant(int precision, int n, int thermal = 0, int march = 0);
-// The wide march (ssfm_wide.cuh) of (precision, n, thermal) if it is the faster one for `count`
-// runs of one class that have the device to themselves, else null.
-const PlainVariant* wide_variant_for(int precision, int n, int thermal, int count);
+// The wide march (ssfm_wide.cuh) of thermal passes of (precision, n) if it is the faster one for
+// `count` runs that have the device to themselves, else null.
+const PlainVariant* wide_thermal_variant(int precision, int n, int count);
+// Plain runs of (precision, n): the level-th variant for few runs, from the widest on, and the
+// number of runs up to which it is the fastest of them; null past the last.
+const PlainVariant* few_runs_variant(int precision, int n, int level, int* upto);
 // Whether a tuner or shg_set_schedule chose a variant for (precision, n, thermal).
 bool has_plain_choice(int precision, int n, int thermal);
 // Every compiled plain variant of (precision, n), default first; returns how many.

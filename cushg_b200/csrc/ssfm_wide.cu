@@ -61,54 +61,48 @@ cudaError_t wide_march(const InstDesc* dev_descs, const InstDesc*, int count, cu
     return e != cudaSuccess ? e : ef;
 }
 
-#define SHG_WIDE_VARIANT(T, PREC, N, THERM, ROUNDS)                                                                  \
+#define SHG_WIDE_VARIANT(T, PREC, N, THERM)                                                                          \
     {PREC, N, 0, WideCfg<T, N, THERM>::NT, 1, THERM ? 1 : 0, WideCfg<T, N, THERM>::smem_bytes, nullptr, &wide_march<T, N, THERM>, \
-     &wide_fit<T, N, THERM>, ROUNDS}
+     &wide_fit<T, N, THERM>}
 
 const PlainVariant kTable[] = {
-    SHG_WIDE_VARIANT(float, 32, 128, false, 2),  SHG_WIDE_VARIANT(float, 32, 192, false, 4),
-    SHG_WIDE_VARIANT(float, 32, 256, false, 2),  SHG_WIDE_VARIANT(float, 32, 512, false, 1),
-    SHG_WIDE_VARIANT(double, 64, 96, false, 4),  SHG_WIDE_VARIANT(double, 64, 128, false, 2),
-    SHG_WIDE_VARIANT(double, 64, 192, false, 2), SHG_WIDE_VARIANT(double, 64, 256, false, 2),
-    SHG_WIDE_VARIANT(double, 64, 512, false, 1),
-    SHG_WIDE_VARIANT(float, 32, 32, true, 2),    SHG_WIDE_VARIANT(float, 32, 64, true, 2),
-    SHG_WIDE_VARIANT(float, 32, 128, true, 1),   SHG_WIDE_VARIANT(float, 32, 256, true, 1),
-    SHG_WIDE_VARIANT(float, 32, 512, true, 1),
-    SHG_WIDE_VARIANT(double, 64, 32, true, 2),   SHG_WIDE_VARIANT(double, 64, 64, true, 2),
-    SHG_WIDE_VARIANT(double, 64, 128, true, 1),  SHG_WIDE_VARIANT(double, 64, 256, true, 1),
-    SHG_WIDE_VARIANT(double, 64, 512, true, 1),
+    SHG_WIDE_VARIANT(float, 32, 128, false),  SHG_WIDE_VARIANT(float, 32, 192, false),
+    SHG_WIDE_VARIANT(float, 32, 256, false),  SHG_WIDE_VARIANT(float, 32, 512, false),
+    SHG_WIDE_VARIANT(double, 64, 96, false),  SHG_WIDE_VARIANT(double, 64, 128, false),
+    SHG_WIDE_VARIANT(double, 64, 192, false), SHG_WIDE_VARIANT(double, 64, 256, false),
+    SHG_WIDE_VARIANT(double, 64, 512, false),
+    SHG_WIDE_VARIANT(float, 32, 32, true),    SHG_WIDE_VARIANT(float, 32, 64, true),
+    SHG_WIDE_VARIANT(float, 32, 128, true),   SHG_WIDE_VARIANT(float, 32, 256, true),
+    SHG_WIDE_VARIANT(float, 32, 512, true),
+    SHG_WIDE_VARIANT(double, 64, 32, true),   SHG_WIDE_VARIANT(double, 64, 64, true),
+    SHG_WIDE_VARIANT(double, 64, 128, true),  SHG_WIDE_VARIANT(double, 64, 256, true),
+    SHG_WIDE_VARIANT(double, 64, 512, true),
 };
 
 }  // namespace
 
-// When the wide march pays.  It takes the whole device for `fit` instances at a time, so its
-// time grows with the rounds of `fit`; the fused march's grows only when its clusters no longer
-// fit side by side, the multi-pass march's slowly with the count.  Measured per step (us), wide
-// against the march a batch takes (fused, or multi-pass for thermal sides 128-512 and 512):
-//   one plain run      FP32: 128 5.6 / 29.1, 192 6.6 / 36.8, 256 7.7 / 20.5, 512 14.4 / 29.2;
-//                      FP64: 96 5.7 / 36.2, 128 5.9 / 18.2, 256 9.0 / 33.8, 512 19.0 / 39.3
-//   thermal, 1 round   FP32: 128 x 4 10.6 / 15.6, 256 x 2 13.0 / 18.6, 512 21.4 / 29.8;
-//                      FP64: 128 x 4 11.7 / 17.5, 256 x 2 17.0 / 22.8, 512 33.0 / 38.0
-//   thermal, 2 rounds  FP32: 64 x 16 21.4 / 40.6, but 128 x 8 20.8 / 19.2, 256 x 4 25.6 / 24.5,
-//                      512 x 2 42.3 / 38.6; FP64: 64 x 16 23.3 / 56.8, but 128 x 8 23.1 / 22.7,
-//                      256 x 4 33.1 / 33.0, 512 x 2 65.4 / 57.8
-//   plain up to 64 (and 96 in FP32): a 16-CTA cluster with a thread per field (SPLIT,
-//                      ssfm_plain.cuh) beats both, figures there
-const PlainVariant* wide_variant_for(int precision, int n, int thermal, int count) {
-    const PlainVariant* best = nullptr;
-    auto look = [&](const PlainVariant* v, int k) {
-        for (int i = 0; i < k && !best; ++i)
-            if (v[i].precision == precision && v[i].n == n && v[i].thermal == (thermal ? 1 : 0)) best = v + i;
-    };
-    const VariantTable split = variants_split();
-    look(split.v, split.count);
-    look(kTable, (int)(sizeof(kTable) / sizeof(kTable[0])));
-    int fit = 0;
-    if (!best || best->fit(&fit) != cudaSuccess) {
-        cudaGetLastError();  // the device cannot hold the launch: the other marches can
-        return nullptr;
+VariantTable variants_wide() { return {kTable, (int)(sizeof(kTable) / sizeof(kTable[0]))}; }
+
+// When the wide march pays for thermal passes.  It takes the whole device for `fit` instances at a
+// time, so its time grows with the rounds of `fit`; the fused march's grows only when its clusters no
+// longer fit side by side, the multi-pass march's slowly with the count.  Measured per step (us), wide
+// against the march a batch takes (fused, or multi-pass from 128 x 128):
+//   1 round   FP32: 128 x 4 10.6 / 15.6, 256 x 2 13.0 / 18.6, 512 21.4 / 29.8;
+//             FP64: 128 x 4 11.7 / 17.5, 256 x 2 17.0 / 22.8, 512 33.0 / 38.0
+//   2 rounds  FP32: 64 x 16 21.4 / 40.6, but 128 x 8 20.8 / 19.2, 256 x 4 25.6 / 24.5,
+//             512 x 2 42.3 / 38.6; FP64: 64 x 16 23.3 / 56.8, but 128 x 8 23.1 / 22.7,
+//             256 x 4 33.1 / 33.0, 512 x 2 65.4 / 57.8
+const PlainVariant* wide_thermal_variant(int precision, int n, int count) {
+    for (const PlainVariant& v : kTable) {
+        if (v.precision != precision || v.n != n || !v.thermal) continue;
+        int fit = 0;
+        if (v.fit(&fit) != cudaSuccess) {
+            cudaGetLastError();  // the device cannot hold the launch: the other marches can
+            return nullptr;
+        }
+        return count <= fit * (n < 128 ? 2 : 1) ? &v : nullptr;
     }
-    return count <= fit * best->rounds ? best : nullptr;
+    return nullptr;
 }
 
 }  // namespace shg

@@ -432,7 +432,7 @@ shg_status thermal_batch_run(const shg_params* ps, int count, const void* const*
             }
             // the wide march while the instances still iterating are few enough for it (the
             // marches agree bit for bit, so an instance's results do not depend on the choice)
-            const PlainVariant* w = p0.march == SHG_MARCH_AUTO ? wide_variant_for(p0.precision, p0.nx, 1, na) : nullptr;
+            const PlainVariant* w = p0.march == SHG_MARCH_AUTO ? wide_thermal_variant(p0.precision, p0.nx, na) : nullptr;
             if ((e = run_variant(w ? w : v, dd, hd.data(), na, nullptr, s)) != cudaSuccess) { rc = cuda_fail(e, "thermal optical pass"); break; }
             cudaEventRecord(ej[2], s);
             if ((e = cudaEventSynchronize(ej[2])) != cudaSuccess) { rc = cuda_fail(e, "thermal optical pass"); break; }

@@ -83,6 +83,23 @@ def test_batches_on_either_side_of_the_rule(precision, sides):
         plan.close()
 
 
+@pytest.mark.parametrize("precision", [64, 32])
+@pytest.mark.parametrize("n", [32, 48, 64, 96, 128, 192])
+def test_every_split_for_few_runs(n, precision):
+    """Batches of every size range that has a variant of its own, against the default variant."""
+    import torch
+    dt = torch.complex128 if precision == 64 else torch.complex64
+    for count in [1, 3, 8, 15, 29, 49, 73, 105] if n < 192 else [1, 10, 20, 40]:
+        ps = [case(n, precision, 3 + i % 2, seed=i) for i in range(count)]
+        res = []
+        for qs in (ps, [other(p) for p in ps]):
+            o = [[torch.empty((n, n), dtype=dt, device="cuda") for _ in qs] for _ in range(2)]
+            res.append((shg.solve_batch_device(qs, *o), o))
+        (pa, a), (pb, b) = res
+        assert np.array_equal(pa, pb), count
+        assert all(torch.equal(u, v) for f in range(2) for u, v in zip(a[f], b[f])), count
+
+
 @pytest.mark.parametrize("n,precision,count", [(32, 64, 1), (64, 32, 1), (128, 64, 1), (128, 32, 9), (256, 32, 1),
                                                (256, 64, 5), (512, 32, 2), (512, 64, 1)])
 def test_thermal_equals_batch_march(n, precision, count):

@@ -20,7 +20,7 @@ namespace shg {
 namespace {
 
 struct AdjVariant {
-    int precision, n, cluster, threads;
+    int precision, n, upto, cluster, threads;  // upto: the batch size up to which it is used
     size_t smem;
     // the full kernel (every phase), and the march-only one (forward and re-march phases)
     cudaError_t (*launch)(const InstDesc*, const AdjDesc*, int count, int phase, int round, cudaStream_t);
@@ -53,19 +53,31 @@ cudaError_t launch_adjoint(const InstDesc* d, const AdjDesc* a, int count, int p
     return cudaLaunchKernelEx(&cfg, kern, d, a, phase, round);
 }
 
-#define SHG_ADJ(T, PREC, N, C, NT)                                                                         \
-    {PREC, N, C, NT, PlainCfg<T, N, C, NT, false>::smem_bytes, &launch_adjoint<T, N, C, NT, false>, \
+#define SHG_ADJ(T, PREC, N, UPTO, C, NT)                                                                         \
+    {PREC, N, UPTO, C, NT, PlainCfg<T, N, C, NT, false>::smem_bytes, &launch_adjoint<T, N, C, NT, false>, \
      &launch_adjoint<T, N, C, NT, true>}
 
+// A march's step lasts as long as one thread's chain, so a small batch takes a wider split than
+// one that fills the device; the fields and each job's terms are the same bits, the jobs' FP64 sums
+// are added in another order.  us per step (100 steps, checkpoints included) at the first and last
+// count of a row / of the split for large batches there: FP32 32 1-32 17-30 / 22-33, 64 1-7 20-22 /
+// 48-51, 8-32 25-40 / 51-60, 128 1-14 27-51 / 97-107, 15-32 63-85 / 108-114; FP64 32 1-36 19-39 /
+// 29-42, 64 1-7 26-30 / 69-73, 8-36 34-80 / 74-84, 128 1-14 39-74 / 81-91.
+constexpr int kAny = 1 << 30;
 const AdjVariant kAdjVariants[] = {
-    SHG_ADJ(float, 32, 32, 1, 128),  SHG_ADJ(float, 32, 64, 1, 256),   SHG_ADJ(float, 32, 128, 2, 256),
-    SHG_ADJ(float, 32, 256, 16, 256), SHG_ADJ(double, 64, 32, 1, 128),  SHG_ADJ(double, 64, 64, 1, 256),
-    SHG_ADJ(double, 64, 128, 4, 256), SHG_ADJ(double, 64, 256, 16, 256),
+    SHG_ADJ(float, 32, 32, 32, 4, 128),    SHG_ADJ(float, 32, 32, kAny, 1, 128),
+    SHG_ADJ(float, 32, 64, 7, 16, 64),     SHG_ADJ(float, 32, 64, 32, 4, 256),   SHG_ADJ(float, 32, 64, kAny, 1, 256),
+    SHG_ADJ(float, 32, 128, 14, 16, 128),  SHG_ADJ(float, 32, 128, 32, 4, 256),  SHG_ADJ(float, 32, 128, kAny, 2, 256),
+    SHG_ADJ(float, 32, 256, kAny, 16, 256),
+    SHG_ADJ(double, 64, 32, 36, 4, 128),   SHG_ADJ(double, 64, 32, kAny, 1, 128),
+    SHG_ADJ(double, 64, 64, 7, 16, 64),    SHG_ADJ(double, 64, 64, 36, 4, 256),  SHG_ADJ(double, 64, 64, kAny, 1, 256),
+    SHG_ADJ(double, 64, 128, 14, 16, 128), SHG_ADJ(double, 64, 128, kAny, 4, 256),
+    SHG_ADJ(double, 64, 256, kAny, 16, 256),
 };
 
-const AdjVariant* find_adj(int precision, int n) {
+const AdjVariant* find_adj(int precision, int n, int count) {
     for (const auto& v : kAdjVariants)
-        if (v.precision == precision && v.n == n) return &v;
+        if (v.precision == precision && v.n == n && count <= v.upto) return &v;
     return nullptr;
 }
 
@@ -112,14 +124,14 @@ shg_status grad_batch(const shg_params* ps, int count, const double* const* poli
     }
     if (!out) return fail(SHG_ERR_INVALID, "out is NULL");
     const shg_params& p0 = ps[0];
-    const AdjVariant* v = find_adj(p0.precision, p0.nx);
+    const AdjVariant* v = find_adj(p0.precision, p0.nx, count);
     if (!v) return fail(SHG_ERR_UNSUPPORTED, "no adjoint kernel for grid side %d at precision %d", p0.nx, p0.precision);
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) {
         cudaGetLastError();
         return fail(SHG_ERR_NO_DEVICE, "no CUDA device visible");
     }
-    const int C = v->cluster;
+    const int C = v->cluster, C0 = find_adj(p0.precision, p0.nx, kAny)->cluster;
     const size_t NN = (size_t)p0.nx * p0.nx;
     const size_t cb = complex_bytes(p0);
     auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
@@ -160,7 +172,8 @@ shg_status grad_batch(const shg_params* ps, int count, const double* const* poli
         J.a.inv2h[1] = 1.0 / (2 * hf);
         J.a.inv2h[2] = 1.0 / (2 * hT);
     }
-    // checkpoint_every <= 0: a batch whose clusters cover every SM keeps every step's fields
+    // checkpoint_every <= 0: a batch whose clusters (of the large batches' split, whatever this
+    // one's: its memory stays) cover every SM keeps every step's fields
     // (one segment, no re-march) when they fit in half the free device memory, since such a
     // batch leaves no idle SMs for the re-march to overlap on; a smaller batch, or one too
     // large for that, keeps about sqrt(steps) checkpoints and re-marches on a second stream
@@ -171,7 +184,7 @@ shg_status grad_batch(const shg_params* ps, int count, const double* const* poli
         nsm = 0;
     }
     bool keep_all = false;
-    if (checkpoint_every <= 0 && nsm > 0 && (size_t)count * C >= (size_t)nsm) {
+    if (checkpoint_every <= 0 && nsm > 0 && (size_t)count * C0 >= (size_t)nsm) {
         size_t need = 0, fr = 0;
         for (GradJob& J : jobs) {
             layout(J, J.nsteps);

@@ -102,11 +102,12 @@ template <typename T>
 __device__ __forceinline__ void rk4_vjp(cx<T> p, cx<T> s, const cx<T>* cf, T hap, T has, T qs, T dz6, cx<T>& gp,
                                         cx<T>& gs, T* sens) {
     using V = cx<T>;
+    auto half = [](V k, V g) { return mk<T>(fma_r((T)0.5, k.x, g.x), fma_r((T)0.5, k.y, g.y)); };  // g + k / 2
     V k1p, k1s, k2p, k2s, k3p, k3s, k4p, k4s;
     dadz<T>(p, s, cf[0], cf[3], hap, has, qs, k1p, k1s);
-    const V u2p = mk<T>(p.x + (T)0.5 * k1p.x, p.y + (T)0.5 * k1p.y), u2s = mk<T>(s.x + (T)0.5 * k1s.x, s.y + (T)0.5 * k1s.y);
+    const V u2p = half(k1p, p), u2s = half(k1s, s);
     dadz<T>(u2p, u2s, cf[1], cf[4], hap, has, qs, k2p, k2s);
-    const V u3p = mk<T>(p.x + (T)0.5 * k2p.x, p.y + (T)0.5 * k2p.y), u3s = mk<T>(s.x + (T)0.5 * k2s.x, s.y + (T)0.5 * k2s.y);
+    const V u3p = half(k2p, p), u3s = half(k2s, s);
     dadz<T>(u3p, u3s, cf[1], cf[4], hap, has, qs, k3p, k3s);
     const V u4p = add<T>(p, k3p), u4s = add<T>(s, k3s);
     (void)k4p;
@@ -126,15 +127,15 @@ __device__ __forceinline__ void rk4_vjp(cx<T> p, cx<T> s, const cx<T>* cf, T hap
     dadz_vjp<T>(u3p, u3s, cf[1], cf[4], hap, has, qs, g3p, g3s, hp, hs, (T)0.25, sens);
     gp = add<T>(gp, hp);
     gs = add<T>(gs, hs);
-    g2p = add<T>(g2p, scale<T>(hp, (T)0.5));
-    g2s = add<T>(g2s, scale<T>(hs, (T)0.5));
+    g2p = half(hp, g2p);
+    g2s = half(hs, g2s);
     hp = mk<T>(0, 0);
     hs = mk<T>(0, 0);
     dadz_vjp<T>(u2p, u2s, cf[1], cf[4], hap, has, qs, g2p, g2s, hp, hs, (T)0.25, sens);
     gp = add<T>(gp, hp);
     gs = add<T>(gs, hs);
-    g1p = add<T>(g1p, scale<T>(hp, (T)0.5));
-    g1s = add<T>(g1s, scale<T>(hs, (T)0.5));
+    g1p = half(hp, g1p);
+    g1s = half(hs, g1s);
     hp = mk<T>(0, 0);
     hs = mk<T>(0, 0);
     dadz_vjp<T>(p, s, cf[0], cf[3], hap, has, qs, g1p, g1s, hp, hs, (T)0, sens);

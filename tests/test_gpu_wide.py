@@ -100,6 +100,22 @@ def test_every_split_for_few_runs(n, precision):
         assert all(torch.equal(u, v) for f in range(2) for u, v in zip(a[f], b[f])), count
 
 
+@pytest.mark.parametrize("precision", [64, 32])
+@pytest.mark.parametrize("n", [32, 64, 128])
+def test_gradient_splits(n, precision):
+    """Gradients of one instance in batches of every size range that has a split of its own.  The
+    fields and per-job terms are the same bits; up to 1e6 of them are added in FP64 in another order
+    (1e-16 each, times a cancellation of up to 1e4 near an optimum: 1e-10 with room)."""
+    p = case(n, precision, 11, seed=2).replace(rho_p=0.0, rho_s=0.0)
+    p.ly = p.lx
+    ref = shg.grad(p, checkpoint_every=4)
+    for count in (8, 15, 33, 37):
+        g = shg.grad_batch([p] + [p.replace(power=5.0 + i) for i in range(count - 1)], checkpoint_every=4)[0]
+        for key in ("sh_power", "d_waist", "d_focus", "d_temp"):
+            assert abs(g[key] - ref[key]) <= 1e-10 * abs(ref[key]), (count, key)
+        assert np.abs(g["d_poling"] - ref["d_poling"]).max() <= 1e-10 * np.abs(ref["d_poling"]).max(), count
+
+
 @pytest.mark.parametrize("n,precision,count", [(32, 64, 1), (64, 32, 1), (128, 64, 1), (128, 32, 9), (256, 32, 1),
                                                (256, 64, 5), (512, 32, 2), (512, 64, 1)])
 def test_thermal_equals_batch_march(n, precision, count):

@@ -115,13 +115,13 @@ typedef struct shg_params {
      * sweep per launch, 2..4 = that many through the TMA-staged blocked kernel.  Every setting gives the same
      * temperatures bit for bit; the checked sweep of each window always runs alone. */
     int32_t jacobi_block;
-    /* Which SSFM march to run (SHG_MARCH_*).  Automatic: a single run, or a batch few enough to
-     * fit on the device side by side, takes the wide march (one instance spread over the whole
-     * GPU by a cooperative launch; small sides a 16-CTA cluster); larger batches of plain runs take the fused cluster march
-     * where one is built for the grid side (planes in shared memory, sides <= 256) and the
+    /* Which SSFM march to run (SHG_MARCH_*).  Automatic, by the number of runs: one or a few
+     * spread over the whole GPU (the wide march, one instance in a cooperative launch; small
+     * sides in clusters of up to 16 CTAs); larger batches of plain runs take the fused cluster
+     * march where one is built for the grid side (planes in shared memory, sides <= 256) and the
      * multi-pass march otherwise (planes in global memory, side 512); larger batches of thermal
-     * runs the multi-pass march where one is built (sides 128, 256) and the fused one otherwise.
-     * All marches give the same bits. */
+     * runs the multi-pass march where one is built (sides 128, 256, 512) and the fused one
+     * otherwise.  All marches give the same bits. */
     int32_t march;
     /* How each outer iteration of a thermal run solves the heat equation (SHG_HEAT_*):
      * Jacobi sweeps as the reference runs them (default), or the sweeps' fixed point computed

@@ -118,8 +118,8 @@ typedef struct shg_params {
     /* Which SSFM march to run (SHG_MARCH_*).  Automatic, by the number of runs: one or a few
      * spread over the whole GPU (the wide march, one instance in a cooperative launch; small
      * sides in clusters of up to 16 CTAs); larger batches of plain runs take the fused cluster
-     * march where one is built for the grid side (planes in shared memory, sides <= 256) and the
-     * multi-pass march otherwise (planes in global memory, side 512); larger batches of thermal
+     * march (planes in shared memory) up to side 192 and the multi-pass march (planes in global
+     * memory, two planes of workspace per run) at 256 and 512; larger batches of thermal
      * runs the multi-pass march where one is built (sides 128, 256, 512) and the fused one
      * otherwise.  All marches give the same bits. */
     int32_t march;

@@ -44,7 +44,7 @@ struct MpCfg {
     static constexpr size_t row_smem = sizeof(cx<T>) * (2 * (size_t)RB * N + 12) + sizeof(mult<T>) * N +
                                        (sizeof(T) == 4 ? 6 * sizeof(Rk4Pack) : 0);
     static constexpr size_t col_smem = sizeof(cx<T>) * (size_t)N * CW + sizeof(mult<T>) * (2 * (size_t)N + CW);
-    static_assert(N % 16 == 0 && RB * RPART == N && N % CW == 0, "bad multi-pass split");
+    static_assert(N % 16 == 0 && RB * RPART == N && N % CW == 0 && RNT % 32 == 0, "bad multi-pass split");
 };
 
 // Per-instance workspace in global memory, at base + inst * stride: the two field planes,

@@ -50,6 +50,9 @@ struct PlainCfg {
     static constexpr int JCB = N * R2 / C;     // CB jobs: (column, k2)
     static constexpr int PLANE = RL * N;       // complex elements per field per CTA
     static_assert(N % 16 == 0 && 16 % C == 0 && RL * C == N, "bad grid / cluster split");
+    // the power sums give each row to one warp and add over its 32 lanes: a part of a warp would
+    // share a row with another (144 threads did)
+    static_assert(NT % 32 == 0, "whole warps only");
     // dynamic shared memory: P, S planes, twiddles + 4 propagator vectors (multiplier
     // tables), 2x6 coefficients, reduction scratch (adjoint)
     // (thermal: plus the running Δk prefix of this CTA's points, FP64)

@@ -50,7 +50,7 @@ const FewRow kFew[] = {
     {32, 128, 72, 2, 512},  {32, 128, 108, 4, 256}, {32, 192, 9, 0, 0},    {32, 192, 16, 8, 192},
     {32, 192, 36, 4, 384},  {32, 192, 56, 8, 192},  {32, 256, 4, 0, 0},    {32, 256, 6, 16, 256},
     {32, 512, 1, 0, 0},
-    {64, 32, 28, 16, 64},   {64, 32, 60, 4, 128},   {64, 48, 14, 16, 144}, {64, 48, 100, 4, 96},
+    {64, 32, 28, 16, 64},   {64, 32, 60, 4, 128},   {64, 48, 14, 16, 160}, {64, 48, 100, 4, 96},
     {64, 48, 148, 1, 288},  {64, 64, 14, 16, 256},  {64, 64, 48, 4, 128},  {64, 64, 72, 2, 256},
     {64, 64, 108, 4, 128},  {64, 96, 6, 0, 0},      {64, 96, 48, 8, 288},  {64, 128, 3, 0, 0},
     {64, 128, 7, 16, 512},  {64, 192, 6, 0, 0},     {64, 256, 4, 0, 0},    {64, 512, 1, 0, 0},

@@ -55,7 +55,7 @@ struct WideCfg {
     static constexpr size_t STAGE_BYTES = THERM ? 6 * sizeof(T) * (size_t)POINTS : 0;
     static constexpr bool STAGE = THERM && BASE_BYTES + STAGE_BYTES <= 227 * 1024;
     static constexpr size_t smem_bytes = BASE_BYTES + (STAGE ? STAGE_BYTES : 0);
-    static_assert(N % 16 == 0 && G % 2 == 0, "bad wide split");
+    static_assert(N % 16 == 0 && G % 2 == 0 && NT % 32 == 0, "bad wide split");
 };
 
 // Workspace: barrier counters (zeroed before the launch), then per instance the two planes and

@@ -58,6 +58,7 @@ struct ResidentArgs {
     int ytiles, tz;  // tiles along y, planes per tile (the last tile may have fewer)
     unsigned *bar, *err;  // arrivals at the grid barriers; set to 1 when a wait ran out
     unsigned long long limit_ns;
+    unsigned withheld;  // as WideWs::withheld
 };
 
 // A voxel's class: which of its directions end at a face (1 x, 2 y, 4 z).  Every branch of
@@ -173,7 +174,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
     const R* qp = Q + col;
     // the rows next to the tile's; at the domain's ends a row of its own, loaded and not used
     const int off_m = ya > 0 ? -n : 0, off_p = yb + 1 < n ? 2 * n : n;
-    unsigned target = 0;
+    unsigned target = ra.withheld;
     for (int s = 0; s < ra.count; ++s) {
         const R* src = ((s & 1) ? Tb : Ta) + col;  // the faces of the previous sweep (at first: the whole grid)
         R* dst = ((s & 1) ? Ta : Tb) + col;
@@ -370,7 +371,9 @@ cudaError_t launch_jacobi_resident(R* Ta, R* Tb, const R* Q, const JacobiCoef<R>
     ra.count = count;
     ra.bar = bar;
     ra.err = err;
-    ra.limit_ns = 2000000000ull;
+    const BarrierLimit bl = barrier_limit();
+    ra.limit_ns = bl.ns;
+    ra.withheld = bl.withheld;
     const cudaError_t e = cudaMemsetAsync(bar, 0, sizeof(unsigned), s);
     if (e != cudaSuccess) return e;
     const int ctas = ra.ytiles * zt;

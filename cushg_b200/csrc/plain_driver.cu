@@ -124,10 +124,8 @@ shg_status plain_solve_device(const shg_params& p, const void* signal_in, void* 
             stats->steps = d.nsteps;
             stats->outer_iterations = 1;
             stats->device_ms = ms;
-            if (!std::isfinite(h[0]) || !std::isfinite(h[1]))
+            if ((rc = march_status(h, 1)) == SHG_OK && (!std::isfinite(h[0]) || !std::isfinite(h[1])))
                 rc = fail(SHG_ERR_NONFINITE, "SH / pump power %g / %g", h[0], h[1]);
-            else if (h[0] < 0.0)
-                rc = fail(SHG_ERR_CUDA, "a grid barrier of the march ran out");
         }
     } while (0);
     if (t0) cudaEventDestroy(t0);
@@ -349,7 +347,7 @@ shg_status plain_solve_batch(const shg_params* params, int count, void* const* p
             rc = cuda_fail(e, "launch ssfm_plain_kernel");
             break;
         }
-        if (sh_power_out) {
+        if (sh_power_out || copies) {  // the host-buffer call waits anyway: it reports a wait that ran out
             std::vector<double> h(2 * (size_t)count);
             if ((e = cudaMemcpyAsync(h.data(), pw, sizeof(double) * 2 * (size_t)count, cudaMemcpyDeviceToHost, stream)) !=
                     cudaSuccess ||
@@ -357,10 +355,9 @@ shg_status plain_solve_batch(const shg_params* params, int count, void* const* p
                 rc = cuda_fail(e, "batch run");
                 break;
             }
-            for (int i = 0; i < count; ++i) sh_power_out[i] = h[2 * (size_t)i];
-            for (int i = 0; i < count && rc == SHG_OK; ++i)
-                if (h[2 * (size_t)i] < 0.0) rc = fail(SHG_ERR_CUDA, "instance %d: a grid barrier of the march ran out", i);
-            for (int i = 0; i < count && rc == SHG_OK; ++i)
+            for (int i = 0; i < count && sh_power_out; ++i) sh_power_out[i] = h[2 * (size_t)i];
+            rc = march_status(h.data(), count);
+            for (int i = 0; i < count && sh_power_out && rc == SHG_OK; ++i)
                 if (!std::isfinite(h[2 * (size_t)i]) || !std::isfinite(h[2 * (size_t)i + 1]))
                     rc = fail(SHG_ERR_NONFINITE, "instance %d: SH / pump power %g / %g", i, h[2 * (size_t)i],
                               h[2 * (size_t)i + 1]);
@@ -480,7 +477,7 @@ extern "C" shg_status shg_batch_plan_powers(shg_batch_plan* plan, double* sh_pow
         (e = cudaStreamSynchronize((cudaStream_t)stream)) != cudaSuccess)
         return cuda_fail(e, "plan powers");
     for (int i = 0; i < plan->count; ++i) sh_power_out[i] = h[2 * (size_t)i];
-    return SHG_OK;
+    return march_status(h.data(), plan->count);
 }
 
 extern "C" void shg_batch_plan_destroy(shg_batch_plan* plan) {

@@ -102,6 +102,21 @@ cudaError_t dev_free_bytes(size_t* bytes) {
     return cudaSuccess;
 }
 
+static thread_local double g_withhold_us = 0.0;
+
+BarrierLimit barrier_limit() {
+    if (g_withhold_us > 0.0) return {(unsigned long long)(1e3 * g_withhold_us), 1u};
+    return {2000000000ull, 0u};
+}
+
+shg_status march_status(const double* powers, int count) {
+    for (int i = 0; i < count; ++i)
+        if (powers[2 * (size_t)i] < 0.0)
+            return count > 1 ? fail(SHG_ERR_CUDA, "instance %d: a grid barrier of the march ran out", i)
+                             : fail(SHG_ERR_CUDA, "a grid barrier of the march ran out");
+    return SHG_OK;
+}
+
 // Physical constants, src/headers/Crystal.h:19-21 (µm, ps, W, V).
 const double kPi = 3.14159265358979323846;
 const double kC = 299792458 * 1E6 / 1E12;
@@ -397,11 +412,19 @@ static shg_status solve_host(const shg_params* p, const void* signal_in, void* p
             rc = cuda_fail(e, "cudaMemcpyAsync H2D");
             break;
         }
+        // a plain run without stats is asynchronous and could not report a wait that ran out; this
+        // call waits anyway
+        shg_stats own;
+        shg_stats* st_out = stats || p->thermal ? stats : &own;
         if (slices) {
-            rc = p->thermal ? thermal_solve_device(*p, din, nullptr, nullptr, dT, stats, s, dp, ds)
-                            : plain_solve_device(*p, din, nullptr, nullptr, stats, s, dp, ds);
+            rc = p->thermal ? thermal_solve_device(*p, din, nullptr, nullptr, dT, st_out, s, dp, ds)
+                            : plain_solve_device(*p, din, nullptr, nullptr, st_out, s, dp, ds);
         } else {
-            rc = shg_solve_device(p, din, dp, ds, dT, stats, s);
+            rc = shg_solve_device(p, din, dp, ds, dT, st_out, s);
+        }
+        if (rc == SHG_ERR_NONFINITE && st_out == &own) {  // powers nobody asked for
+            clear_error();
+            rc = SHG_OK;
         }
         if (rc != SHG_OK) break;
         if (dp && (e = cudaMemcpyAsync(pump_out, dp, outb, cudaMemcpyDeviceToHost, s)) != cudaSuccess) {
@@ -502,6 +525,13 @@ shg_status shg_heat_steady_device(const shg_params* p, void* temperature_dev, co
     if (((uintptr_t)temperature_dev & al) || ((uintptr_t)q_dev & al))
         return fail(SHG_ERR_INVALID, "temperature and Q must be aligned to %d bytes", (int)al + 1);
     return heat_steady_device(q, temperature_dev, q_dev, residual_out, (cudaStream_t)stream);
+}
+
+shg_status shg_selftest_withhold_arrival(double wait_us) {
+    clear_error();
+    if (!(wait_us >= 0.0 && wait_us <= 2e6)) return fail(SHG_ERR_INVALID, "wait_us must be in 0..2e6");
+    g_withhold_us = wait_us;
+    return SHG_OK;
 }
 
 shg_status shg_reserve_device_memory(int64_t bytes) {

@@ -31,6 +31,17 @@ cudaError_t dev_alloc(void** ptr, size_t bytes, cudaStream_t s);
 // Device memory dev_alloc can still hand out: what is free, and what the pool holds unused.
 cudaError_t dev_free_bytes(size_t* bytes);
 
+// Bound of a grid barrier's wait (grid_barrier.cuh), and how many arrivals beyond the real ones it
+// waits for: 0, or 1 while the calling thread runs shg_selftest_withhold_arrival.
+struct BarrierLimit {
+    unsigned long long ns;
+    unsigned withheld;
+};
+BarrierLimit barrier_limit();
+// SHG_ERR_CUDA if one of `count` instances' {SH, pump} powers, stored one after the other, is the
+// negative mark of a march whose barrier wait ran out (kWideTimedOut); its fields are unfinished.
+shg_status march_status(const double* powers, int count);
+
 double sellmeier(int crystal, double L, double T);
 double delta_k(const shg_params& p, double T);
 // dn/dT and dΔk/dT in closed form (crystal.cuh)

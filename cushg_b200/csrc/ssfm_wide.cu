@@ -41,7 +41,9 @@ cudaError_t wide_march(const InstDesc* dev_descs, const InstDesc*, int count, cu
     ws.off_s = plane;
     ws.off_part = 2 * plane;
     ws.stride = 2 * plane + up(sizeof(double) * 2 * N);
-    ws.limit_ns = 2000000000ull;
+    const BarrierLimit bl = barrier_limit();
+    ws.limit_ns = bl.ns;
+    ws.withheld = bl.withheld;
     const int batch = count < fit ? count : fit;
     char* buf = nullptr;
     const size_t bars = up(sizeof(unsigned) * 2 * (size_t)count);

@@ -65,6 +65,7 @@ struct WideWs {
     char* base;
     size_t stride, off_s, off_part;
     unsigned long long limit_ns;  // bound of each barrier wait
+    unsigned withheld;            // arrivals every barrier waits for beyond those there are (self-test; else 0)
 };
 
 // SH and pump power an instance reports when one of its barrier waits ran out (powers are sums
@@ -357,7 +358,7 @@ __global__ void __launch_bounds__(WideCfg<T, N, THERM>::NT, WideCfg<T, N, THERM>
     if constexpr (THERM) stage_slice(0);
     points(0, -1);
     rows_out();
-    unsigned target = 0;
+    unsigned target = ws.withheld;
     double z = 0.0;
     bool ok = true;
     for (int s = 0; s < nsteps; ++s) {

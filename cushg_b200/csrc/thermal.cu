@@ -92,7 +92,7 @@ __global__ void thermal_power_kernel(const InstDesc* __restrict__ descs) {
     for (int i = lane; i < n; i += 32) a += d.w_out[((size_t)f * n + i) * n];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-    if (lane == 0 && d.power_out[f] >= 0.0) d.power_out[f] = a * (f ? d.pw_p : d.pw_s);  // < 0: the march gave up
+    if (lane == 0) d.power_out[f] = a * (f ? d.pw_p : d.pw_s);
 }
 
 template <typename R>

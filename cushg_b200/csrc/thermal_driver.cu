@@ -200,7 +200,7 @@ shg_status ti_alloc(ThermalInst<R>& t, cudaStream_t s) {
     const size_t nt = (size_t)n * n * nz, arr = sizeof(R) * nt;
     const size_t npart = jacobi_partials(p);
     const size_t nw = 2 * (size_t)n * n;
-    const size_t bytes = 6 * arr + sizeof(double) * (npart + 4 + nw) + 256;
+    const size_t bytes = 6 * arr + sizeof(double) * (npart + 2 + nw) + 256;
     cudaError_t e;
     if ((e = dev_alloc((void**)&t.buf, bytes, s)) != cudaSuccess) return cuda_fail(e, "cudaMallocAsync");
     t.Ta = reinterpret_cast<R*>(t.buf);
@@ -211,8 +211,7 @@ shg_status ti_alloc(ThermalInst<R>& t, cudaStream_t s) {
     t.NS = t.NP + nt;
     t.partial = reinterpret_cast<double*>(t.NS + nt);
     t.resid = t.partial + npart;                            // [0] convergence value, [1] staging-error word
-    t.power = t.resid + 2;                                  // [2]
-    t.w_out = t.power + 2;                                  // [2][n*n]
+    t.w_out = t.resid + 2;                                  // [2][n*n]
     t.tb_err = reinterpret_cast<unsigned*>(t.resid + 1);    // set by a blocked sweep whose staging timed out
     t.k = make_jacobi_coef<R>(p);
     // Solver.h:332: tol = 5e-4 / TSIZE in the working precision
@@ -231,7 +230,7 @@ shg_status ti_alloc(ThermalInst<R>& t, cudaStream_t s) {
 template <typename R>
 shg_status ti_init(ThermalInst<R>& t, cudaStream_t s) {
     cudaError_t e;
-    if ((e = cudaMemsetAsync(t.resid, 0, 4 * sizeof(double), s)) != cudaSuccess) return cuda_fail(e, "memset");
+    if ((e = cudaMemsetAsync(t.resid, 0, 2 * sizeof(double), s)) != cudaSuccess) return cuda_fail(e, "memset");
     if ((e = launch_thermal_init<R>(t.Ta, t.Tb, t.Q, *t.p, s)) != cudaSuccess) return cuda_fail(e, "thermal init");
     return SHG_OK;
 }
@@ -372,6 +371,8 @@ shg_status thermal_batch_run(const shg_params* ps, int count, const void* const*
     std::vector<ThermalState> states(count);
     std::vector<int> act(count);
     InstDesc* dd = nullptr;
+    double* pw = nullptr;  // device, {SH, pump} power per instance
+    std::vector<double> h(2 * (size_t)count);
     std::unique_ptr<HeatDirect> heat;  // one FP64 workspace for the batch's direct heat solves
     for (int i = 0; i < count; ++i)
         if (ps[i].heat_solver == SHG_HEAT_DIRECT && !heat) heat.reset(new HeatDirect);
@@ -385,12 +386,14 @@ shg_status thermal_batch_run(const shg_params* ps, int count, const void* const*
     cudaEvent_t ej[3] = {nullptr, nullptr, nullptr};
     for (auto& ev : ej) cudaEventCreate(&ev);
     do {
-        if ((e = dev_alloc((void**)&dd, sizeof(InstDesc) * (size_t)count, s)) != cudaSuccess) {
+        if ((e = dev_alloc((void**)&dd, (sizeof(InstDesc) + 2 * sizeof(double)) * (size_t)count, s)) != cudaSuccess) {
             rc = cuda_fail(e, "cudaMallocAsync");
             break;
         }
+        pw = reinterpret_cast<double*>(dd + count);
         for (int i = 0; i < count && rc == SHG_OK; ++i) {
             ti[i].p = &ps[i];
+            ti[i].power = pw + 2 * (size_t)i;
             ti[i].signal_in = signal_in ? signal_in[i] : nullptr;
             ti[i].pump_out = pump_out ? pump_out[i] : nullptr;
             ti[i].signal_out = signal_out ? signal_out[i] : nullptr;
@@ -402,6 +405,10 @@ shg_status thermal_batch_run(const shg_params* ps, int count, const void* const*
         // the device time starts after the workspace is allocated (a pool that grows maps
         // memory on the host's time, while the stream idles)
         cudaEventRecord(t0, s);
+        if ((e = cudaMemsetAsync(pw, 0, 2 * sizeof(double) * (size_t)count, s)) != cudaSuccess) {
+            rc = cuda_fail(e, "memset");
+            break;
+        }
         for (int i = 0; i < count && rc == SHG_OK; ++i) rc = ti_init<R>(ti[i], s);
         if (rc != SHG_OK) break;
         for (int g = 0; rc == SHG_OK; ++g) {
@@ -435,7 +442,14 @@ shg_status thermal_batch_run(const shg_params* ps, int count, const void* const*
             const PlainVariant* w = p0.march == SHG_MARCH_AUTO ? wide_thermal_variant(p0.precision, p0.nx, na) : nullptr;
             if ((e = run_variant(w ? w : v, dd, hd.data(), na, nullptr, s)) != cudaSuccess) { rc = cuda_fail(e, "thermal optical pass"); break; }
             cudaEventRecord(ej[2], s);
-            if ((e = cudaEventSynchronize(ej[2])) != cudaSuccess) { rc = cuda_fail(e, "thermal optical pass"); break; }
+            // the wide march writes power slots only to report a barrier wait that ran out (the powers
+            // come at the end): seen before the next outer iteration reads the pass's heat source
+            if (w && (e = cudaMemcpyAsync(h.data(), pw, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, s)) != cudaSuccess) {
+                rc = cuda_fail(e, "thermal optical pass");
+                break;
+            }
+            if ((e = cudaStreamSynchronize(s)) != cudaSuccess) { rc = cuda_fail(e, "thermal optical pass"); break; }
+            if (w && (rc = march_status(h.data(), count)) != SHG_OK) break;
             float ms = 0.f;
             cudaEventElapsedTime(&ms, ej[1], ej[2]);
             for (int a = 0; a < na; ++a) {
@@ -466,10 +480,8 @@ shg_status thermal_batch_run(const shg_params* ps, int count, const void* const*
                 rc = cuda_fail(e, "thermal powers");
                 break;
             }
-            std::vector<double> h(2 * (size_t)count);
-            for (int i = 0; i < count && e == cudaSuccess; ++i)
-                e = cudaMemcpyAsync(&h[2 * (size_t)i], ti[i].power, 2 * sizeof(double), cudaMemcpyDeviceToHost, s);
-            if (e != cudaSuccess || (e = cudaStreamSynchronize(s)) != cudaSuccess) {
+            if ((e = cudaMemcpyAsync(h.data(), pw, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
+                (e = cudaStreamSynchronize(s)) != cudaSuccess) {
                 rc = cuda_fail(e, "thermal run");
                 break;
             }
@@ -487,7 +499,6 @@ shg_status thermal_batch_run(const shg_params* ps, int count, const void* const*
                 st.device_ms = ms;
                 st.jacobi_ms = ti[i].jacobi_ms;
                 st.optics_ms = ti[i].optics_ms;
-                if (rc == SHG_OK && st.sh_power < 0.0) rc = fail(SHG_ERR_CUDA, "a grid barrier of the march ran out");
                 if (rc == SHG_OK && (!std::isfinite(st.sh_power) || !std::isfinite(st.pump_power)))
                     rc = count > 1 ? fail(SHG_ERR_NONFINITE, "instance %d: SH / pump power %g / %g", i, st.sh_power,
                                           st.pump_power)

@@ -28,7 +28,7 @@ EXPORTS = (
     "shg_status_string", "shg_version", "shg_heat_sweeps_device", "shg_batch_plan_create", "shg_batch_plan_launch",
     "shg_batch_plan_powers", "shg_batch_plan_destroy", "shg_autotune", "shg_grad_batch", "shg_solve_batch",
     "shg_thermal_grad", "shg_autotune_batch", "shg_autotune_reset", "shg_set_schedule",
-    "shg_reserve_device_memory", "shg_fp32_error_estimate", "shg_selftest_bounded_wait",
+    "shg_reserve_device_memory", "shg_fp32_error_estimate", "shg_selftest_bounded_wait", "shg_selftest_withhold_arrival",
     "shg_thermal_batch", "shg_heat_steady_device", "shg_heat_operator_modes",
 )
 
@@ -86,6 +86,8 @@ def lib() -> ctypes.CDLL:
         L.shg_thermal_batch.restype = ctypes.c_int
         L.shg_selftest_bounded_wait.argtypes = [ctypes.c_int32, ctypes.c_double, ctypes.c_int32]
         L.shg_selftest_bounded_wait.restype = ctypes.c_int
+        L.shg_selftest_withhold_arrival.argtypes = [ctypes.c_double]
+        L.shg_selftest_withhold_arrival.restype = ctypes.c_int
         L.shg_fp32_error_estimate.argtypes = [P]
         L.shg_fp32_error_estimate.restype = ctypes.c_double
         L.shg_steps.argtypes = [P]
@@ -173,6 +175,12 @@ def selftest_bounded_wait(precision: int, wait_us: float, withhold_plane: int) -
     """shg_selftest_bounded_wait: raises ShgError(SHG_ERR_CUDA) when a staged plane's wait ran
     out."""
     _check(lib().shg_selftest_bounded_wait(int(precision), float(wait_us), int(withhold_plane)))
+
+
+def selftest_withhold_arrival(wait_us: float) -> None:
+    """shg_selftest_withhold_arrival: while wait_us > 0, this thread's cooperative launches wait for
+    an arrival that never comes and report that the wait ran out; 0: as usual."""
+    _check(lib().shg_selftest_withhold_arrival(float(wait_us)))
 
 
 def steps(p: ShgParams) -> int:

@@ -224,7 +224,10 @@ SHG_API shg_status shg_solve_slices(const shg_params* p, const void* signal_in, 
 
 /* The same with device buffers on a caller stream (a cudaStream_t, NULL = legacy
  * default stream).  Plain runs are asynchronous; thermal runs synchronise at each
- * Jacobi convergence check.  stats, if given, is filled after a synchronise. */
+ * Jacobi convergence check.  stats, if given, is filled after a synchronise.  A run on its own
+ * takes a march of cooperative launches (shg_params.march), whose waits are bounded: one that runs
+ * out (2 s) leaves the outputs unfinished and the call returns SHG_ERR_CUDA, except a plain run
+ * with stats NULL, which has returned by then. */
 SHG_API shg_status shg_solve_device(const shg_params* p, const void* signal_in_dev,
                             void* pump_out_dev, void* signal_out_dev,
                             void* temperature_out_dev, shg_stats* stats, void* stream);
@@ -235,7 +238,8 @@ SHG_API shg_status shg_solve_device(const shg_params* p, const void* signal_in_d
  * fed by a device work queue.  Replaces the one-process-per-point sweep of
  * src/cuSHG.sh:58-94.  All instances must share `precision` and have thermal == 0.
  * pump_out[i] / signal_out[i]: device buffers (nx_i*ny_i complex) or NULL entries.
- * sh_power_out: host array of `count` doubles or NULL.
+ * sh_power_out: host array of `count` doubles or NULL.  NULL: the call is asynchronous and cannot
+ * report a march whose bounded wait ran out (shg_solve_device); shg_solve_batch always does.
  */
 SHG_API shg_status shg_solve_batch_device(const shg_params* params, int32_t count,
                                   void* const* pump_out_dev, void* const* signal_out_dev,
@@ -264,7 +268,8 @@ SHG_API shg_status shg_solve_batch(const shg_params* params, int32_t count, void
  *   shg_batch_plan_launch   replays the graph on `stream`; launches of one plan that overlap
  *                           on the GPU race on its work queues and power slots.
  *   shg_batch_plan_powers   copies the SH powers of the last finished replay to the host
- *                           array sh_power_out[count] (stream-ordered, then synchronises).
+ *                           array sh_power_out[count] (stream-ordered, then synchronises);
+ *                           SHG_ERR_CUDA if a bounded wait of that replay's marches ran out.
  *   shg_batch_plan_destroy  synchronises the device and frees the plan.
  */
 typedef struct shg_batch_plan shg_batch_plan;
@@ -428,6 +433,15 @@ SHG_API shg_status shg_thermal_batch(const shg_params* params, int32_t count, vo
  * in the reference.
  */
 SHG_API shg_status shg_selftest_bounded_wait(int32_t precision, double wait_us, int32_t withhold_plane);
+
+/*
+ * Diagnostics: the bounded waits of the cooperative launches (the marches of single runs and few
+ * instances, resident Jacobi sweeps).  While wait_us > 0, those that the calling thread launches or
+ * captures wait at every grid barrier for one arrival more than there are, wait_us microseconds at
+ * most, then stop and report: the calls return SHG_ERR_CUDA.  0 (the state of a new thread):
+ * as usual.  The device stays usable.  No counterpart in the reference.
+ */
+SHG_API shg_status shg_selftest_withhold_arrival(double wait_us);
 
 /* Gradients of the SH output power (plain runs), from shg_grad. */
 typedef struct shg_grad_result {

@@ -572,6 +572,23 @@ shg_status shg_reserve_device_memory(int64_t bytes) {
     return rc;
 }
 
+shg_status shg_release_device_memory(int64_t keep_bytes) {
+    clear_error();
+    if (keep_bytes < 0) return fail(SHG_ERR_INVALID, "keep_bytes must be >= 0");
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return fail(SHG_ERR_NO_DEVICE, "no CUDA device visible");
+    }
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    if (dev >= 0 && dev < 64 && g_pools[dev] && (e = cudaMemPoolTrimTo(g_pools[dev], (size_t)keep_bytes)) != cudaSuccess)
+        return cuda_fail(e, "cudaMemPoolTrimTo");
+    // workspaces of batch plans are graph memory nodes
+    e = cudaDeviceGraphMemTrim(dev);
+    return e == cudaSuccess ? SHG_OK : cuda_fail(e, "cudaDeviceGraphMemTrim");
+}
+
 shg_status shg_solve_batch(const shg_params* params, int32_t count, void* const* pump_out, void* const* signal_out,
                            double* sh_power_out) {
     clear_error();

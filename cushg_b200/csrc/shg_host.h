@@ -24,7 +24,7 @@ void clear_error();
 // every step's fields (42 GB for 18 FP64 256 x 256 x 400 instances) spent 570 ms and more of
 // each call on it, against 115 ms of kernels.  What the pool holds unused is not lost to the
 // process: the driver hands it to any other allocation (cudaMalloc and everything built on it)
-// that would fail without it.
+// that would fail without it.  shg_release_device_memory gives it back to other processes.
 constexpr unsigned long long kPoolKeepFraction = 4;
 // Inside a stream capture it falls back to cudaMallocAsync (a graph memory node).
 cudaError_t dev_alloc(void** ptr, size_t bytes, cudaStream_t s);

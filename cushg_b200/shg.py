@@ -28,7 +28,8 @@ EXPORTS = (
     "shg_status_string", "shg_version", "shg_heat_sweeps_device", "shg_batch_plan_create", "shg_batch_plan_launch",
     "shg_batch_plan_powers", "shg_batch_plan_destroy", "shg_autotune", "shg_grad_batch", "shg_solve_batch",
     "shg_thermal_grad", "shg_autotune_batch", "shg_autotune_reset", "shg_set_schedule",
-    "shg_reserve_device_memory", "shg_fp32_error_estimate", "shg_selftest_bounded_wait", "shg_selftest_withhold_arrival",
+    "shg_reserve_device_memory", "shg_release_device_memory", "shg_fp32_error_estimate", "shg_selftest_bounded_wait",
+    "shg_selftest_withhold_arrival",
     "shg_thermal_batch", "shg_heat_steady_device", "shg_heat_operator_modes",
 )
 
@@ -142,6 +143,8 @@ def lib() -> ctypes.CDLL:
         L.shg_set_schedule.restype = ctypes.c_int
         L.shg_reserve_device_memory.argtypes = [ctypes.c_int64]
         L.shg_reserve_device_memory.restype = ctypes.c_int
+        L.shg_release_device_memory.argtypes = [ctypes.c_int64]
+        L.shg_release_device_memory.restype = ctypes.c_int
         L.shg_last_error.restype = ctypes.c_char_p
         L.shg_status_string.argtypes = [ctypes.c_int32]
         L.shg_status_string.restype = ctypes.c_char_p
@@ -498,6 +501,11 @@ def autotune_reset() -> None:
 def reserve_device_memory(nbytes: int) -> None:
     """shg_reserve_device_memory: grow the library's pool to hold nbytes and keep them."""
     _check(lib().shg_reserve_device_memory(int(nbytes)))
+
+
+def release_device_memory(keep_bytes: int = 0) -> None:
+    """shg_release_device_memory: give what the library's pool holds unused back to the device."""
+    _check(lib().shg_release_device_memory(int(keep_bytes)))
 
 
 def set_schedule(precision: int, n: int, cluster: int, threads: int) -> None:

@@ -323,6 +323,14 @@ SHG_API shg_status shg_autotune_batch(const shg_params* params, int32_t count, s
  * Synchronous.  No counterpart in the reference. */
 SHG_API shg_status shg_reserve_device_memory(int64_t bytes);
 
+/* Give the memory that the library's pool on the current device holds unused back to the device,
+ * all but keep_bytes of it.  Between calls the pool keeps up to a quarter of the device
+ * (SHG_POOL_KEEP_MB); the driver hands that to other allocations of this process by itself, but
+ * not to other processes.  Workspace whose call has not finished on the GPU stays; what batch
+ * plans' replays used goes back once they are destroyed.  Later calls map memory again as they
+ * need it.  No counterpart in the reference. */
+SHG_API shg_status shg_release_device_memory(int64_t keep_bytes);
+
 /* Forget the choices of shg_autotune / shg_autotune_batch: later runs use the compiled
  * default schedules.  No counterpart in the reference. */
 SHG_API void shg_autotune_reset(void);

@@ -165,3 +165,11 @@ def test_fp32_error_estimate_follows_the_phase_mismatch_cancellation():
     assert abs(longer / matched - 2.0) < 1e-6
     # an elliptical beam goes through the general envelope
     assert shg.fp32_error_estimate(p.replace(waist_y=45.0)) > 0
+
+
+def test_release_device_memory_checks_its_argument():
+    import torch
+    L = shg.lib()
+    assert L.shg_release_device_memory(-1) == P.SHG_ERR_INVALID
+    if not torch.cuda.is_available():
+        assert L.shg_release_device_memory(0) == P.SHG_ERR_NO_DEVICE

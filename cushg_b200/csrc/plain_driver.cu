@@ -62,6 +62,18 @@ const PlainVariant* few_choice(const shg_params& p, const PlainVariant* v, int l
     return few_runs_variant(v->precision, v->n, level, upto);
 }
 
+// run_variant, or where a march's workspace cannot be had the fused march, which needs none and gives
+// the same bits, on the sides it is built for.
+cudaError_t run_plain(const PlainVariant* v, const InstDesc* dev_descs, const InstDesc* host_descs, int count, int* queue,
+                      cudaStream_t stream) {
+    const cudaError_t e = run_variant(v, dev_descs, host_descs, count, queue, stream);
+    if (e != cudaErrorMemoryAllocation || !v->mp) return e;
+    const PlainVariant* fused = find_plain_variant(v->precision, v->n, 0, SHG_MARCH_FUSED);
+    if (!fused) return e;
+    cudaGetLastError();
+    return run_variant(fused, dev_descs, host_descs, count, queue, stream);
+}
+
 // The descriptor of one run, as a kernel argument: no copy from the caller's stack.
 __global__ void put_desc_kernel(InstDesc d, InstDesc* out) {
     if (threadIdx.x == 0) *out = d;
@@ -107,7 +119,7 @@ shg_status plain_solve_device(const shg_params& p, const void* signal_in, void* 
             cudaEventCreate(&t1);
             cudaEventRecord(t0, stream);
         }
-        if ((e = run_variant(v, dd, &d, 1, nullptr, stream)) != cudaSuccess) { rc = cuda_fail(e, "launch ssfm_plain_kernel"); break; }
+        if ((e = run_plain(v, dd, &d, 1, nullptr, stream)) != cudaSuccess) { rc = cuda_fail(e, "launch ssfm_plain_kernel"); break; }
         if (stats) {
             cudaEventRecord(t1, stream);
             double h[2] = {0, 0};
@@ -241,8 +253,8 @@ static cudaError_t enqueue_batch(const BatchLayout& L, const InstDesc* dd, int* 
     const int ng = (int)L.groups.size();
     if ((e = cudaMemsetAsync(queues, 0, sizeof(int) * (size_t)ng, stream)) != cudaSuccess) return e;
     if (ng == 1) {
-        if ((e = run_variant(L.groups[0].v, dd + L.groups[0].begin, L.descs.data() + L.groups[0].begin,
-                             L.groups[0].end - L.groups[0].begin, queues, stream)) != cudaSuccess)
+        if ((e = run_plain(L.groups[0].v, dd + L.groups[0].begin, L.descs.data() + L.groups[0].begin,
+                           L.groups[0].end - L.groups[0].begin, queues, stream)) != cudaSuccess)
             return e;
         return copy_group_outputs(L, L.groups[0], ho, cbytes, stream);
     }
@@ -252,7 +264,7 @@ static cudaError_t enqueue_batch(const BatchLayout& L, const InstDesc* dd, int* 
         if ((e = cudaStreamWaitEvent(fs[g], ev[nfork], 0)) != cudaSuccess) return e;
     for (int g = 0; g < ng; ++g) {
         const BatchLayout::Group& G = L.groups[g];
-        if ((e = run_variant(G.v, dd + G.begin, L.descs.data() + G.begin, G.end - G.begin, queues + g, fs[g % nf])) !=
+        if ((e = run_plain(G.v, dd + G.begin, L.descs.data() + G.begin, G.end - G.begin, queues + g, fs[g % nf])) !=
                 cudaSuccess ||
             (e = copy_group_outputs(L, G, ho, cbytes, fs[g % nf])) != cudaSuccess)
             return e;

@@ -440,7 +440,13 @@ shg_status thermal_batch_run(const shg_params* ps, int count, const void* const*
             // the wide march while the instances still iterating are few enough for it (the
             // marches agree bit for bit, so an instance's results do not depend on the choice)
             const PlainVariant* w = p0.march == SHG_MARCH_AUTO ? wide_thermal_variant(p0.precision, p0.nx, na) : nullptr;
-            if ((e = run_variant(w ? w : v, dd, hd.data(), na, nullptr, s)) != cudaSuccess) { rc = cuda_fail(e, "thermal optical pass"); break; }
+            e = run_variant(w ? w : v, dd, hd.data(), na, nullptr, s);
+            if (w && e == cudaErrorMemoryAllocation) {  // no workspace for it
+                cudaGetLastError();
+                w = nullptr;
+                e = run_variant(v, dd, hd.data(), na, nullptr, s);
+            }
+            if (e != cudaSuccess) { rc = cuda_fail(e, "thermal optical pass"); break; }
             cudaEventRecord(ej[2], s);
             // the wide march writes power slots only to report a barrier wait that ran out (the powers
             // come at the end): seen before the next outer iteration reads the pass's heat source

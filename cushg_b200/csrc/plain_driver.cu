@@ -171,7 +171,8 @@ static BatchLayout batch_layout(const shg_params* params, int count, void* const
     }
     // A small batch takes the variants for few runs, each class from its widest on until the batch
     // fits: the classes share the device, so the parts of it that they fill must add up to at most one.
-    for (int level = 0; level < kFewLevels; ++level) {
+    bool fits = false;
+    for (int level = 0; level < kFewLevels && !fits; ++level) {
         std::vector<const PlainVariant*> few;
         double share = 0.0;
         for (int i = 0; i < count && share < 1.0 + 1e-9; ++i) {
@@ -184,7 +185,19 @@ static BatchLayout batch_layout(const shg_params* params, int count, void* const
         }
         if ((int)few.size() < count || share >= 1.0 + 1e-9) continue;
         for (int i = 0; i < count; ++i) items[i].v = few[i];
-        break;
+        fits = true;
+    }
+    if (!fits) {
+        auto small = [&](int i) { return items[i].v->precision == 32 && items[i].v->n == 64 && params[i].march == SHG_MARCH_AUTO; };
+        int runs64 = 0, to_128 = 0, above = 0;
+        for (int i = 0; i < count; ++i) {
+            runs64 += small(i);
+            to_128 += items[i].v->n > 64 && items[i].v->n <= 128;
+            above += items[i].v->n > 128;
+        }
+        const PlainVariant* w = has_plain_choice(32, 64, 0) ? nullptr : many_small_variant(runs64, to_128, above);
+        for (int i = 0; i < count && w; ++i)
+            if (small(i)) items[i].v = w;
     }
     std::stable_sort(items.begin(), items.end(), [](const Item& a, const Item& b) {
         if (a.v != b.v) return a.v < b.v;

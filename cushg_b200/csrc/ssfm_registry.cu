@@ -33,7 +33,7 @@ void for_each_variant(F&& f, bool few = false) {
 // us per step at the first and last count of a row (parts of the step count's start-up included) /
 // of the default there:
 //   FP32 32: 1-28 3.4-4.8 / 5.3-5.8.  48: 1-14 3.9-4.9 / 11, 15-100 7.3-12.0 / 11-12.
-//   64: 1-14 4.1-5.0 / 14.1, 15-104 7.8-14.0 / 14.2-15.2, from 149 26.7 / 30.0 (220 runs).  96: 1-7 5.6-5.7 / 30.5, 8-48 10-19 /
+//   64: 1-14 4.1-5.0 / 14.1, 15-104 7.8-14.0 / 14.2-15.2.  96: 1-7 5.6-5.7 / 30.5, 8-48 10-19 /
 //   31, 49-72 24 / 31.  128: 1-2 6.3-6.7 / 29.8, 3-7 7.5 / 29.8, 8-48 12-27 / 30.5, 73-108 44 / 61.
 //   192: 1-9 7.2-23 / 37.6, 10-16 27 / 37.6, 37-56 58-61 / 74.  256: 1-4 8.4-18 / 24,
 //   5-6 21.5 / 24.
@@ -45,7 +45,7 @@ void for_each_variant(F&& f, bool few = false) {
 struct FewRow { int precision, n, upto, cluster, threads; };
 const FewRow kFew[] = {
     {32, 32, 28, 16, 64},   {32, 48, 14, 16, 96},   {32, 48, 100, 4, 96},  {32, 64, 14, 16, 128},
-    {32, 64, 104, 4, 128},  {32, 64, 148, 1, 512},  {32, 64, 1 << 20, 4, 128}, {32, 96, 7, 16, 288},
+    {32, 64, 104, 4, 128},  {32, 64, 148, 1, 512},  {32, 96, 7, 16, 288},
     {32, 96, 48, 8, 288},   {32, 96, 72, 2, 192},   {32, 128, 2, 0, 0},     {32, 128, 7, 16, 256}, {32, 128, 48, 8, 256},
     {32, 128, 72, 2, 512},  {32, 128, 108, 4, 256}, {32, 192, 9, 0, 0},    {32, 192, 16, 8, 192},
     {32, 192, 36, 4, 384},  {32, 192, 56, 8, 192},  {32, 256, 4, 0, 0},    {32, 256, 6, 16, 256},
@@ -78,6 +78,25 @@ const PlainVariant* few_runs_variant(int precision, int n, int level, int* upto)
         return v;
     }
     return nullptr;
+}
+
+const PlainVariant* find_split(int precision, int n, int cluster, int threads) {
+    const PlainVariant* v = nullptr;
+    for_each_variant([&](const PlainVariant* c) {
+        if (c->precision == precision && c->n == n && !c->thermal && c->cluster == cluster && c->threads == threads) v = c;
+        return v != nullptr;
+    });
+    return v;
+}
+
+// 64 x 64 FP32 runs past the rows of kFew: 4-CTA clusters, five CTAs to an SM, take 26.7 us per step where
+// one CTA of 512 threads per run takes 30.0 (220 runs), as 149 of those are a second wave.  Beside
+// larger sides their CTAs hold up the clusters that need a whole SM: 160 runs of 64 x 64 and 8 of 128 x 128
+// (61 slices) took 2.73 ms against 1.90, with two of 256 x 256 3.2 against 2.0, a sweep of 256 runs over
+// 64-256 75.2 against 74.1.  With up to three runs of 96 x 96 or 128 x 128 beside 149-700 they were
+// never slower (three of 96 x 96 beside 160: 1.87 against 2.70), with four sometimes (128 x 128: 2.66 against 1.87).
+const PlainVariant* many_small_variant(int runs64, int runs_to_128, int runs_above) {
+    return runs64 >= 149 && runs_to_128 <= 3 && runs_above == 0 ? find_split(32, 64, 4, 128) : nullptr;
 }
 
 const PlainVariant* find_plain_variant(int precision, int n, int thermal, int march) {

@@ -1,0 +1,58 @@
+"""Which march and split plain calls take, from the names of the kernels they launch (the profiler's
+records): the rule by the number of runs, and what tuned and pinned schedules do to it."""
+import re
+
+import pytest
+
+from cushg_b200 import params as P
+from cushg_b200 import shg
+
+pytestmark = pytest.mark.gpu
+
+
+def marches(call):
+    """The march kernels that `call` launches: 'plain<float, 64, 4, 128>', 'wide<float, 128>',
+    'multipass<float, 256>'."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    call()
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        call()
+        torch.cuda.synchronize()
+    out = set()
+    for e in prof.events():
+        m = re.search(r"ssfm_plain_kernel<(\w+), (\d+), (\d+), (\d+)", e.name)
+        if m:
+            out.add("plain<%s, %s, %s, %s>" % m.groups())
+        m = re.search(r"(ssfm_wide|mp_row)_kernel<(\w+), (\d+)", e.name)
+        if m:
+            out.add("%s<%s, %s>" % ("wide" if m.group(1) == "ssfm_wide" else "multipass", m.group(2), m.group(3)))
+    return out
+
+
+def run(n, precision=32, nz=4):
+    return P.workload(n, nz, 6000.0, 20.0, 30.0, 3000.0, 30.0, precision=precision)
+
+
+def batch(*classes):
+    ps = [run(n) for n, count in classes for _ in range(count)]
+    return lambda: shg.solve_batch_device(ps)
+
+
+def test_rule_by_the_number_of_runs():
+    assert marches(lambda: shg.solve(run(128))) == {"wide<float, 128>"}
+    assert marches(lambda: shg.solve(run(48, 64))) == {"plain<double, 48, 16, 160>"}
+    assert marches(batch((256, 7))) == {"multipass<float, 256>"}
+    assert marches(batch((64, 160))) == {"plain<float, 64, 4, 128>"}
+    assert marches(batch((128, 200))) == {"plain<float, 128, 2, 512>"}
+
+
+def test_many_small_runs_beside_others():
+    """Four-CTA clusters of 64 x 64 FP32 runs hold up clusters that need a whole SM: they are for
+    batches of small sides, with at most three runs of 96 or 128 beside them."""
+    for others in [(), ((32, 40),), ((48, 8),), ((96, 3),), ((128, 3),)]:
+        assert "plain<float, 64, 4, 128>" in marches(batch((64, 160), *others)), others
+    for others in [((96, 8),), ((128, 4),), ((96, 2), (128, 2)), ((256, 2),), ((192, 1),)]:
+        assert "plain<float, 64, 1, 512>" in marches(batch((64, 160), *others)), others
+    assert marches(batch((64, 140))) == {"plain<float, 64, 1, 512>"}

@@ -6,7 +6,8 @@
 // The tuning batch: enough instances of the class to fill the device three times over for
 // the variant with the most resident clusters, nz = 33 (32 steps), parameters spread like a
 // sweep (waist, focus, power), so the timing sees the steady state of a persistent launch.
-// Each variant runs once untimed, then three times between CUDA events; the median counts.
+// Each variant runs once untimed, then three times between CUDA events; the median counts.  The first
+// is the one that an automatic batch of these runs takes; where it wins, nothing is chosen.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -22,8 +23,8 @@ extern "C" shg_status shg_autotune(int32_t precision, int32_t n, shg_tune_result
     clear_error();
     if (!out) return fail(SHG_ERR_INVALID, "out is NULL");
     if (precision != 32 && precision != 64) return fail(SHG_ERR_INVALID, "precision must be 32 or 64");
-    const PlainVariant* cand[16];
-    const int nc = plain_candidates(precision, n, cand, 16);
+    const PlainVariant* cand[17];
+    int nc = plain_candidates(precision, n, cand, 16);
     if (nc == 0) return fail(SHG_ERR_UNSUPPORTED, "no kernel built for grid side %d at precision %d", n, precision);
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) {
@@ -45,6 +46,7 @@ extern "C" shg_status shg_autotune(int32_t precision, int32_t n, shg_tune_result
     base.precision = precision;
     base.lz = 10000.0;
     std::vector<InstDesc> descs(count);
+    std::vector<shg_params> ps(count);
     for (int i = 0; i < count; ++i) {
         shg_params q = base;
         const double u = (i + 0.5) / count;
@@ -54,14 +56,22 @@ extern "C" shg_status shg_autotune(int32_t precision, int32_t n, shg_tune_result
         q.power = 1.0 + 49.0 * (1.0 - u);
         descs[i] = make_plain_desc(q, q.temp, q.temp);
         descs[i].slot = i;
+        ps[i] = q;
     }
+    clear_plain_choice(precision, n);
+    int runs = 0;
+    const PlainVariant* automatic = plain_batch_variant(ps.data(), count, n, &runs);
+    int at = 0;
+    while (at < nc && cand[at] != automatic) ++at;
+    if (at == nc) cand[nc++] = automatic;
+    std::swap(cand[0], cand[at]);
     cudaStream_t s = nullptr;
     cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
     if (e != cudaSuccess) return cuda_fail(e, "cudaStreamCreate");
     void* buf = nullptr;
     cudaEvent_t ev[2] = {nullptr, nullptr};
     shg_status rc = SHG_OK;
-    double rate[16] = {0};
+    double rate[17] = {0};
     do {
         if ((e = dev_alloc((void**)&buf, sizeof(InstDesc) * (size_t)count + 256, s)) != cudaSuccess) {
             rc = cuda_fail(e, "cudaMallocAsync");
@@ -101,8 +111,9 @@ extern "C" shg_status shg_autotune(int32_t precision, int32_t n, shg_tune_result
     int best = 0;
     for (int c = 1; c < nc; ++c)
         if (rate[c] > rate[best]) best = c;
-    set_plain_choice(cand[best]);
+    if (best) set_plain_choice(cand[best], count);
     std::memset(out, 0, sizeof(*out));
+    out->automatic = best == 0;
     out->precision = precision;
     out->n = n;
     out->cluster = cand[best]->cluster;
@@ -117,9 +128,9 @@ extern "C" shg_status shg_autotune(int32_t precision, int32_t n, shg_tune_result
 // given batch.  The classes of a mixed batch run side by side on forked streams and share
 // the SMs, so the variant that is fastest for a class alone can slow the batch (a class that
 // fills every SM with its own CTAs holds back the clusters of the larger classes).
-// Coordinate descent from the compiled defaults: for each class, largest total work first,
+// Coordinate descent from the automatic choices: for each class, largest total work first,
 // every other compiled variant is timed with the rest fixed and kept if the batch is at
-// least 1 % faster.  A timing is the median of three runs of the batch (no field outputs,
+// least 1 % faster.  A class without such a variant stays automatic.  A timing is the median of three runs of the batch (no field outputs,
 // SH powers kept on the device) after one untimed run.
 extern "C" shg_status shg_autotune_batch(const shg_params* params, int32_t count, shg_tune_result* out,
                                          int32_t max_out, int32_t* n_out) {
@@ -154,14 +165,21 @@ extern "C" shg_status shg_autotune_batch(const shg_params* params, int32_t count
     }
     std::sort(cls.begin(), cls.end(), [](const Cls& a, const Cls& b) { return a.work > b.work; });
     if ((int)cls.size() > max_out) return fail(SHG_ERR_INVALID, "the batch has %d classes, out holds %d", (int)cls.size(), max_out);
-    // start from the compiled defaults
+    // start from the automatic choices (the null candidate)
     std::vector<std::vector<const PlainVariant*>> cand(cls.size());
-    std::vector<int> pick(cls.size(), 0);
+    std::vector<int> pick(cls.size(), 0), runs(cls.size(), 0);
+    auto choose = [&](size_t k, int c) {
+        if (cand[k][c]) set_plain_choice(cand[k][c], runs[k]);
+        else clear_plain_choice(precision, cls[k].n);
+    };
+    for (size_t k = 0; k < cls.size(); ++k) clear_plain_choice(precision, cls[k].n);
     for (size_t k = 0; k < cls.size(); ++k) {
         const PlainVariant* c[16];
         const int nc = plain_candidates(precision, cls[k].n, c, 16);
-        cand[k].assign(c, c + nc);
-        set_plain_choice(cand[k][0]);
+        const PlainVariant* automatic = plain_batch_variant(params, count, cls[k].n, &runs[k]);
+        cand[k].push_back(nullptr);
+        for (int i = 0; i < nc && runs[k] > 0; ++i)
+            if (c[i] != automatic) cand[k].push_back(c[i]);
     }
     cudaStream_t s = nullptr;
     cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
@@ -192,7 +210,7 @@ extern "C" shg_status shg_autotune_batch(const shg_params* params, int32_t count
         t_best = t_default;
         for (size_t k = 0; k < cls.size() && rc == SHG_OK; ++k) {
             for (int c = 1; c < (int)cand[k].size() && rc == SHG_OK; ++c) {
-                set_plain_choice(cand[k][c]);
+                choose(k, c);
                 double t = 0.0;
                 if ((rc = time_batch(&t)) != SHG_OK) break;
                 if (t < 0.99 * t_best) {
@@ -200,7 +218,7 @@ extern "C" shg_status shg_autotune_batch(const shg_params* params, int32_t count
                     pick[k] = c;
                 }
             }
-            set_plain_choice(cand[k][pick[k]]);
+            choose(k, pick[k]);
         }
     } while (0);
     for (cudaEvent_t x : ev)
@@ -208,7 +226,7 @@ extern "C" shg_status shg_autotune_batch(const shg_params* params, int32_t count
     cudaStreamSynchronize(s);
     cudaStreamDestroy(s);
     if (rc != SHG_OK) {
-        for (size_t k = 0; k < cls.size(); ++k) set_plain_choice(cand[k][0]);
+        for (size_t k = 0; k < cls.size(); ++k) choose(k, 0);
         return rc;
     }
     for (size_t k = 0; k < cls.size(); ++k) {
@@ -216,8 +234,15 @@ extern "C" shg_status shg_autotune_batch(const shg_params* params, int32_t count
         std::memset(&r, 0, sizeof(r));
         r.precision = precision;
         r.n = cls[k].n;
-        r.cluster = cand[k][pick[k]]->cluster;
-        r.threads = cand[k][pick[k]]->threads;
+        // automatic: the batch's split where shg_set_schedule knows it, else the class's default
+        int all = 0;
+        const PlainVariant* v = cand[k][pick[k]];
+        r.automatic = v == nullptr;
+        if (!v) v = plain_batch_variant(params, count, cls[k].n, &all);
+        if (!v || !find_split(precision, cls[k].n, v->cluster, v->threads))
+            v = default_variant(precision, cls[k].n, 0, SHG_MARCH_AUTO);
+        r.cluster = v->cluster;
+        r.threads = v->threads;
         r.candidates = (int)cand[k].size();
         r.pt_steps_per_s = work / (t_best * 1e-3);
         r.default_pt_steps_per_s = work / (t_default * 1e-3);
@@ -237,7 +262,7 @@ extern "C" shg_status shg_set_schedule(int32_t precision, int32_t n, int32_t clu
     const int nc = plain_candidates(precision, n, cand, 16);
     for (int i = 0; i < nc; ++i)
         if (cand[i]->cluster == cluster && cand[i]->threads == threads) {
-            set_plain_choice(cand[i]);
+            set_plain_choice(cand[i], 0);
             return SHG_OK;
         }
     return fail(SHG_ERR_UNSUPPORTED, "no compiled variant of grid side %d at precision %d with %d-CTA clusters x %d threads",

@@ -55,13 +55,6 @@ cudaError_t fork_streams(int dev, ForkStreams** out) {
 
 constexpr int kFewLevels = 5;  // at most so many variants for few runs per class
 
-// The level-th variant for few plain runs of variant v's class (few_runs_variant); null past the
-// last and where the caller or a tuner chose the march.
-const PlainVariant* few_choice(const shg_params& p, const PlainVariant* v, int level, int* upto) {
-    if (p.march != SHG_MARCH_AUTO || has_plain_choice(v->precision, v->n, 0)) return nullptr;
-    return few_runs_variant(v->precision, v->n, level, upto);
-}
-
 // run_variant, or where a march's workspace cannot be had the fused march, which needs none and gives
 // the same bits, on the sides it is built for.
 cudaError_t run_plain(const PlainVariant* v, const InstDesc* dev_descs, const InstDesc* host_descs, int count, int* queue,
@@ -87,8 +80,10 @@ shg_status plain_solve_device(const shg_params& p, const void* signal_in, void* 
     int out32 = 0;
     const PlainVariant* v = plain_variant_of(p, &out32);
     if (!v) return fail(SHG_ERR_UNSUPPORTED, "no kernel for grid side %d", p.nx);
-    int upto = 0;
-    if (const PlainVariant* w = few_choice(p, v, 0, &upto)) v = w;
+    if (p.march == SHG_MARCH_AUTO && !plain_choice_rules(v->precision, v->n, 1)) {
+        int upto = 0;
+        if (const PlainVariant* w = few_runs_variant(v->precision, v->n, 0, &upto)) v = w;
+    }
     InstDesc d = make_plain_desc(p, p.temp, p.temp);
     d.out32 = out32;
     d.signal_in = signal_in;
@@ -160,46 +155,83 @@ struct BatchLayout {
     std::vector<Group> groups;
 };
 
-static BatchLayout batch_layout(const shg_params* params, int count, void* const* pump_out, void* const* signal_out,
-                                double* power_slots) {
-    struct Item { const PlainVariant* v; int idx; double cost; int out32; };
-    std::vector<Item> items(count);
+struct BatchItem {
+    const PlainVariant* v;
+    int idx;
+    double cost;
+    int out32;
+};
+
+// The instances of a batch and the variant that each takes.
+static std::vector<BatchItem> batch_items(const shg_params* params, int count) {
+    // the classes of the batch, by the variant they have to themselves: `automatic` where neither the
+    // caller nor a tuner chose the march
+    struct Class {
+        const PlainVariant* v;
+        bool automatic;
+        int runs;
+        const PlainVariant* take;
+    };
+    std::vector<Class> cls;
+    std::vector<BatchItem> items(count);
+    std::vector<int> of(count);
     for (int i = 0; i < count; ++i) {
         int out32 = 0;
         const PlainVariant* v = plain_variant_of(params[i], &out32);
         items[i] = {v, i, (double)params[i].nx * params[i].nx * shg_steps(&params[i]), out32};
+        const bool automatic = params[i].march == SHG_MARCH_AUTO;
+        size_t c = 0;
+        while (c < cls.size() && (cls[c].v != v || cls[c].automatic != automatic)) ++c;
+        if (c == cls.size()) cls.push_back({v, automatic, 0, v});
+        ++cls[c].runs;
+        of[i] = (int)c;
     }
+    for (Class& c : cls) c.automatic = c.automatic && !plain_choice_rules(c.v->precision, c.v->n, c.runs);
     // A small batch takes the variants for few runs, each class from its widest on until the batch
     // fits: the classes share the device, so the parts of it that they fill must add up to at most one.
     bool fits = false;
     for (int level = 0; level < kFewLevels && !fits; ++level) {
-        std::vector<const PlainVariant*> few;
         double share = 0.0;
-        for (int i = 0; i < count && share < 1.0 + 1e-9; ++i) {
-            const PlainVariant* w = nullptr;
+        for (Class& c : cls) {
             int upto = 0;
-            for (int l = level; l >= 0 && !w; --l) w = few_choice(params[i], items[i].v, l, &upto);  // its last, if fewer
-            if (!w) break;
-            few.push_back(w);
-            share += 1.0 / upto;
+            c.take = nullptr;
+            for (int l = level; c.automatic && l >= 0 && !c.take; --l)  // its last, if fewer
+                c.take = few_runs_variant(c.v->precision, c.v->n, l, &upto);
+            share += c.take ? (double)c.runs / upto : 2.0;
         }
-        if ((int)few.size() < count || share >= 1.0 + 1e-9) continue;
-        for (int i = 0; i < count; ++i) items[i].v = few[i];
-        fits = true;
+        fits = share < 1.0 + 1e-9;
     }
     if (!fits) {
-        auto small = [&](int i) { return items[i].v->precision == 32 && items[i].v->n == 64 && params[i].march == SHG_MARCH_AUTO; };
-        int runs64 = 0, to_128 = 0, above = 0;
-        for (int i = 0; i < count; ++i) {
-            runs64 += small(i);
-            to_128 += items[i].v->n > 64 && items[i].v->n <= 128;
-            above += items[i].v->n > 128;
+        Class* small = nullptr;
+        int to_128 = 0, above = 0;
+        for (Class& c : cls) {
+            c.take = c.v;
+            if (c.automatic && c.v->precision == 32 && c.v->n == 64) small = &c;
+            to_128 += c.v->n > 64 && c.v->n <= 128 ? c.runs : 0;
+            above += c.v->n > 128 ? c.runs : 0;
         }
-        const PlainVariant* w = has_plain_choice(32, 64, 0) ? nullptr : many_small_variant(runs64, to_128, above);
-        for (int i = 0; i < count && w; ++i)
-            if (small(i)) items[i].v = w;
+        if (small && small->v == default_variant(32, 64, 0, SHG_MARCH_AUTO))
+            if (const PlainVariant* w = many_small_variant(small->runs, to_128, above)) small->take = w;
     }
-    std::stable_sort(items.begin(), items.end(), [](const Item& a, const Item& b) {
+    for (int i = 0; i < count; ++i) items[i].v = cls[of[i]].take;
+    return items;
+}
+
+const PlainVariant* plain_batch_variant(const shg_params* params, int count, int n, int* runs) {
+    const PlainVariant* v = nullptr;
+    *runs = 0;
+    for (const BatchItem& it : batch_items(params, count))
+        if (params[it.idx].nx == n && !it.out32) {
+            v = it.v;
+            ++*runs;
+        }
+    return v;
+}
+
+static BatchLayout batch_layout(const shg_params* params, int count, void* const* pump_out, void* const* signal_out,
+                                double* power_slots) {
+    std::vector<BatchItem> items = batch_items(params, count);
+    std::stable_sort(items.begin(), items.end(), [](const BatchItem& a, const BatchItem& b) {
         if (a.v != b.v) return a.v < b.v;
         return a.cost > b.cost;
     });

@@ -66,6 +66,10 @@ shg_status plain_solve_device(const shg_params& p, const void* signal_in, void* 
                               void* slices_s = nullptr, const double* poling_dev = nullptr);
 // pump_host / signal_host (optional, indexed like params): host arrays the outputs are copied
 // to, each group's right after its march on the stream that ran it.
+struct PlainVariant;
+// The variant that the runs of side n in a batch take (null if there are none), and how many they are;
+// runs that an FP32 batch's guard promotes to FP64 aside.
+const PlainVariant* plain_batch_variant(const shg_params* params, int count, int n, int* runs);
 shg_status plain_solve_batch(const shg_params* params, int count, void* const* pump_out, void* const* signal_out,
                              double* sh_power_out, cudaStream_t stream, void* const* pump_host = nullptr,
                              void* const* signal_host = nullptr);

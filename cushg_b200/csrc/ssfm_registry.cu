@@ -11,7 +11,13 @@ namespace shg {
 namespace {
 
 std::mutex g_mu;
-std::vector<const PlainVariant*> g_chosen;  // tuned variants, one per (precision, n, thermal)
+// Chosen plain variants, one per (precision, n); from: the number of runs from which the choice
+// also holds against the variants for few runs.
+struct Choice {
+    const PlainVariant* v;
+    int from;
+};
+std::vector<Choice> g_chosen;
 
 // f(variant) until it returns true; with `few` also the variants kept for few runs
 template <typename F>
@@ -100,12 +106,16 @@ const PlainVariant* many_small_variant(int runs64, int runs_to_128, int runs_abo
 }
 
 const PlainVariant* find_plain_variant(int precision, int n, int thermal, int march) {
-    const int th = thermal ? 1 : 0;
-    if (march == SHG_MARCH_AUTO) {
+    if (march == SHG_MARCH_AUTO && !thermal) {
         std::lock_guard<std::mutex> lk(g_mu);
-        for (const PlainVariant* v : g_chosen)
-            if (v->precision == precision && v->n == n && v->thermal == th) return v;
+        for (const Choice& c : g_chosen)
+            if (c.v->precision == precision && c.v->n == n) return c.v;
     }
+    return default_variant(precision, n, thermal, march);
+}
+
+const PlainVariant* default_variant(int precision, int n, int thermal, int march) {
+    const int th = thermal ? 1 : 0;
     const PlainVariant *fused = nullptr, *multi = nullptr;
     for_each_variant([&](const PlainVariant* v) {
         if (v->precision == precision && v->n == n && v->thermal == th) {
@@ -126,10 +136,10 @@ const PlainVariant* find_plain_variant(int precision, int n, int thermal, int ma
     return fused ? fused : multi;
 }
 
-bool has_plain_choice(int precision, int n, int thermal) {
+bool plain_choice_rules(int precision, int n, int runs) {
     std::lock_guard<std::mutex> lk(g_mu);
-    for (const PlainVariant* v : g_chosen)
-        if (v->precision == precision && v->n == n && v->thermal == (thermal ? 1 : 0)) return true;
+    for (const Choice& c : g_chosen)
+        if (c.v->precision == precision && c.v->n == n) return runs >= c.from;
     return false;
 }
 
@@ -147,14 +157,23 @@ void clear_plain_choices() {
     g_chosen.clear();
 }
 
-void set_plain_choice(const PlainVariant* v) {
+void clear_plain_choice(int precision, int n) {
     std::lock_guard<std::mutex> lk(g_mu);
-    for (const PlainVariant*& c : g_chosen)
-        if (c->precision == v->precision && c->n == v->n && c->thermal == v->thermal) {
-            c = v;
+    for (size_t i = 0; i < g_chosen.size(); ++i)
+        if (g_chosen[i].v->precision == precision && g_chosen[i].v->n == n) {
+            g_chosen.erase(g_chosen.begin() + i);
             return;
         }
-    g_chosen.push_back(v);
+}
+
+void set_plain_choice(const PlainVariant* v, int from) {
+    std::lock_guard<std::mutex> lk(g_mu);
+    for (Choice& c : g_chosen)
+        if (c.v->precision == v->precision && c.v->n == v->n) {
+            c = {v, from};
+            return;
+        }
+    g_chosen.push_back({v, from});
 }
 
 }  // namespace shg

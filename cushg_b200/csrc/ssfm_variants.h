@@ -62,9 +62,9 @@ VariantTable variants_split64();
 VariantTable variants_wide();
 
 // The variant the drivers use for (precision, n, thermal) under march preference `march`
-// (SHG_MARCH_*): automatic = the tuned one if shg_autotune chose one, else the default
-// (the first compiled fused variant, else the multi-pass one); fused / multi-pass = the
-// default of that kind.  Null if none is built.
+// (SHG_MARCH_*) where the number of runs does not say otherwise: automatic = the one a tuner or
+// shg_set_schedule chose, else the default (ssfm_registry.cu: the first compiled fused variant, or the
+// multi-pass one); fused / multi-pass = the default of that kind.  Null if none is built.
 const PlainVariant* find_plain_variant(int precision, int n, int thermal = 0, int march = 0);
 // The wide march (ssfm_wide.cuh) of thermal passes of (precision, n) if it is the faster one for
 // `count` runs that have the device to themselves, else null.
@@ -75,13 +75,21 @@ const PlainVariant* few_runs_variant(int precision, int n, int level, int* upto)
 // The variant of the 64 x 64 FP32 runs of a larger batch that holds `runs64` of them, `runs_to_128` runs of
 // the sides above 64 up to 128 and `runs_above` of larger ones; null: the default.
 const PlainVariant* many_small_variant(int runs64, int runs_to_128, int runs_above);
-// Whether a tuner or shg_set_schedule chose a variant for (precision, n, thermal).
-bool has_plain_choice(int precision, int n, int thermal);
-// Every compiled plain variant of (precision, n), default first; returns how many.
+// find_plain_variant without the choices below.
+const PlainVariant* default_variant(int precision, int n, int thermal, int march);
+// Every compiled plain variant of (precision, n) but those for few runs; returns how many.
 int plain_candidates(int precision, int n, const PlainVariant** out, int max);
-// Make v the variant find_plain_variant returns for its (precision, n, thermal).
-void set_plain_choice(const PlainVariant* v);
-// forget every tuned choice: later runs use the compiled defaults
+// The one of them with this split; null if there is none.
+const PlainVariant* find_split(int precision, int n, int cluster, int threads);
+// Make v the variant find_plain_variant returns for its plain (precision, n).  Against the variants for
+// few runs it holds in calls with at least `from` runs of the class: 0 where a caller pins it, the
+// number of runs it was measured with where a tuner chose it, so that tuning a large batch leaves
+// the single runs of its classes as they were.
+void set_plain_choice(const PlainVariant* v, int from);
+// Whether such a choice rules a call with `runs` runs of the class.
+bool plain_choice_rules(int precision, int n, int runs);
+void clear_plain_choice(int precision, int n);
+// forget every choice: later runs use the compiled defaults
 void clear_plain_choices();
 
 }  // namespace shg

@@ -44,7 +44,7 @@ class ShgThermalGradResult(ctypes.Structure):
 class ShgTuneResult(ctypes.Structure):
     """``shg_tune_result`` of include/shg.h."""
     _fields_ = [("precision", ctypes.c_int32), ("n", ctypes.c_int32), ("cluster", ctypes.c_int32),
-                ("threads", ctypes.c_int32), ("candidates", ctypes.c_int32), ("reserved", ctypes.c_int32),
+                ("threads", ctypes.c_int32), ("candidates", ctypes.c_int32), ("automatic", ctypes.c_int32),
                 ("pt_steps_per_s", ctypes.c_double), ("default_pt_steps_per_s", ctypes.c_double)]
 
 
@@ -489,7 +489,7 @@ def autotune(precision: int, n: int) -> dict:
     r = ShgTuneResult()
     _check(lib().shg_autotune(int(precision), int(n), ctypes.byref(r)))
     return {"precision": r.precision, "n": r.n, "cluster": r.cluster, "threads": r.threads,
-            "candidates": r.candidates, "pt_steps_per_s": r.pt_steps_per_s,
+            "candidates": r.candidates, "automatic": bool(r.automatic), "pt_steps_per_s": r.pt_steps_per_s,
             "default_pt_steps_per_s": r.default_pt_steps_per_s}
 
 
@@ -522,5 +522,5 @@ def autotune_batch(ps: list[ShgParams]) -> list[dict]:
     k = ctypes.c_int32(0)
     _check(lib().shg_autotune_batch(arr, n, out, 16, ctypes.byref(k)))
     return [{"precision": r.precision, "n": r.n, "cluster": r.cluster, "threads": r.threads,
-             "candidates": r.candidates, "pt_steps_per_s": r.pt_steps_per_s,
+             "candidates": r.candidates, "automatic": bool(r.automatic), "pt_steps_per_s": r.pt_steps_per_s,
              "default_pt_steps_per_s": r.default_pt_steps_per_s} for r in out[:k.value]]

@@ -282,20 +282,21 @@ SHG_API void shg_batch_plan_destroy(shg_batch_plan* plan);
 /* Result of shg_autotune. */
 typedef struct shg_tune_result {
     int32_t precision, n;       /* the grid-size class tuned */
-    int32_t cluster, threads;   /* the chosen split: CTAs per instance, threads per CTA */
+    int32_t cluster, threads;   /* the chosen split: CTAs per instance (0: multi-pass), threads per CTA */
     int32_t candidates;         /* compiled variants timed */
-    int32_t reserved;
+    int32_t automatic;          /* 1: the automatic choice was the fastest and stays; nothing to set later */
     double pt_steps_per_s;      /* the chosen variant's rate on the tuning batch */
-    double default_pt_steps_per_s; /* the default variant's rate on the same batch */
+    double default_pt_steps_per_s; /* the automatic choice's rate on the same batch */
 } shg_tune_result;
 
 /*
- * Autotuner of the fused march's schedule for one (precision, grid side) class: times every
- * compiled variant of the class (cluster split and threads per CTA of the row / column FFT
- * passes) on a synthetic batch that fills the device several times over, and makes the
- * fastest the variant every later plain run and batch of that class uses in this process
- * (results are the same to the last bit of the fields; SH powers may differ in the last
- * bits, the cluster reduction order being the split's).  Synchronous; call it before any
+ * Autotuner of the schedule for one (precision, grid side) class: times every compiled variant
+ * of the class (cluster split and threads per CTA of the row / column FFT passes, the multi-pass
+ * march) on a synthetic batch that fills the device several times over, and makes the fastest
+ * the variant that later plain batches of that class use in this process, if it is not the
+ * automatic choice anyway.  Single runs and small batches, which have variants of their own, keep
+ * those: a choice rules calls with at least as many runs of the class as it was timed with, and
+ * smaller ones only where there is no such variant.  Results are the same bits.  Synchronous; call it before any
  * stream capture.  No counterpart in the reference (compile-time launch shapes,
  * src/cuSHG.cu:22-23).
  */
@@ -304,11 +305,10 @@ SHG_API shg_status shg_autotune(int32_t precision, int32_t n, shg_tune_result* o
 /*
  * Autotuner for a given mixed batch (shg_solve_batch_device arguments, all march ==
  * SHG_MARCH_AUTO): the classes of a batch run side by side and share the SMs, so the split
- * that is fastest for a class alone can slow the batch.  Starting from the compiled
- * defaults, each class (largest total work first) tries its other compiled variants with the
+ * that is fastest for a class alone can slow the batch.  Starting from the automatic
+ * choices, each class (largest total work first) tries its other compiled variants with the
  * rest fixed, and keeps one that makes the whole batch at least 1 % faster on this device.
- * The choices hold for every later plain run and batch in this process, as for
- * shg_autotune.  out[0 .. *n_out-1]: one entry per class, largest work first, with
+ * The choices hold for later plain batches in this process, as for shg_autotune.  out[0 .. *n_out-1]: one entry per class, largest work first, with
  * pt_steps_per_s the batch's rate with the chosen schedule and default_pt_steps_per_s its
  * rate with the defaults.  Synchronous (runs the batch 4 times per trial); call it before
  * any stream capture.  No counterpart in the reference.
@@ -336,8 +336,8 @@ SHG_API shg_status shg_release_device_memory(int64_t keep_bytes);
 SHG_API void shg_autotune_reset(void);
 
 /* Choose a class's compiled variant by its split (the cluster and threads fields of a
- * shg_tune_result), without timing: e.g. to reuse a schedule that shg_autotune_batch found in
- * an earlier process.  SHG_ERR_UNSUPPORTED if no such variant is compiled.  No counterpart in
+ * shg_tune_result), without timing, for every later run and batch of the class whatever its size:
+ * e.g. to reuse a schedule that shg_autotune_batch found in an earlier process.  SHG_ERR_UNSUPPORTED if no such variant is compiled.  No counterpart in
  * the reference. */
 SHG_API shg_status shg_set_schedule(int32_t precision, int32_t n, int32_t cluster, int32_t threads);
 

@@ -56,3 +56,48 @@ def test_many_small_runs_beside_others():
     for others in [((96, 8),), ((128, 4),), ((96, 2), (128, 2)), ((256, 2),), ((192, 1),)]:
         assert "plain<float, 64, 1, 512>" in marches(batch((64, 160), *others)), others
     assert marches(batch((64, 140))) == {"plain<float, 64, 1, 512>"}
+
+
+@pytest.fixture
+def no_choices():
+    shg.autotune_reset()
+    yield
+    shg.autotune_reset()
+
+
+def test_the_class_tuner_starts_from_the_automatic_choice(no_choices):
+    """256 x 256 batches are automatically on the multi-pass march, 1.4 times as fast as the fused
+    splits on a full device: the tuner's reference rate is that march's, and it stays automatic."""
+    r = shg.autotune(32, 256)
+    assert r["automatic"] and r["cluster"] == 0
+    assert r["pt_steps_per_s"] == r["default_pt_steps_per_s"]
+    assert marches(batch((256, 60))) == {"multipass<float, 256>"}
+
+
+def test_tuning_a_sweep_leaves_single_runs_alone(no_choices):
+    """Whatever the tuners choose for large batches, single runs and small batches of the classes keep
+    the variants they have of their own."""
+    ps = [run(n, nz=30) for n in (64, 128, 192, 256) for _ in range(24)]
+    res = shg.autotune_batch(ps)
+    assert sorted(r["n"] for r in res) == [64, 128, 192, 256]
+    shg.autotune(32, 128)
+    assert marches(lambda: shg.solve(run(128))) == {"wide<float, 128>"}
+    assert marches(lambda: shg.solve(run(64))) == {"plain<float, 64, 16, 128>"}
+    assert marches(batch((128, 5))) == {"plain<float, 128, 16, 256>"}
+    for r in res:  # and each result can be set again
+        if not r["automatic"]:
+            shg.set_schedule(r["precision"], r["n"], r["cluster"], r["threads"])
+
+
+def test_tuning_a_small_batch_keeps_the_faster_march(no_choices):
+    """Two 128 x 128 FP32 runs take 6.5 us per step on the wide march and 30 on the fused one."""
+    ps = [run(128, nz=60), run(128, nz=60)]
+    r = shg.autotune_batch(ps)[0]
+    assert r["automatic"] and r["pt_steps_per_s"] == r["default_pt_steps_per_s"]
+    assert marches(lambda: shg.solve_batch_device(ps)) == {"wide<float, 128>"}
+
+
+def test_a_pinned_schedule_holds_for_single_runs_too(no_choices):
+    shg.set_schedule(32, 128, 2, 256)
+    assert marches(lambda: shg.solve(run(128))) == {"plain<float, 128, 2, 256>"}
+    assert marches(batch((128, 5))) == {"plain<float, 128, 2, 256>"}

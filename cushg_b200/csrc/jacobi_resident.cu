@@ -30,6 +30,7 @@
 #include "dft.cuh"
 #include "grid_barrier.cuh"
 #include "jacobi_point.cuh"
+#include "jacobi_tiles.h"
 #include "shg_host.h"
 #include "thermal.h"
 
@@ -45,7 +46,6 @@ constexpr int kResThreads = 256;
 // Planes that share a barrier, and planes of Q and of the face rows in flight.  1 / 3 / 4 / 6
 // measured 13.7 / 8.3 / 8.5 / 9.5 us a sweep at 128 x 128 x 200 FP64.
 constexpr int AH = 3;
-constexpr size_t kResSmem = 208 * 1024;  // of the tile: 26 planes of 1024 FP64 voxels, 52 of FP32
 
 // A condition known at compile time, passed like a run-time one.
 template <bool B>
@@ -298,27 +298,27 @@ __global__ void __launch_bounds__(kResThreads, 1)
     }
 }
 
-// Tiles of a grid: rows of TY = 1024 / n (side a power of two, 32 to 256, so that 256 threads of
-// 2 x 2 voxels cover a tile's plane) by enough planes for one CTA per SM.
-template <typename R>
-bool resident_tiles(int n, int nz, int sms, ResidentArgs* ra, int* ztiles) {
-    if (n != 32 && n != 64 && n != 128 && n != 256) return false;
-    const int ty = 1024 / n;
-    ra->ytiles = n / ty;
-    const int zt = std::max(1, std::min(nz, sms / ra->ytiles));
-    ra->tz = (nz + zt - 1) / zt;
-    *ztiles = (nz + ra->tz - 1) / ra->tz;
-    return sizeof(R) * 1024 * (size_t)ra->tz <= kResSmem;
+// The kernel's attribute, once per device, and the CTAs that a cooperative launch of it may have there.
+template <typename R, int BOUND, int N, bool HASQ>
+cudaError_t resident_ctas(int* ctas) {
+    auto kern = jacobi_resident_kernel<R, BOUND, N, HASQ>;
+    constexpr size_t smem = kResSmem + 2 * sizeof(R) * N;
+    static PerDevice<int> state;
+    return state.get(
+        [&](int dev, int& v) {
+            int sms = 0, per_sm = 0;
+            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+            if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kResThreads, smem);
+            v = sms * per_sm;
+            return e;
+        },
+        ctas);
 }
 
 template <typename R, int BOUND, int N, bool HASQ>
-cudaError_t launch_source(R* Ta, R* Tb, const R* Q, const JacobiCoef<R>& k, const ResidentArgs& ra, int ctas, cudaStream_t s) {
+cudaError_t launch_tiles(R* Ta, R* Tb, const R* Q, const JacobiCoef<R>& k, const ResidentArgs& ra, int ctas, cudaStream_t s) {
     auto kern = jacobi_resident_kernel<R, BOUND, N, HASQ>;
-    static PerDevice<int> attr;
-    cudaError_t e = attr.get([&](int, int&) {
-        return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kResSmem + 2 * sizeof(R) * N));
-    });
-    if (e != cudaSuccess) return e;
     R *ta = Ta, *tb = Tb;
     const R* q = Q;
     JacobiCoef<R> kk = k;
@@ -328,21 +328,26 @@ cudaError_t launch_source(R* Ta, R* Tb, const R* Q, const JacobiCoef<R>& k, cons
                                        sizeof(R) * (1024 * (size_t)ra.tz + 2 * N), s);
 }
 
-template <typename R, int BOUND, int N>
-cudaError_t launch_side(R* Ta, R* Tb, const R* Q, const JacobiCoef<R>& k, const ResidentArgs& ra, int ctas, cudaStream_t s) {
-    return Q ? launch_source<R, BOUND, N, true>(Ta, Tb, Q, k, ra, ctas, s)
-             : launch_source<R, BOUND, N, false>(Ta, Tb, Q, k, ra, ctas, s);
+// f's instantiation for a grid side, boundary and source
+template <typename R, int BOUND, int N, typename F>
+cudaError_t with_source(bool q, F&& f) {
+    return q ? f(&resident_ctas<R, BOUND, N, true>, &launch_tiles<R, BOUND, N, true>)
+             : f(&resident_ctas<R, BOUND, N, false>, &launch_tiles<R, BOUND, N, false>);
 }
-
-template <typename R, int BOUND>
-cudaError_t launch_any(R* Ta, R* Tb, const R* Q, const JacobiCoef<R>& k, const ResidentArgs& ra, int ctas, cudaStream_t s) {
-    switch (k.n) {
-        case 32: return launch_side<R, BOUND, 32>(Ta, Tb, Q, k, ra, ctas, s);
-        case 64: return launch_side<R, BOUND, 64>(Ta, Tb, Q, k, ra, ctas, s);
-        case 128: return launch_side<R, BOUND, 128>(Ta, Tb, Q, k, ra, ctas, s);
-        case 256: return launch_side<R, BOUND, 256>(Ta, Tb, Q, k, ra, ctas, s);
+template <typename R, int BOUND, typename F>
+cudaError_t with_side(int n, bool q, F&& f) {
+    switch (n) {
+        case 32: return with_source<R, BOUND, 32>(q, f);
+        case 64: return with_source<R, BOUND, 64>(q, f);
+        case 128: return with_source<R, BOUND, 128>(q, f);
+        case 256: return with_source<R, BOUND, 256>(q, f);
     }
     return cudaErrorInvalidValue;
+}
+template <typename R, typename F>
+cudaError_t with_kernel(int boundary, int n, bool q, F&& f) {
+    return boundary == SHG_BOUNDARY_OVEN_SURROUNDED ? with_side<R, SHG_BOUNDARY_OVEN_SURROUNDED>(n, q, f)
+                                                    : with_side<R, SHG_BOUNDARY_TOP_OPEN>(n, q, f);
 }
 
 int sm_count() {
@@ -356,34 +361,42 @@ int sm_count() {
 }  // namespace
 
 template <typename R>
-bool jacobi_resident_fits(const JacobiCoef<R>& k) {
-    ResidentArgs ra;
-    int zt = 0;
-    return resident_tiles<R>(k.n, k.nz, sm_count(), &ra, &zt);
+bool jacobi_resident_fits(const JacobiCoef<R>& k, int boundary, bool source) {
+    int ctas = 0;
+    const cudaError_t e = with_kernel<R>(boundary, k.n, source, [&](auto fit, auto) { return fit(&ctas); });
+    if (e != cudaSuccess) {
+        cudaGetLastError();  // the one-sweep kernels can
+        return false;
+    }
+    ResidentTiles t;
+    return resident_tiles(sizeof(R), k.n, k.nz, sm_count(), ctas, &t);
 }
 
 template <typename R>
 cudaError_t launch_jacobi_resident(R* Ta, R* Tb, const R* Q, const JacobiCoef<R>& k, int boundary, int count, unsigned* bar,
                                    unsigned* err, cudaStream_t s) {
-    ResidentArgs ra;
-    int zt = 0;
-    if (!resident_tiles<R>(k.n, k.nz, sm_count(), &ra, &zt)) return cudaErrorInvalidValue;
-    ra.count = count;
-    ra.bar = bar;
-    ra.err = err;
-    const BarrierLimit bl = barrier_limit();
-    ra.limit_ns = bl.ns;
-    ra.withheld = bl.withheld;
-    const cudaError_t e = cudaMemsetAsync(bar, 0, sizeof(unsigned), s);
-    if (e != cudaSuccess) return e;
-    const int ctas = ra.ytiles * zt;
-    return boundary == SHG_BOUNDARY_OVEN_SURROUNDED
-               ? launch_any<R, SHG_BOUNDARY_OVEN_SURROUNDED>(Ta, Tb, Q, k, ra, ctas, s)
-               : launch_any<R, SHG_BOUNDARY_TOP_OPEN>(Ta, Tb, Q, k, ra, ctas, s);
+    return with_kernel<R>(boundary, k.n, Q != nullptr, [&](auto fit, auto launch) {
+        int ctas = 0;
+        cudaError_t e = fit(&ctas);
+        if (e != cudaSuccess) return e;
+        ResidentTiles t;
+        if (!resident_tiles(sizeof(R), k.n, k.nz, sm_count(), ctas, &t)) return cudaErrorInvalidValue;
+        ResidentArgs ra;
+        ra.count = count;
+        ra.ytiles = t.ytiles;
+        ra.tz = t.tz;
+        ra.bar = bar;
+        ra.err = err;
+        const BarrierLimit bl = barrier_limit();
+        ra.limit_ns = bl.ns;
+        ra.withheld = bl.withheld;
+        if ((e = cudaMemsetAsync(bar, 0, sizeof(unsigned), s)) != cudaSuccess) return e;
+        return launch(Ta, Tb, Q, k, ra, t.ytiles * t.ztiles, s);
+    });
 }
 
-template bool jacobi_resident_fits<float>(const JacobiCoef<float>&);
-template bool jacobi_resident_fits<double>(const JacobiCoef<double>&);
+template bool jacobi_resident_fits<float>(const JacobiCoef<float>&, int, bool);
+template bool jacobi_resident_fits<double>(const JacobiCoef<double>&, int, bool);
 template cudaError_t launch_jacobi_resident<float>(float*, float*, const float*, const JacobiCoef<float>&, int, int, unsigned*,
                                                    unsigned*, cudaStream_t);
 template cudaError_t launch_jacobi_resident<double>(double*, double*, const double*, const JacobiCoef<double>&, int, int,

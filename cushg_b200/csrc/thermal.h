@@ -43,7 +43,7 @@ size_t jacobi_partials(const shg_params& p);
 // for grids that fit: from Ta, which with Tb holds the faces between tiles meanwhile, into Ta
 // (count even) or Tb (odd).  Arrays 2-real aligned; bar: a scratch word; *err is set to 1 if a
 // barrier wait ran out.
-template <typename R> bool jacobi_resident_fits(const JacobiCoef<R>& k);
+template <typename R> bool jacobi_resident_fits(const JacobiCoef<R>& k, int boundary, bool source);
 template <typename R>
 cudaError_t launch_jacobi_resident(R* Ta, R* Tb, const R* Q, const JacobiCoef<R>& k, int boundary, int count, unsigned* bar,
                                    unsigned* err, cudaStream_t s);

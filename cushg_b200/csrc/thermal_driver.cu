@@ -79,8 +79,8 @@ cudaError_t run_sweeps(R*& cur, R*& nxt, const R* Ta, const SweepMaps<R>& m, con
 // launch.
 constexpr int64_t kResidentMin = 8;
 template <typename R>
-bool resident(const shg_params& p, const JacobiCoef<R>& k, int64_t count) {
-    return p.jacobi_block == 0 && count >= kResidentMin && jacobi_resident_fits<R>(k);
+bool resident(const shg_params& p, const JacobiCoef<R>& k, const R* Q, int64_t count) {
+    return p.jacobi_block == 0 && count >= kResidentMin && jacobi_resident_fits<R>(k, p.boundary, Q != nullptr);
 }
 
 // `count` unchecked sweeps on the resident kernel; cur / nxt as run_sweeps leaves them.  err[1] is
@@ -140,7 +140,7 @@ constexpr int64_t kSweepGraphMin = 64;
 template <typename R>
 cudaError_t run_sweeps_graphed(ThermalInst<R>& t, int64_t count, cudaStream_t s) {
     const shg_params& p = *t.p;
-    if (resident<R>(p, t.k, count)) return run_resident<R>(t.cur, t.nxt, t.Q, t.k, p.boundary, count, t.tb_err, s);
+    if (resident<R>(p, t.k, t.Q, count)) return run_resident<R>(t.cur, t.nxt, t.Q, t.k, p.boundary, count, t.tb_err, s);
     if (t.depth > 1 || count < kSweepGraphMin)
         return run_sweeps<R>(t.cur, t.nxt, t.Ta, t.maps, t.Q, t.k, p.boundary, t.depth, count, t.tb_err, s);
     const int parity = t.cur == t.Ta ? 0 : 1;
@@ -544,7 +544,7 @@ shg_status heat_run(const shg_params& p, R* T, const R* Q, int64_t sweeps, cudaS
         SweepMaps<R> maps;
         if (depth > 1 && (rc = make_sweep_maps<R>(T, other, Q, n, nz, &maps)) != SHG_OK) break;
         const JacobiCoef<R> k = make_jacobi_coef<R>(p);
-        const bool res = resident<R>(p, k, sweeps);
+        const bool res = resident<R>(p, k, Q, sweeps);
         // both buffers start alike, so the voxels no sweep writes (Dirichlet faces) agree (the
         // resident kernel writes them too)
         if ((!res && (e = cudaMemcpyAsync(other, T, arr, cudaMemcpyDeviceToDevice, s)) != cudaSuccess) ||

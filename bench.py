@@ -37,13 +37,13 @@ from cushg_b200 import params as P  # noqa: E402
 
 B200_SMS = 148
 FP32_LANES_PER_SM = 128
-# DRAM bytes (read + write) per launch of the dominant kernel of the sweep, the 256 x 256 FP32
-# class (ssfm_plain_kernel<float, 256, 16, 256>), from one ncu launch-list capture of this
-# bench (`--steps 2 --warmup 3 --no-cpu-baseline --no-autotune --no-extras`, dram__bytes_read.sum
-# and dram__bytes_write.sum); the fields stay on chip, so this is descriptors and outputs
-SWEEP_256_DRAM_BYTES_PER_LAUNCH = 9.78e6
+# DRAM bytes (read + write) per march step of the sweep's dominant class, 256 x 256 FP32 on the
+# multi-pass march (one launch each of mp_row_kernel and mp_col_kernel over all its instances), from
+# an ncu capture of 14 steps (dram__bytes_read.sum 3.2 MB, dram__bytes_write.sum 116 MB, L2 kept
+# between launches): both planes of every instance are read from L2 and written back
+SWEEP_256_DRAM_BYTES_PER_STEP = 119e6
 # bytes of one instance descriptor the batch call uploads (shg::InstDesc)
-INST_DESC_BYTES = 376
+INST_DESC_BYTES = 384
 
 
 def flops_per_point_step(n: int) -> float:
@@ -53,6 +53,26 @@ def flops_per_point_step(n: int) -> float:
     192 flops each (4 evaluations of dA/dz at 35, 3 stage inputs at 8, the weighted sum
     at 20 and the update at 8)."""
     return 4 * 5 * math.log2(n * n) + 2 * 6 + 2 * 192
+
+
+def march_kernels(ps, multipass) -> int:
+    """Kernels that one batch of plain runs launches: one persistent launch per (precision the
+    instance runs in, grid side) class on the fused march; on the multi-pass march (the classes in
+    `multipass`), per round of 256 instances, the set-up, the first row pass, a column and a row pass
+    per step and the power sums."""
+    from cushg_b200 import shg
+    classes = {}
+    for p in ps:
+        promoted = p.fp32_guard > 0 and shg.fp32_error_estimate(p) > p.fp32_guard
+        classes.setdefault((64 if promoted else p.precision, p.nx), []).append(p.nz - 1)
+    n = 0
+    for key, steps in classes.items():
+        if key not in multipass:
+            n += 1
+            continue
+        steps.sort(reverse=True)
+        n += sum(3 + 2 * steps[i] for i in range(0, len(steps), 256))
+    return n
 
 
 def point_steps(ps) -> int:
@@ -171,7 +191,8 @@ def run_ours(args, rank: int, world: int, local_rank: int) -> dict | None:
         tuned.append({"n": args.class_side, "cluster": c, "threads": t, "candidates": 1, "gain": 1.0})
     elif not args.no_autotune:
         for r in shg.autotune_batch(ps):
-            tuned.append({"n": r["n"], "cluster": r["cluster"], "threads": r["threads"], "candidates": r["candidates"],
+            tuned.append({"n": r["n"], "cluster": r["cluster"], "threads": r["threads"],
+                          "candidates": r["candidates"], "automatic": r["automatic"],
                           "gain": r["pt_steps_per_s"] / r["default_pt_steps_per_s"]})
 
     def sweep():
@@ -248,6 +269,12 @@ def run_ours(args, rank: int, world: int, local_rank: int) -> dict | None:
     if rank != 0:
         return None
 
+    # the classes on the multi-pass march: automatically those from 256 x 256 on, in batches past the
+    # marches for a few runs (a schedule's cluster is 0 there); runs that the guard promotes stay fused
+    chosen = {t["n"]: t["cluster"] == 0 for t in tuned}
+    multipass = {(args.precision, n) for n in {p.nx for p in ps} if chosen.get(n, n >= 256)}
+    dom_mp = (args.precision, nmax) in multipass
+
     pts = point_steps(ps)
     value = total_pts / (ms * 1e-3)
     e2e_value = total_pts / (e2e_ms * 1e-3)
@@ -321,27 +348,30 @@ def run_ours(args, rank: int, world: int, local_rank: int) -> dict | None:
                         f"batched plain SSFM sweep, 256 instances (seed 0) split over {world} ranks",
             "instances": len(ps), "grid_sides": [64, 128, 192, 256], "nz_range": [100, 400],
             "point_steps_per_gpu": pts, "precision": args.precision,
-            "l2": "a 256 MB buffer is written between timed steps (L2 flushed); fields stay in shared memory",
+            "l2": "a 256 MB buffer is written between timed steps (L2 flushed); the fused classes' fields stay in "
+                  "shared memory, the multi-pass class's planes in global memory",
             "schedule": tuned or "compiled defaults",
         },
         "e2e": {"value": e2e_value, "unit": "grid-pt·steps/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                 "ms_per_step": e2e_ms},
-        # one persistent launch per (precision the instance runs in, grid side) group per step
-        "gpu_launches": args.steps * len({(64 if (p.fp32_guard > 0 and shg.fp32_error_estimate(p) > p.fp32_guard)
-                                           else p.precision, p.nx) for p in ps}),
+        "gpu_launches": args.steps * march_kernels(ps, multipass),
         "roofline": {"bound": "fp32-issue" if args.precision == 32 else "fp64-issue", "achieved": achieved_tflops,
                      "peak": peak, "unit": "TFLOP/s", "frac": achieved_tflops / peak,
-                     "traffic": SWEEP_256_DRAM_BYTES_PER_LAUNCH if (args.precision == 32 and not args.class_side) else None,
-                     "traffic_note": "DRAM bytes per launch of the 256x256 FP32 class, ncu capture of this bench",
+                     "traffic": SWEEP_256_DRAM_BYTES_PER_STEP if (dom_mp and args.precision == 32 and not args.class_side) else None,
+                     "traffic_note": "DRAM bytes per march step (two launches) of the 256x256 FP32 class on the multi-pass "
+                                     "march, ncu capture",
                      "peak_source": f"nominal {B200_SMS} SMs x {lanes} lanes x 2 flop x measured median SM clock {sm_mhz:.0f} MHz",
-                     "kernel": f"ssfm_plain_kernel, {nmax}x{nmax} class ({len(dom)} FP32 instances), one launch, "
-                               + next((f"{t['cluster']}-CTA clusters x {t['threads']} threads (tuned)"
+                     "kernel": f"mp_row_kernel + mp_col_kernel, {nmax}x{nmax} class ({len(dom)} FP32 instances), two launches per "
+                               f"step, planes in global memory" if dom_mp else
+                               f"ssfm_plain_kernel, {nmax}x{nmax} class ({len(dom)} FP32 instances), one launch, "
+                               + next((f"{t['cluster']}-CTA clusters x {t['threads']} threads "
+                                       + ("(automatic)" if t.get("automatic") else "(chosen)")
                                        for t in tuned if t["n"] == nmax), "compiled default split"),
                      "launch_ms": dom_ms, "flops_per_launch": algorithmic_flops(dom),
                      "sweep": {"achieved": sweep_tflops, "frac": sweep_tflops / peak, "flops": fl,
                                "note": "all four classes, concurrent on forked streams"},
                      "hbm": {"achieved": hbm_achieved, "peak": hbm_peak, "unit": "GB/s", "frac": hbm_achieved / hbm_peak,
-                             "note": "32 B/pt-step algorithmic (FP32) against measured copy bandwidth; the fields do not touch HBM between steps"}},
+                             "note": "32 B/pt-step algorithmic (FP32) against measured copy bandwidth; the fused classes' fields do not touch HBM between steps"}},
         "clocks": clocks,
     }
     if err is not None:

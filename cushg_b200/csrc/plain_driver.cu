@@ -2,10 +2,11 @@
 // instances with uneven grid sizes and step counts.
 //
 // The batch replaces the one-process-per-point sweep of src/cuSHG.sh:58-94.  Instances are
-// grouped by compiled variant (precision, grid side); each group is ONE persistent launch
-// of the fused march, as many clusters as fit on the device, fed by a device work queue
-// (an atomic counter over the group's descriptors, ordered longest march first, so the
-// clusters drain it like a longest-processing-time schedule).  Groups run concurrently on
+// grouped by compiled variant (precision, grid side).  On the fused march a group is ONE persistent
+// launch, as many clusters as fit on the device, fed by a device work queue (an atomic counter
+// over the group's descriptors, ordered longest march first, so the clusters drain it like a
+// longest-processing-time schedule); on the multi-pass march two launches per step over all its
+// runs, on the wide march (few runs) a cooperative launch per round of runs.  Groups run concurrently on
 // forked streams, the largest total work first, so the smaller classes fill the SMs the
 // largest one frees at its tail.  A batch plan (shg_batch_plan_*) captures the same
 // sequence once into a CUDA graph and replays it.

@@ -31,8 +31,9 @@ struct MpCfg {
     // is bound by the dependent chains of its per-voxel coefficients and RK4, so it takes small
     // CTAs of four threads a job, four to an SM (FP32: 128 registers): four 512 x 512 instances,
     // 8 rows x 4 threads 42 us, 2 x 4 36 us in FP32; 4 x 2 81 us, 2 x 4 63 us in FP64.  A plain
-    // pass is bound by the FMA pipe and runs a job on one thread (8 rows: 44 us for eight
-    // instances, 4 rows or two threads a job 44-45 us).
+    // pass is bound by the FMA pipe (58 % of the SMs' active cycles) and the wave its last CTAs leave
+    // half empty, and runs a job on one thread (8 rows: 44 us for eight instances, 4 rows or two
+    // threads a job 44-45 us).
     static constexpr int RB = THERM ? 2 : sizeof(T) == 4 ? 8 : 4;
     static constexpr int PX = THERM ? 4 : 1;
     static constexpr int JOBS = RB * 16, RNT = JOBS * PX;  // row-pass jobs and threads

@@ -4,7 +4,7 @@
 namespace shg {
 
 static const PlainVariant kTable[] = {
-    SHG_VARIANT(float, 32, 256, 16, 256, 2, false),  // default: 16-CTA clusters, 2 CTAs per SM
+    SHG_VARIANT(float, 32, 256, 16, 256, 2, false),  // the fused default: 16-CTA clusters, 2 CTAs per SM
     SHG_VARIANT(float, 32, 256, 8, 256, 1, false),
     SHG_VARIANT(float, 32, 256, 16, 512, 1, false),
 };

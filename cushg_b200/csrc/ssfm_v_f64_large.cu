@@ -4,7 +4,8 @@
 namespace shg {
 
 static const PlainVariant kTable[] = {
-    // the first of each side is its default: the split shg_autotune measured fastest on a
+    // the first of each side is its fused default (256: for runs that an FP32 batch's guard promotes;
+    // other batches take the multi-pass march): the split shg_autotune measured fastest on a
     // device-filling batch of the class (128: 19.5 against 18.3 G pt-steps/s; 192: 14.3
     // against 12.4 G)
     SHG_VARIANT(double, 64, 128, 8, 128, 2, false),

@@ -1,9 +1,9 @@
-// ssfm_variants.h — registry of the compiled variants of the fused SSFM march.
+// ssfm_variants.h — registry of the compiled variants of the SSFM marches.
 //
-// A variant fixes the precision, the grid side N, the cluster split C (CTAs per instance),
-// the threads per CTA and the CTAs per SM the register budget targets.  Each (precision, N)
-// has a default variant and possibly alternatives with another split; shg_autotune times
-// them and makes the fastest the one the drivers use.
+// A variant of the fused march fixes the precision, the grid side N, the cluster split C (CTAs per
+// instance), the threads per CTA and the CTAs per SM the register budget targets; the multi-pass and
+// wide marches have one variant each where they are built.  Each (precision, N) has a default
+// variant, variants for few runs, and possibly alternatives with another split, which the tuners time.
 #pragma once
 
 #include <cuda_runtime.h>

@@ -56,6 +56,7 @@ struct WideCfg {
     static constexpr bool STAGE = THERM && BASE_BYTES + STAGE_BYTES <= 227 * 1024;
     static constexpr size_t smem_bytes = BASE_BYTES + (STAGE ? STAGE_BYTES : 0);
     static_assert(N % 16 == 0 && G % 2 == 0 && NT % 32 == 0, "bad wide split");
+    static_assert(!PACK || R2 % 2 == 0, "packed points go in pairs");
 };
 
 // Workspace: barrier counters (zeroed before the launch), then per instance the two planes and
@@ -247,16 +248,6 @@ __global__ void __launch_bounds__(WideCfg<T, N, THERM>::NT, WideCfg<T, N, THERM>
                     Ps[o1] = make_float2(P.r.y, P.i.y);
                     Ss[o0] = make_float2(S.r.x, S.i.x);
                     Ss[o1] = make_float2(S.r.y, S.i.y);
-                }
-                if constexpr (R2 & 1) {  // the odd one out
-                    for (int j = tid; j < RT * 16; j += NT) {
-                        const int o = sidx<N, R2, SW>(j >> 4, (j & 15) + 16 * (R2 - 1));
-                        V p = Ps[o], q = Ss[o];
-                        rk4_point<T>(p, q, cf_prev, hap, has, qs, dz6);
-                        rk4_point<T>(p, q, cf_next, hap, has, qs, dz6);
-                        Ps[o] = p;
-                        Ss[o] = q;
-                    }
                 }
                 return;
             }

@@ -235,7 +235,8 @@ SHG_API shg_status shg_solve_device(const shg_params* p, const void* signal_in_d
 /*
  * Batched plain runs: `count` independent instances, each with its own parameter
  * set (grid size, nz, crystal, beam), in one persistent launch per grid-size class
- * fed by a device work queue.  Replaces the one-process-per-point sweep of
+ * fed by a device work queue (sides 256 and 512: two launches per step over all its runs; a few
+ * runs: marches of their own, see shg_params.march).  Replaces the one-process-per-point sweep of
  * src/cuSHG.sh:58-94.  All instances must share `precision` and have thermal == 0.
  * pump_out[i] / signal_out[i]: device buffers (nx_i*ny_i complex) or NULL entries.
  * sh_power_out: host array of `count` doubles or NULL.  NULL: the call is asynchronous and cannot
@@ -381,15 +382,17 @@ SHG_API shg_status shg_heat_sweeps_device(const shg_params* p, void* temperature
  * reference, whose Jacobi loop (Solver.h:339-355) approaches it one sweep at a time.
  * With the faces' coefficients of Tfield.h:93-240 scaled to a common form the sweep's linear
  * system is the sum of three one-dimensional operators (Robin, or next to a Dirichlet face,
- * at each end); the solve diagonalises the x and y operators (FP64 transforms cached per
- * device and operator) and solves a tridiagonal system along z for every (x, y) mode.
+ * at each end); the solve diagonalises the x operator and the cheaper of the y and z operators
+ * (FP64 transforms; those of x and y cached per device and operator) and solves a tridiagonal
+ * system along the third direction for every pair of modes.
  *   temperature_dev  nx*ny*nz reals: the Dirichlet voxels hold their values on entry and keep
  *                    them; every other voxel receives the solution (rounded to the precision).
  *   q_dev            nx*ny*nz reals: the heat source Q, or NULL for none.
  *   residual_out     optional: max |J(T) - T| of one FP64 Jacobi sweep applied to the FP64
  *                    solution (the sweep's own measure of how far T is from its fixed point).
  * Uses the grid, precision, kappa, h_conv, t_inf and boundary of *p.  Works in FP64 with two
- * workspace buffers of nx*ny*nz doubles from the stream's pool.  Stream-ordered on `stream`;
+ * workspace buffers of nx*ny*nz doubles (and nz*nz for the z modes where they are used) from the
+ * stream's pool.  Stream-ordered on `stream`;
  * synchronises once at the end.
  */
 SHG_API shg_status shg_heat_steady_device(const shg_params* p, void* temperature_dev, const void* q_dev,

@@ -83,7 +83,7 @@ shg_status plain_solve_device(const shg_params& p, const void* signal_in, void* 
     if (!v) return fail(SHG_ERR_UNSUPPORTED, "no kernel for grid side %d", p.nx);
     if (p.march == SHG_MARCH_AUTO && !plain_choice_rules(v->precision, v->n, 1)) {
         int upto = 0;
-        if (const PlainVariant* w = few_runs_variant(v->precision, v->n, 0, &upto)) v = w;
+        if (const PlainVariant* w = few_runs_variant(v->precision, v->n, 0, true, &upto)) v = w;
     }
     InstDesc d = make_plain_desc(p, p.temp, p.temp);
     d.out32 = out32;
@@ -197,7 +197,7 @@ static std::vector<BatchItem> batch_items(const shg_params* params, int count) {
             int upto = 0;
             c.take = nullptr;
             for (int l = level; c.automatic && l >= 0 && !c.take; --l)  // its last, if fewer
-                c.take = few_runs_variant(c.v->precision, c.v->n, l, &upto);
+                c.take = few_runs_variant(c.v->precision, c.v->n, l, cls.size() == 1, &upto);
             share += c.take ? (double)c.runs / upto : 2.0;
         }
         fits = share < 1.0 + 1e-9;

@@ -41,32 +41,35 @@ void for_each_variant(F&& f, bool few = false) {
 //   FP32 32: 1-28 3.4-4.8 / 5.3-5.8.  48: 1-14 3.9-4.9 / 11, 15-100 7.3-12.0 / 11-12.
 //   64: 1-14 4.1-5.0 / 14.1, 15-104 7.8-14.0 / 14.2-15.2.  96: 1-7 5.6-5.7 / 30.5, 8-48 10-19 /
 //   31, 49-72 24 / 31.  128: 1-2 6.3-6.7 / 29.8, 3-7 7.5 / 29.8, 8-48 12-27 / 30.5, 73-108 44 / 61.
-//   192: 1-9 7.2-23 / 37.6, 10-16 27 / 37.6, 37-56 58-61 / 74.  256: 1-4 8.4-18 / 24,
-//   5-6 21.5 / 24.
+//   192: 1-9 7.2-23 / 37.6, 10-15 26 / 37.4 (16: 39.8 / 37.4), 37-48 58-61 / 74 (51: 79.9 / 75).
+//   256: 1-4 8.4-18 / 24, 5-7 21-21.3 / 21-23.6 (8: 34 / 23.4).
 //   512: 1 14.4 / 29.2 (multi-pass)
 //   FP64 32: 1-28 3.5-5.5 / 6.8-7.1, 29-60 5.8-6.9 / 7.3.  48: 1-14 4.2-8.0 / 8.3, 101-148 17.5 /
 //   16-22.  64: 1-14 4.9-9.3 / 15, 15-48 9.9-14.7 / 15.5, 73-108 20.5 / 26.  96: 1-6 6.2-8.6 / 32.4,
 //   7-48 13-32 / 33.  128: 1-3 6.5-8.3 / 19.1, 4-7 11 / 19.1.  192: 1-6 8.5-21 / 25.8.
-//   256: 1-4 9.7-24 / 34.  512: 1 19.0 / 39.3 (multi-pass)
-struct FewRow { int precision, n, upto, cluster, threads; };
+//   256: 1-4 9.7-24 / 34, 5-7 33.7 / 33.6-36.6 (8: 66.8 / 37.6).  512: 1 19.0 / 39.3 (multi-pass)
+// `beside`: the runs that count as a full device in a batch with other classes, where that is not upto
+// (0: the row is for its class alone).
+struct FewRow { int precision, n, upto, cluster, threads, beside = -1; };
 const FewRow kFew[] = {
     {32, 32, 28, 16, 64},   {32, 48, 14, 16, 96},   {32, 48, 100, 4, 96},  {32, 64, 14, 16, 128},
     {32, 64, 104, 4, 128},  {32, 64, 148, 1, 512},  {32, 96, 7, 16, 288},
     {32, 96, 48, 8, 288},   {32, 96, 72, 2, 192},   {32, 128, 2, 0, 0},     {32, 128, 7, 16, 256}, {32, 128, 48, 8, 256},
-    {32, 128, 72, 2, 512},  {32, 128, 108, 4, 256}, {32, 192, 9, 0, 0},    {32, 192, 16, 8, 192},
-    {32, 192, 36, 4, 384},  {32, 192, 56, 8, 192},  {32, 256, 4, 0, 0},    {32, 256, 6, 16, 256},
+    {32, 128, 72, 2, 512},  {32, 128, 108, 4, 256}, {32, 192, 9, 0, 0},    {32, 192, 15, 8, 192, 16},
+    {32, 192, 36, 4, 384},  {32, 192, 48, 8, 192, 56},  {32, 256, 4, 0, 0},    {32, 256, 7, 16, 256, 6},
     {32, 512, 1, 0, 0},
     {64, 32, 28, 16, 64},   {64, 32, 60, 4, 128},   {64, 48, 14, 16, 160}, {64, 48, 100, 4, 96},
     {64, 48, 148, 1, 288},  {64, 64, 14, 16, 256},  {64, 64, 48, 4, 128},  {64, 64, 72, 2, 256},
     {64, 64, 108, 4, 128},  {64, 96, 6, 0, 0},      {64, 96, 48, 8, 288},  {64, 128, 3, 0, 0},
-    {64, 128, 7, 16, 512},  {64, 192, 6, 0, 0},     {64, 256, 4, 0, 0},    {64, 512, 1, 0, 0},
+    {64, 128, 7, 16, 512},  {64, 192, 6, 0, 0},     {64, 256, 4, 0, 0},
+    {64, 256, 7, 16, 256, 0},  {64, 512, 1, 0, 0},
 };
 
 }  // namespace
 
-const PlainVariant* few_runs_variant(int precision, int n, int level, int* upto) {
+const PlainVariant* few_runs_variant(int precision, int n, int level, bool alone, int* upto) {
     for (const FewRow& r : kFew) {
-        if (r.precision != precision || r.n != n || level-- > 0) continue;
+        if (r.precision != precision || r.n != n || (r.beside == 0 && !alone) || level-- > 0) continue;
         const PlainVariant* v = nullptr;
         for_each_variant([&](const PlainVariant* c) {
             if (c->precision == precision && c->n == n && !c->thermal && c->cluster == r.cluster &&
@@ -80,7 +83,7 @@ const PlainVariant* few_runs_variant(int precision, int n, int level, int* upto)
             level = 0;
             continue;
         }
-        *upto = r.upto;
+        *upto = alone || r.beside < 0 ? r.upto : r.beside;
         return v;
     }
     return nullptr;

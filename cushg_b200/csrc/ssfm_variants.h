@@ -70,8 +70,9 @@ const PlainVariant* find_plain_variant(int precision, int n, int thermal = 0, in
 // `count` runs that have the device to themselves, else null.
 const PlainVariant* wide_thermal_variant(int precision, int n, int count);
 // Plain runs of (precision, n): the level-th variant for few runs, from the widest on, and the
-// number of runs up to which it is the fastest of them; null past the last.
-const PlainVariant* few_runs_variant(int precision, int n, int level, int* upto);
+// number of runs up to which it is the fastest of them, with no other class (alone) or beside some;
+// null past the last.
+const PlainVariant* few_runs_variant(int precision, int n, int level, bool alone, int* upto);
 // The variant of the 64 x 64 FP32 runs of a larger batch that holds `runs64` of them, `runs_to_128` runs of
 // the sides above 64 up to 128 and `runs_above` of larger ones; null: the default.
 const PlainVariant* many_small_variant(int runs64, int runs_to_128, int runs_above);

@@ -203,16 +203,19 @@ static std::vector<BatchItem> batch_items(const shg_params* params, int count) {
         fits = share < 1.0 + 1e-9;
     }
     if (!fits) {
-        Class* small = nullptr;
-        int to_128 = 0, above = 0;
+        int small = -1, to_128 = 0, above = 0;
         for (Class& c : cls) {
             c.take = c.v;
-            if (c.automatic && c.v->precision == 32 && c.v->n == 64) small = &c;
+            if (c.automatic && c.v == default_variant(32, 64, 0, SHG_MARCH_AUTO)) small = (int)(&c - cls.data());
             to_128 += c.v->n > 64 && c.v->n <= 128 ? c.runs : 0;
             above += c.v->n > 128 ? c.runs : 0;
         }
-        if (small && small->v == default_variant(32, 64, 0, SHG_MARCH_AUTO))
-            if (const PlainVariant* w = many_small_variant(small->runs, to_128, above)) small->take = w;
+        if (small >= 0) {
+            std::vector<int> steps;
+            for (int i = 0; i < count; ++i)
+                if (of[i] == small) steps.push_back(shg_steps(&params[i]));
+            if (const PlainVariant* w = many_small_variant(std::move(steps), to_128, above)) cls[small].take = w;
+        }
     }
     for (int i = 0; i < count; ++i) items[i].v = cls[of[i]].take;
     return items;

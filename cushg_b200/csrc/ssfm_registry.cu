@@ -1,6 +1,9 @@
 // ssfm_registry.cu — lookup of the compiled fused-march variants and the autotuner's
 // choices (see ssfm_variants.h).
+#include <algorithm>
+#include <functional>
 #include <mutex>
+#include <queue>
 #include <vector>
 
 #include "../../include/shg.h"
@@ -98,14 +101,34 @@ const PlainVariant* find_split(int precision, int n, int cluster, int threads) {
     return v;
 }
 
-// 64 x 64 FP32 runs past the rows of kFew: 4-CTA clusters, five CTAs to an SM, take 26.7 us per step where
-// one CTA of 512 threads per run takes 30.0 (220 runs), as 149 of those are a second wave.  Beside
-// larger sides their CTAs hold up the clusters that need a whole SM: 160 runs of 64 x 64 and 8 of 128 x 128
-// (61 slices) took 2.73 ms against 1.90, with two of 256 x 256 3.2 against 2.0, a sweep of 256 runs over
-// 64-256 75.2 against 74.1.  With up to three runs of 96 x 96 or 128 x 128 beside 149-700 they were
-// never slower (three of 96 x 96 beside 160: 1.87 against 2.70), with four sometimes (128 x 128: 2.66 against 1.87).
-const PlainVariant* many_small_variant(int runs64, int runs_to_128, int runs_above) {
-    return runs64 >= 149 && runs_to_128 <= 3 && runs_above == 0 ? find_split(32, 64, 4, 128) : nullptr;
+// 64 x 64 FP32 runs past the rows of kFew, by the modelled time of the two splits.  One CTA of 512
+// threads per run: 13.3 us per step, 148 runs at a time, the longest first.  4-CTA clusters, five CTAs to
+// an SM: 17.8 us per step of the longest run, and 0.099 us per step of all of them together.  Over 152 to 600
+// runs of equal, nearly equal, uniform, log-uniform and two lengths the choice was at most 4 %
+// slower than the other.  ms on one CTA / on clusters: 160 equal runs of 149 steps 3.95 / 2.65, 300 5.93 /
+// 4.48, 600 9.95 / 8.73; 296 (two full waves) of 60 steps 1.77 / 1.93; 160 of 99-399 steps 5.24 / 6.45, 300 of
+// 20-250 3.35 / 4.17.
+//   Beside larger sides the clusters' CTAs hold up clusters that need a whole SM: 160 runs of 64 x 64 and
+// 8 of 128 x 128 (61 slices) took 2.73 ms against 1.90, with two of 256 x 256 3.2 against 2.0, a sweep of
+// 256 runs over 64-256 75.2 against 74.1.  With up to three runs of 96 x 96 or 128 x 128 beside 149-450
+// equal ones they were never slower (three of 96 x 96 beside 160: 1.87 against 2.70), with four
+// sometimes (128 x 128: 2.66 against 1.87).
+const PlainVariant* many_small_variant(std::vector<int> steps64, int runs_to_128, int runs_above) {
+    constexpr int kPlaces = 148;
+    if ((int)steps64.size() <= kPlaces || runs_to_128 > 3 || runs_above > 0) return nullptr;
+    std::sort(steps64.begin(), steps64.end(), [](int a, int b) { return a > b; });
+    std::priority_queue<long long, std::vector<long long>, std::greater<long long>> ends;  // of the places' queues
+    for (int i = 0; i < kPlaces; ++i) ends.push(0);
+    long long total = 0, last = 0;
+    for (int st : steps64) {
+        const long long e = ends.top() + st;
+        ends.pop();
+        ends.push(e);
+        last = std::max(last, e);
+        total += st;
+    }
+    const double clusters = std::max(17.8 * steps64[0], 0.099 * (double)total);
+    return clusters < 13.3 * (double)last ? find_split(32, 64, 4, 128) : nullptr;
 }
 
 const PlainVariant* find_plain_variant(int precision, int n, int thermal, int march) {

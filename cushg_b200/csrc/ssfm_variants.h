@@ -9,6 +9,8 @@
 #include <cuda_runtime.h>
 #include <stddef.h>
 
+#include <vector>
+
 #include "shg_internal.h"
 
 namespace shg {
@@ -73,9 +75,9 @@ const PlainVariant* wide_thermal_variant(int precision, int n, int count);
 // number of runs up to which it is the fastest of them, with no other class (alone) or beside some;
 // null past the last.
 const PlainVariant* few_runs_variant(int precision, int n, int level, bool alone, int* upto);
-// The variant of the 64 x 64 FP32 runs of a larger batch that holds `runs64` of them, `runs_to_128` runs of
-// the sides above 64 up to 128 and `runs_above` of larger ones; null: the default.
-const PlainVariant* many_small_variant(int runs64, int runs_to_128, int runs_above);
+// The variant of the 64 x 64 FP32 runs of a larger batch with these step counts, beside `runs_to_128`
+// runs of the sides above 64 up to 128 and `runs_above` of larger ones; null: the default.
+const PlainVariant* many_small_variant(std::vector<int> steps64, int runs_to_128, int runs_above);
 // find_plain_variant without the choices below.
 const PlainVariant* default_variant(int precision, int n, int thermal, int march);
 // Every compiled plain variant of (precision, n) but those for few runs; returns how many.

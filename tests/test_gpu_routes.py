@@ -72,6 +72,19 @@ def test_many_small_runs_beside_others():
     assert marches(batch((64, 140))) == {"plain<float, 64, 1, 512>"}
 
 
+def test_many_small_runs_by_their_lengths():
+    """One CTA per run is the faster split where the runs fill the device's waves (two full waves of
+    equal runs) or where the longest bounds the batch."""
+    assert marches(batch((64, 230))) == {"plain<float, 64, 4, 128>"}
+    assert marches(batch((64, 296))) == {"plain<float, 64, 1, 512>"}
+    assert marches(batch((64, 330))) == {"plain<float, 64, 4, 128>"}
+    assert marches(batch((64, 444))) == {"plain<float, 64, 1, 512>"}
+    ps = [run(64, nz=20 + i % 60) for i in range(200)]
+    assert marches(lambda: shg.solve_batch_device(ps)) == {"plain<float, 64, 1, 512>"}
+    ps = [run(64, nz=40 + i % 3) for i in range(200)]
+    assert marches(lambda: shg.solve_batch_device(ps)) == {"plain<float, 64, 4, 128>"}
+
+
 @pytest.fixture
 def no_choices():
     shg.autotune_reset()

@@ -171,6 +171,7 @@ static std::vector<BatchItem> batch_items(const shg_params* params, int count) {
         const PlainVariant* v;
         bool automatic;
         int runs;
+        double work;
         const PlainVariant* take;
     };
     std::vector<Class> cls;
@@ -183,8 +184,9 @@ static std::vector<BatchItem> batch_items(const shg_params* params, int count) {
         const bool automatic = params[i].march == SHG_MARCH_AUTO;
         size_t c = 0;
         while (c < cls.size() && (cls[c].v != v || cls[c].automatic != automatic)) ++c;
-        if (c == cls.size()) cls.push_back({v, automatic, 0, v});
+        if (c == cls.size()) cls.push_back({v, automatic, 0, 0.0, v});
         ++cls[c].runs;
+        cls[c].work += items[i].cost;
         of[i] = (int)c;
     }
     for (Class& c : cls) c.automatic = c.automatic && !plain_choice_rules(c.v->precision, c.v->n, c.runs);
@@ -204,9 +206,19 @@ static std::vector<BatchItem> batch_items(const shg_params* params, int count) {
     }
     if (!fits) {
         int small = -1, to_128 = 0, above = 0;
+        Class* large = nullptr;             // 256 x 256 FP32
+        double share = 0.0, most = 0.0;  // of the classes above 64 beside it: the device their clusters fill, most work
         for (Class& c : cls) {
             c.take = c.v;
             if (c.automatic && c.v == default_variant(32, 64, 0, SHG_MARCH_AUTO)) small = (int)(&c - cls.data());
+            if (c.automatic && c.v == default_variant(32, 256, 0, SHG_MARCH_AUTO)) {
+                large = &c;
+            } else if (c.v->n > 64) {
+                int fit = 0;
+                if (c.v->fit && c.v->fit(&fit) != cudaSuccess) cudaGetLastError();
+                share += fit > 0 ? (double)c.runs / fit : 2.0;  // multi-pass: the whole device
+                most = std::max(most, c.work);
+            }
             to_128 += c.v->n > 64 && c.v->n <= 128 ? c.runs : 0;
             above += c.v->n > 128 ? c.runs : 0;
         }
@@ -216,6 +228,8 @@ static std::vector<BatchItem> batch_items(const shg_params* params, int count) {
                 if (of[i] == small) steps.push_back(shg_steps(&params[i]));
             if (const PlainVariant* w = many_small_variant(std::move(steps), to_128, above)) cls[small].take = w;
         }
+        if (large)
+            if (const PlainVariant* w = mixed_256_variant(large->runs, large->work, most, share)) large->take = w;
     }
     for (int i = 0; i < count; ++i) items[i].v = cls[of[i]].take;
     return items;

@@ -71,7 +71,7 @@ cudaError_t plain_fit(int* instances) {
 
 #define SHG_VARIANT(T, PREC, N, C, NT, MINB, THERM)                                                  \
     {PREC, N, C, NT, MINB, THERM ? 1 : 0, PlainCfg<T, N, C, NT, THERM>::smem_bytes,                   \
-     &launch_plain<T, N, C, NT, THERM, MINB>, nullptr}
+     &launch_plain<T, N, C, NT, THERM, MINB>, nullptr, &plain_fit<T, N, C, NT, THERM, MINB, false>}
 // with a thread per field and point pair (plain runs)
 #define SHG_SPLIT_VARIANT(T, PREC, N, C, NT, MINB)                                        \
     {PREC, N, C, NT, MINB, 0, PlainCfg<T, N, C, NT>::smem_bytes,                          \

@@ -131,6 +131,23 @@ const PlainVariant* many_small_variant(std::vector<int> steps64, int runs_to_128
     return clusters < 13.3 * (double)last ? find_split(32, 64, 4, 128) : nullptr;
 }
 
+// 256 x 256 FP32 runs of a larger batch beside smaller ones.  The multi-pass march that these runs take
+// by themselves is a row of launches, and each of them waits for places that the persistent CTAs of 128 x 128
+// and 192 x 192 runs hold; 16-CTA clusters hold theirs.  While the device is not full the batch lasts
+// as long as its longest run, and the clusters win: sweeps of 16-48 runs over 64-256 (100-400
+// slices) took 1.0-1.17 times as long on the multi-pass march, of 64-128 runs 0.79-0.98.  `share` is the part
+// of the device that the batch's clusters fill, 14 of these runs to a device; the line lies at 1.5 (1.46
+// 1.12, 1.51 1.00, 1.72 0.95).  With only 64 x 64 runs beside, whose CTAs leave by themselves, the
+// multi-pass march is as fast or faster; beside less than a tenth of the others it is from 11 runs on
+// (8 runs and one of 128 x 128 1.25, 10 and one 1.07, 13 and one 0.87); with 14 runs or more the clusters
+// leave no place for the others, and where another class has more work it goes first and holds theirs.
+const PlainVariant* mixed_256_variant(int runs, double work, double others_work, double others_share) {
+    const double share = runs / 14.0 + others_share;
+    if (others_share <= 0.0 || runs > 13 || share > 1.5 || others_work > work) return nullptr;
+    if (runs > 10 && others_share < 0.1) return nullptr;
+    return default_variant(32, 256, 0, SHG_MARCH_FUSED);
+}
+
 const PlainVariant* find_plain_variant(int precision, int n, int thermal, int march) {
     if (march == SHG_MARCH_AUTO && !thermal) {
         std::lock_guard<std::mutex> lk(g_mu);

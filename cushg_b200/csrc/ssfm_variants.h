@@ -78,6 +78,10 @@ const PlainVariant* few_runs_variant(int precision, int n, int level, bool alone
 // The variant of the 64 x 64 FP32 runs of a larger batch with these step counts, beside `runs_to_128`
 // runs of the sides above 64 up to 128 and `runs_above` of larger ones; null: the default.
 const PlainVariant* many_small_variant(std::vector<int> steps64, int runs_to_128, int runs_above);
+// The variant of the `runs` 256 x 256 FP32 runs of a larger batch: work is their point-steps, others_work the
+// most that a class of 128 x 128 or 192 x 192 runs has, others_share the part of the device that those classes'
+// clusters fill; null: the default.
+const PlainVariant* mixed_256_variant(int runs, double work, double others_work, double others_share);
 // find_plain_variant without the choices below.
 const PlainVariant* default_variant(int precision, int n, int thermal, int march);
 // Every compiled plain variant of (precision, n) but those for few runs; returns how many.

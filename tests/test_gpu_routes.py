@@ -85,6 +85,20 @@ def test_many_small_runs_by_their_lengths():
     assert marches(lambda: shg.solve_batch_device(ps)) == {"plain<float, 64, 4, 128>"}
 
 
+
+def test_256_fp32_runs_beside_smaller_ones():
+    """While the batch's clusters do not fill the device the 256 x 256 FP32 runs of a mixed batch stay on
+    clusters of their own; alone, in larger batches and beside 64 x 64 runs only they take the multi-pass march."""
+    fused, multi = "plain<float, 256, 16, 256>", "multipass<float, 256>"
+    for classes in [((256, 9), (192, 8), (128, 8), (64, 8)), ((256, 7), (192, 6), (128, 8)), ((256, 12), (192, 12), (64, 12))]:
+        got = marches(batch(*classes))
+        assert fused in got and multi not in got, classes
+    for classes in [((256, 9),), ((256, 9), (64, 100)), ((256, 30), (192, 30)), ((256, 13), (128, 1)), ((256, 8), (192, 40)),
+                    ((256, 9), (512, 2), (192, 8))]:
+        got = marches(batch(*classes))
+        assert multi in got and fused not in got, classes
+
+
 @pytest.fixture
 def no_choices():
     shg.autotune_reset()

@@ -484,11 +484,11 @@ __device__ __forceinline__ double sum_rows(Get&& row, int lane) {
 // The thread index for the power sums of the fused march: the march's own, or threadIdx.x again.  Kept
 // alive for these sums it cost the 384-thread split of 192 x 192 FP32 runs, which is at its register
 // limit, a spill in every step (17 / 60 / 148 runs of 200 steps: 7.50 / 15.04 / 37.2 ms kept, 7.25 /
-// 14.65 / 36.3 taken again).  The splits with fewer threads are not at theirs, and most are 1-5 %
-// slower with it taken again.
-template <int NT, bool SPLIT>
+// 14.65 / 36.3 taken again).  192 x 192 FP64 runs are 1.2-1.5 % faster with it taken again (300 runs of
+// 100 steps 76.2 / 75.1 ms); most other splits, which are not at their limit, 1-5 % slower.
+template <typename T, int N, int NT, bool SPLIT>
 __device__ __forceinline__ int power_tid(int tid) {
-    if constexpr (!SPLIT && NT >= 384) return threadIdx.x;
+    if constexpr (!SPLIT && (NT >= 384 || (sizeof(T) == 8 && N == 192))) return threadIdx.x;
     else return tid;
 }
 
@@ -949,7 +949,7 @@ __global__ void __launch_bounds__(NT, MINB)
         // ---- SH and pump power: row sums (in the twiddles' place), then the rows ------------
         if constexpr (!THERM) {
             double* rows = reinterpret_cast<double*>(tw);  // [2][RL]: SH, pump
-            const int pt = power_tid<NT, SPLIT>(tid), warp = pt >> 5, lane = pt & 31;
+            const int pt = power_tid<T, N, NT, SPLIT>(tid), warp = pt >> 5, lane = pt & 31;
             __syncthreads();
             for (int r = warp; r < 2 * Cfg::RL; r += NT / 32) {
                 const double a = row_abs2<T, N>(r < Cfg::RL ? Ss : Ps, r % Cfg::RL, lane);

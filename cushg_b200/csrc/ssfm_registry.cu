@@ -51,28 +51,36 @@ void for_each_variant(F&& f, bool few = false) {
 //   16-22.  64: 1-14 4.9-9.3 / 15, 15-48 9.9-14.7 / 15.5, 73-108 20.5 / 26.  96: 1-6 6.2-8.6 / 32.4,
 //   7-48 13-32 / 33.  128: 1-3 6.5-8.3 / 19.1, 4-7 11 / 19.1.  192: 1-6 8.5-21 / 25.8.
 //   256: 1-4 9.7-24 / 34, 5-7 33.7 / 33.6-36.6 (8: 66.8 / 37.6).  512: 1 19.0 / 39.3 (multi-pass)
-// `beside`: the runs that count as a full device in a batch with other classes, where that is not upto
-// (0: the row is for its class alone).
-struct FewRow { int precision, n, upto, cluster, threads, beside = -1; };
+// us1, us: of one run on the row's variant, and of upto of them.  beside: the runs that count as a full
+// device in a batch with other classes, where that is not upto (0: the row is for its class alone).
+struct FewRow { int precision, n, upto, cluster, threads; double us1, us; int beside = -1; };
 const FewRow kFew[] = {
-    {32, 32, 28, 16, 64},   {32, 48, 14, 16, 96},   {32, 48, 100, 4, 96},  {32, 64, 14, 16, 128},
-    {32, 64, 104, 4, 128},  {32, 64, 148, 1, 512},  {32, 96, 7, 16, 288},
-    {32, 96, 48, 8, 288},   {32, 96, 72, 2, 192},   {32, 128, 2, 0, 0},     {32, 128, 7, 16, 256}, {32, 128, 48, 8, 256},
-    {32, 128, 72, 2, 512},  {32, 128, 108, 4, 256}, {32, 192, 9, 0, 0},    {32, 192, 15, 8, 192, 16},
-    {32, 192, 36, 4, 384},  {32, 192, 48, 8, 192, 56},  {32, 256, 4, 0, 0},    {32, 256, 7, 16, 256, 6},
-    {32, 512, 1, 0, 0},
-    {64, 32, 28, 16, 64},   {64, 32, 60, 4, 128},   {64, 48, 14, 16, 160}, {64, 48, 100, 4, 96},
-    {64, 48, 148, 1, 288},  {64, 64, 14, 16, 256},  {64, 64, 48, 4, 128},  {64, 64, 72, 2, 256},
-    {64, 64, 108, 4, 128},  {64, 96, 6, 0, 0},      {64, 96, 48, 8, 288},  {64, 128, 3, 0, 0},
-    {64, 128, 7, 16, 512},  {64, 192, 6, 0, 0},     {64, 256, 4, 0, 0},
-    {64, 256, 7, 16, 256, 0},  {64, 512, 1, 0, 0},
+    {32, 32, 28, 16, 64, 2.9, 4.1},      {32, 48, 14, 16, 96, 3.5, 4.3},      {32, 48, 100, 4, 96, 6.5, 10.6},
+    {32, 64, 14, 16, 128, 3.6, 4.5},     {32, 64, 104, 4, 128, 7.1, 12.6},    {32, 64, 148, 1, 512, 13.2, 14.6},
+    {32, 96, 7, 16, 288, 5.2, 5.3},      {32, 96, 48, 8, 288, 9.5, 18.3},     {32, 96, 72, 2, 192, 23.0, 23.2},
+    {32, 128, 2, 0, 0, 5.9, 6.2},        {32, 128, 7, 16, 256, 7.0, 7.0},     {32, 128, 48, 8, 256, 11.0, 25.4},
+    {32, 128, 72, 2, 512, 29.0, 30.1},   {32, 128, 108, 4, 256, 20.0, 59.2},  {32, 192, 9, 0, 0, 6.8, 22.9},
+    {32, 192, 15, 8, 192, 26.2, 26.4, 16}, {32, 192, 36, 4, 384, 36.1, 37.4}, {32, 192, 48, 8, 192, 26.2, 60.6, 56},
+    {32, 256, 4, 0, 0, 8.0, 18.6},       {32, 256, 7, 16, 256, 20.6, 21.0, 6}, {32, 512, 1, 0, 0, 14.7, 14.7},
+    {64, 32, 28, 16, 64, 3.0, 4.7},      {64, 32, 60, 4, 128, 4.8, 6.0},      {64, 48, 14, 16, 160, 3.9, 7.6},
+    {64, 48, 100, 4, 96, 7.6, 14.4},     {64, 48, 148, 1, 288, 15.8, 16.0},   {64, 64, 14, 16, 256, 4.5, 8.8},
+    {64, 64, 48, 4, 128, 9.4, 13.9},     {64, 64, 72, 2, 256, 14.3, 15.1},    {64, 64, 108, 4, 128, 9.4, 23.6},
+    {64, 96, 6, 0, 0, 5.9, 8.9},         {64, 96, 48, 8, 288, 12.8, 30.7},    {64, 128, 3, 0, 0, 6.2, 7.9},
+    {64, 128, 7, 16, 512, 10.8, 10.8},   {64, 192, 6, 0, 0, 8.0, 21.2},       {64, 192, 7, 16, 192, 24.9, 25.3, 0},
+    {64, 256, 4, 0, 0, 9.5, 24.6},       {64, 256, 7, 16, 256, 33.1, 33.4, 0}, {64, 512, 1, 0, 0, 19.5, 19.5},
 };
 
 }  // namespace
 
-const PlainVariant* few_runs_variant(int precision, int n, int level, bool alone, int* upto) {
+FewRuns few_runs_variant(int precision, int n, int runs, int level, bool alone, const PlainVariant* own) {
     for (const FewRow& r : kFew) {
-        if (r.precision != precision || r.n != n || (r.beside == 0 && !alone) || level-- > 0) continue;
+        if (r.precision != precision || r.n != n) continue;
+        if (r.beside == 0 && !alone && !(own && own->cluster == r.cluster && own->threads == r.threads)) continue;
+        if (level > 0) {
+            --level;
+            continue;
+        }
+        if (own && r.cluster == 0) continue;
         const PlainVariant* v = nullptr;
         for_each_variant([&](const PlainVariant* c) {
             if (c->precision == precision && c->n == n && !c->thermal && c->cluster == r.cluster &&
@@ -83,13 +91,12 @@ const PlainVariant* few_runs_variant(int precision, int n, int level, bool alone
         int fit = 0;
         if (v && v->fit && v->fit(&fit) != cudaSuccess) {
             cudaGetLastError();  // the device cannot hold the launch: the next row, the default can
-            level = 0;
             continue;
         }
-        *upto = alone || r.beside < 0 ? r.upto : r.beside;
-        return v;
+        const double at = r.upto > 1 ? std::min(1.0, (runs - 1.0) / (r.upto - 1.0)) : 0.0;
+        return {v, alone || r.beside <= 0 ? r.upto : r.beside, r.us1 + (r.us - r.us1) * at, r.cluster == 0};
     }
-    return nullptr;
+    return {nullptr, 0, 0.0, false};
 }
 
 const PlainVariant* find_split(int precision, int n, int cluster, int threads) {
@@ -137,13 +144,14 @@ const PlainVariant* many_small_variant(std::vector<int> steps64, int runs_to_128
 // as long as its longest run, and the clusters win: sweeps of 16-48 runs over 64-256 (100-400
 // slices) took 1.0-1.17 times as long on the multi-pass march, of 64-128 runs 0.79-0.98.  `share` is the part
 // of the device that the batch's clusters fill, 14 of these runs to a device; the line lies at 1.5 (1.46
-// 1.12, 1.51 1.00, 1.72 0.95).  With only 64 x 64 runs beside, whose CTAs leave by themselves, the
+// 1.12, 1.51 1.00, 1.72 0.95), and at 1 where a tenth and more of it is runs that a guard promotes to FP64,
+// whose clusters go first (guarded sweeps of 16-48 runs: up to 1 1.0-1.3, above 0.79-1.13).  With only 64 x 64 runs beside, whose CTAs leave by themselves, the
 // multi-pass march is as fast or faster; beside less than a tenth of the others it is from 11 runs on
 // (8 runs and one of 128 x 128 1.25, 10 and one 1.07, 13 and one 0.87); with 14 runs or more the clusters
 // leave no place for the others, and where another class has more work it goes first and holds theirs.
-const PlainVariant* mixed_256_variant(int runs, double work, double others_work, double others_share) {
+const PlainVariant* mixed_256_variant(int runs, double work, double others_work, double others_share, double promoted_share) {
     const double share = runs / 14.0 + others_share;
-    if (others_share <= 0.0 || runs > 13 || share > 1.5 || others_work > work) return nullptr;
+    if (others_share <= 0.0 || runs > 13 || share > (promoted_share < 0.1 ? 1.5 : 1.0) || others_work > work) return nullptr;
     if (runs > 10 && others_share < 0.1) return nullptr;
     return default_variant(32, 256, 0, SHG_MARCH_FUSED);
 }

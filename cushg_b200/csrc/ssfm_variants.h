@@ -71,17 +71,23 @@ const PlainVariant* find_plain_variant(int precision, int n, int thermal = 0, in
 // The wide march (ssfm_wide.cuh) of thermal passes of (precision, n) if it is the faster one for
 // `count` runs that have the device to themselves, else null.
 const PlainVariant* wide_thermal_variant(int precision, int n, int count);
-// Plain runs of (precision, n): the level-th variant for few runs, from the widest on, and the
-// number of runs up to which it is the fastest of them, with no other class (alone) or beside some;
-// null past the last.
-const PlainVariant* few_runs_variant(int precision, int n, int level, bool alone, int* upto);
+// Plain runs of (precision, n): the level-th variant for few runs, from the widest on; v is null past the
+// last.  alone: with no other class.  own, if given: no wide march (a cooperative launch, which has the
+// device to itself while it runs) but the next row, the class's own variant among them.
+struct FewRuns {
+    const PlainVariant* v;
+    int upto;   // the number of runs up to which it is the fastest, or that fill the device beside other classes
+    double us;  // per step, of `runs` runs
+    bool wide;
+};
+FewRuns few_runs_variant(int precision, int n, int runs, int level, bool alone, const PlainVariant* own = nullptr);
 // The variant of the 64 x 64 FP32 runs of a larger batch with these step counts, beside `runs_to_128`
 // runs of the sides above 64 up to 128 and `runs_above` of larger ones; null: the default.
 const PlainVariant* many_small_variant(std::vector<int> steps64, int runs_to_128, int runs_above);
 // The variant of the `runs` 256 x 256 FP32 runs of a larger batch: work is their point-steps, others_work the
 // most that a class of 128 x 128 or 192 x 192 runs has, others_share the part of the device that those classes'
-// clusters fill; null: the default.
-const PlainVariant* mixed_256_variant(int runs, double work, double others_work, double others_share);
+// clusters fill, promoted_share the FP64 ones' part of it; null: the default.
+const PlainVariant* mixed_256_variant(int runs, double work, double others_work, double others_share, double promoted_share);
 // find_plain_variant without the choices below.
 const PlainVariant* default_variant(int precision, int n, int thermal, int march);
 // Every compiled plain variant of (precision, n) but those for few runs; returns how many.

@@ -99,6 +99,17 @@ def test_256_fp32_runs_beside_smaller_ones():
         assert multi in got and fused not in got, classes
 
 
+
+def test_wide_march_in_a_mixed_batch():
+    """A cooperative launch has the device to itself, so the classes beside it wait: a mixed batch takes it
+    where its class bounds the batch, and clusters side by side where another class does."""
+    def got(n_large, n_small):
+        ps = [run(192, 64, nz=n_large)] + [run(64, 64, nz=n_small)] * 3
+        return marches(lambda: shg.solve_batch_device(ps))
+    assert got(60, 5) == {"wide<double, 192>", "plain<double, 64, 16, 256>"}
+    assert got(6, 60) == {"plain<double, 192, 16, 192>", "plain<double, 64, 16, 256>"}
+
+
 @pytest.fixture
 def no_choices():
     shg.autotune_reset()
